@@ -151,25 +151,25 @@ constexpr int kSteps = 64;
 // BVH with 8-bit boxes, 3 4-wide FP16 nodes).
 template <int MINB, int PREC>
 __global__ void __launch_bounds__(kTraceThreads, MINB) k_trace_closest(DevScene S, Ctrl* ctrl, int b, FrameBufs fb,
-                                                                       int steps) {
+                                                                       int steps, int min_lanes) {
   const int count = ctrl->count[b];
   bool overflow = false;
   tr::trace_persistent<false, kSteps, QueueRays, HitOut, PREC>(
       S, count, &ctrl->work[2 * b], QueueRays{fb.q_o[(b + 1) & 1], fb.q_d[(b + 1) & 1]}, HitOut{fb.hit_t, fb.hit_prim},
-      &overflow, steps);
+      &overflow, steps, min_lanes);
   if (overflow) atomicExch(&ctrl->error, kDevErrStack);
 }
 
 template <int MINB, int PREC>
 __global__ void __launch_bounds__(kTraceThreads, MINB) k_trace_shadow(DevScene S, Ctrl* ctrl, int b, int mode,
-                                                                      FrameBufs fb, int kahan, int steps) {
+                                                                      FrameBufs fb, int kahan, int steps, int min_lanes) {
   // mode 0: shadow slots are the compacted survivor slots (flagged by pixel >= 0)
   const int count = mode == 0 ? ctrl->count[b + 1] : ctrl->shadow[b];
   bool overflow = false;
   unsigned traced = 0;
   tr::trace_persistent<true, kSteps, ShadowRays, ShadowResolve, PREC>(
       S, count, &ctrl->work[2 * b + 1], ShadowRays{fb.s_o, fb.s_d},
-      ShadowResolve{fb.s_o, fb.s_c, fb.film, fb.film_c, kahan, &traced}, &overflow, steps);
+      ShadowResolve{fb.s_o, fb.s_c, fb.film, fb.film_c, kahan, &traced}, &overflow, steps, min_lanes);
   unsigned long long tot = traced;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) tot += __shfl_down_sync(0xffffffffu, tot, o);
@@ -696,39 +696,39 @@ int wide_blocks_per_sm() {
 int quad_steps_of(int steps) { return std::max(2, steps / 2); }
 template <int MINB>
 void launch_traces(cudaStream_t st, int grid, const DevScene& S, Ctrl* ctrl, int b, int mode, FrameBufs fb, int kahan,
-                   bool closest) {
+                   bool closest, int min_lanes) {
   const int steps = tuning_ref().refill_steps;
   if (S.bitstack && S.precision <= 1) {
     if (closest) {
-      if (S.precision == 1) k_trace_closest<MINB, 5><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, fb, steps);
-      else k_trace_closest<MINB, 4><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, fb, steps);
+      if (S.precision == 1) k_trace_closest<MINB, 5><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, fb, steps, min_lanes);
+      else k_trace_closest<MINB, 4><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, fb, steps, min_lanes);
     } else {
-      if (S.precision == 1) k_trace_shadow<MINB, 5><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, mode, fb, kahan, steps);
-      else k_trace_shadow<MINB, 4><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, mode, fb, kahan, steps);
+      if (S.precision == 1) k_trace_shadow<MINB, 5><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, mode, fb, kahan, steps, min_lanes);
+      else k_trace_shadow<MINB, 4><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, mode, fb, kahan, steps, min_lanes);
     }
     return;
   }
   if (closest) {
     const int f = S.precision;
     if (f == 3)
-      k_trace_closest<MINB, 3><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, fb, quad_steps_of(steps));
+      k_trace_closest<MINB, 3><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, fb, quad_steps_of(steps), min_lanes);
     else if (f == 2)
-      k_trace_closest<kWideMinBlocks, 2><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, fb, wide_steps_of(steps));
+      k_trace_closest<kWideMinBlocks, 2><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, fb, wide_steps_of(steps), min_lanes);
     else if (f == 1)
-      k_trace_closest<MINB, 1><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, fb, steps);
+      k_trace_closest<MINB, 1><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, fb, steps, min_lanes);
     else
-      k_trace_closest<MINB, 0><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, fb, steps);
+      k_trace_closest<MINB, 0><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, fb, steps, min_lanes);
   } else {
     const int f = S.precision;
     if (f == 3)
-      k_trace_shadow<MINB, 3><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, mode, fb, kahan, quad_steps_of(steps));
+      k_trace_shadow<MINB, 3><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, mode, fb, kahan, quad_steps_of(steps), min_lanes);
     else if (f == 2)
       k_trace_shadow<kWideMinBlocks, 2><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, mode, fb, kahan,
-                                                                        wide_steps_of(steps));
+                                                                        wide_steps_of(steps), min_lanes);
     else if (f == 1)
-      k_trace_shadow<MINB, 1><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, mode, fb, kahan, steps);
+      k_trace_shadow<MINB, 1><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, mode, fb, kahan, steps, min_lanes);
     else
-      k_trace_shadow<MINB, 0><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, mode, fb, kahan, steps);
+      k_trace_shadow<MINB, 0><<<grid, kTraceThreads, 0, st>>>(S, ctrl, b, mode, fb, kahan, steps, min_lanes);
   }
 }
 }  // namespace
@@ -763,7 +763,7 @@ unsigned tuning_version() { return g_tuning_version.load(); }
 
 // One persistent traversal launch over a queue of at most N rays.
 void launch_trace(cudaStream_t st, const DevScene& S, Ctrl* ctrl, int b, int mode, FrameBufs fb, int kahan, bool closest,
-                  int N, int num_sms, bool shared) {
+                  int N, int num_sms, bool shared, int min_lanes) {
   static int bps[17] = {};
   static int wide_bps = 0;
   const int minb = closest ? trace_minb() : shadow_minb();
@@ -774,15 +774,15 @@ void launch_trace(cudaStream_t st, const DevScene& S, Ctrl* ctrl, int b, int mod
   const int want = closest ? trace_grid_bps() : shadow_grid_bps();
   const int per_sm = !shared ? fit : want > 0 ? std::min(want, fit) : std::max(1, fit / 2);
   const int grid = std::max(1, std::min(num_sms * per_sm, (N + kTraceThreads - 1) / kTraceThreads));
-  if (minb == 16) launch_traces<16>(st, grid, S, ctrl, b, mode, fb, kahan, closest);
-  else if (minb == 12) launch_traces<12>(st, grid, S, ctrl, b, mode, fb, kahan, closest);
-  else launch_traces<8>(st, grid, S, ctrl, b, mode, fb, kahan, closest);
+  if (minb == 16) launch_traces<16>(st, grid, S, ctrl, b, mode, fb, kahan, closest, min_lanes);
+  else if (minb == 12) launch_traces<12>(st, grid, S, ctrl, b, mode, fb, kahan, closest, min_lanes);
+  else launch_traces<8>(st, grid, S, ctrl, b, mode, fb, kahan, closest, min_lanes);
 }
 
 int launch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const PassParams* d_pp, int mode, int max_depth,
                 int kahan, int width, int height, Ctrl* ctrl, FrameBufs fb, unsigned long long* status,
                 size_t status_stride, int num_sms, cudaEvent_t* ev, unsigned long long* totals, bool shared,
-                cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, int shade_split_req) {
+                cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, int shade_split_req, int min_lanes) {
   const bool two_launches = shade_split_req < 0 ? shade_split() : shade_split_req != 0;
   const int N = width * height;
   static int shade_bps[6] = {};
@@ -793,7 +793,7 @@ int launch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const PassP
   // for them
   const bool split = side && fork && join && !ev && tuning_ref().shadow_stream;
   if (split) shared = true;
-  auto trace = [&](bool closest, int b) { launch_trace(st, S, ctrl, b, mode, fb, kahan, closest, N, num_sms, shared); };
+  auto trace = [&](bool closest, int b) { launch_trace(st, S, ctrl, b, mode, fb, kahan, closest, N, num_sms, shared, min_lanes); };
   // persistent traversal: one resident wave, or fewer blocks for a small frame
   // (a queue never exceeds the frame's pixels), leaving SMs to other streams
   const int tiles = (N + kShadeThreads - 1) / kShadeThreads;
@@ -851,7 +851,7 @@ int launch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const PassP
     if (split) {
       cudaEventRecord(fork, st);
       cudaStreamWaitEvent(side, fork, 0);
-      launch_trace(side, S, ctrl, b, mode, fb, kahan, false, N, num_sms, shared);
+      launch_trace(side, S, ctrl, b, mode, fb, kahan, false, N, num_sms, shared, min_lanes);
       cudaEventRecord(join, side);
     } else {
       trace(false, b);
@@ -879,7 +879,7 @@ __global__ void k_raygen_batch(BatchFrames B, int total, Ctrl* ctrl, FrameBufs f
 
 int launch_batch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const int* d_start, const int* d_film,
                       const PassParams* d_pp, int nframes, int total, int max_depth, int kahan, Ctrl* ctrl,
-                      FrameBufs fb, int num_sms, unsigned long long* totals, bool shared) {
+                      FrameBufs fb, int num_sms, unsigned long long* totals, bool shared, int min_lanes) {
   const BatchFrames B{d_start, d_film, d_pp, nframes};
   static int shade_bps = 0;
   if (shade_bps == 0) shade_bps = shade_blocks_per_sm(4);
@@ -887,7 +887,7 @@ int launch_batch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const
   const int sgrid = std::max(1, std::min(num_sms * shade_bps, tiles));
   k_raygen_batch<<<(total + 255) / 256, 256, 0, st>>>(B, total, ctrl, fb);
   for (int b = 1; b <= max_depth; ++b) {
-    launch_trace(st, S, ctrl, b, 1, fb, kahan, true, total, num_sms, shared);
+    launch_trace(st, S, ctrl, b, 1, fb, kahan, true, total, num_sms, shared, min_lanes);
     if (shade_split()) {
       k_shade_hit<4, 0, BatchFrames><<<sgrid, kShadeThreads, 0, st>>>(S, E, B, ctrl, b, fb);
       if (S.tex_on)
@@ -898,7 +898,7 @@ int launch_batch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const
       k_shade<4, true, 0, BatchFrames><<<sgrid, kShadeThreads, 0, st>>>(S, E, B, ctrl, b, fb);
     else
       k_shade<4, false, 0, BatchFrames><<<sgrid, kShadeThreads, 0, st>>>(S, E, B, ctrl, b, fb);
-    launch_trace(st, S, ctrl, b, 1, fb, kahan, false, total, num_sms, shared);
+    launch_trace(st, S, ctrl, b, 1, fb, kahan, false, total, num_sms, shared, min_lanes);
   }
   if (totals) k_accumulate<<<1, 32, 0, st>>>(ctrl, max_depth, total, totals);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;

@@ -23,6 +23,15 @@ struct FrameBufs {
   int* live;        // queue slots of the paths that go on after the hit phase (two-launch shading)
 };
 
+// Rays of a short queue kept together in a warp, by how many frames or streams
+// of passes run side by side. Alone, one ray to a warp is fastest (1, 2, 4, 8,
+// 16, 32: the 200k soup at 800 x 600 12.2, 12.3, 12.5, 12.7, 13.3, 14.2 ms); with
+// six 1080p frames of the 1M soup in flight the GPU's issue slots are taken and
+// the spread rays' instructions cost (46.8, 46.6, 46.4, 46.1, 45.5, 45.2 ms for
+// eight frames); a served mix on four streams lies between (12.5, 12.7, 12.8, 13.1,
+// 13.5, 14.3 ms).
+inline int tail_lanes(int beside) { return beside <= 1 ? 1 : beside <= 4 ? 8 : 32; }
+
 // Launch shapes of the hot kernels, process-wide (one GPU per process):
 // closest_minb / shadow_minb: the traversal build, by the resident blocks per
 // SM its registers are bounded for (8, 12, 16); closest_grid / shadow_grid:
@@ -46,18 +55,20 @@ unsigned tuning_version();         // bumped by every set_tuning (jobs recapture
 // blocks an SM can hold, leaving room for their kernels.
 // side, fork, join: a second stream and two events of the caller's; with the
 // tuning's shadow_stream on, the shadow rays run there.
+// min_lanes: rays of a short queue that a traversal warp takes at least
+// (tail_lanes; tr::trace_persistent).
 // A merged batch pass (benchmark semantics, full-map environment sampling):
 // frames 0 .. nframes-1 share the queues; path g belongs to the frame k with
 // d_start[k] <= g < d_start[k+1] (pixel g - d_start[k]), its film slots start at
 // d_film[k], its parameters are d_pp[k]. total = d_start[nframes].
 int launch_batch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const int* d_start, const int* d_film,
                       const PassParams* d_pp, int nframes, int total, int max_depth, int kahan, Ctrl* ctrl,
-                      FrameBufs fb, int num_sms, unsigned long long* totals, bool shared = false);
+                      FrameBufs fb, int num_sms, unsigned long long* totals, bool shared = false, int min_lanes = 1);
 int launch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const PassParams* d_pp, int mode,
                 int max_depth, int kahan, int width, int height, Ctrl* ctrl, FrameBufs fb,
                 unsigned long long* status, size_t status_stride, int num_sms, cudaEvent_t* events,
                 unsigned long long* totals, bool shared = false, cudaStream_t side = nullptr,
-                cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr, int shade_split = -1);
+                cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr, int shade_split = -1, int min_lanes = 1);
 // The process's benchmark-semantics shading setting (MT_SHADE_SPLIT): -1 render
 // jobs choose per frame (shade_split_for) and other passes run two launches; 0
 // always one launch; 1 always two.

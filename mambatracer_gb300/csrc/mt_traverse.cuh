@@ -624,11 +624,11 @@ __device__ __forceinline__ bool wide_steps(const DevScene& S, RayT& r, WideState
 // given at run time).
 template <bool ANY, int STEPS, class Src, class Dst>
 __device__ __forceinline__ void trace_persistent_wide(const DevScene& S, int count, int* work, Src src, Dst dst,
-                                                      bool* overflow, int steps) {
+                                                      bool* overflow, int steps, int width) {
   const int lane = threadIdx.x & 31;
   uint2 stack[kWideStack];
   int i = -1;
-  bool exhausted = false;
+  bool exhausted = lane >= width;
   RayT r;
   WideState w;
   int sp = 0, hit = -1;
@@ -663,11 +663,11 @@ __device__ __forceinline__ void trace_persistent_wide(const DevScene& S, int cou
 
 template <bool ANY, int STEPS, class Src, class Dst, int PREC>
 __device__ __forceinline__ void trace_persistent_binary(const DevScene& S, int count, int* work, Src src, Dst dst,
-                                                        bool* overflow, int steps) {
+                                                        bool* overflow, int steps, int width) {
   const int lane = threadIdx.x & 31;
   typename StackEntry<ANY>::type stack[PREC == 3 ? kQuadStack : PREC >= 4 ? 1 : kStackDepth], top;
   int i = -1;
-  bool exhausted = false;
+  bool exhausted = lane >= width;
   RayT r;
   int ref = 0, sp = 0, hit = -1, leaf = kQuadEmpty, par = -1, sib = -1;
   unsigned long long bits = 0;
@@ -717,13 +717,23 @@ __device__ __forceinline__ void trace_persistent_binary(const DevScene& S, int c
 // PREC: 0 FP32 records, 1 FP16 records (binary, the reference's visit order),
 // 2 the wide BVH with 8-bit child boxes, 3 4-wide FP16 nodes, 4 / 5 FP32 / FP16
 // records traversed without a stack (bitstack_steps).
+// min_lanes: a queue too short to fill every warp of the grid is spread over
+// all of them, at least this many rays to a warp. A short queue is bound by its
+// longest ray (up to 350 node visits, one dependent read each), and in a warp
+// of 32 such rays every visit also waits for the others' reads and triangle
+// tests: one ray to a warp, the last bounce of the 1M soup (1128 rays) takes 229
+// us against 334 packed, bounce 8's shadow rays 154 against 242. Spread rays
+// issue their instructions once each, so frames that share the GPU keep more of
+// them together (tail_lanes).
 template <bool ANY, int STEPS, class Src, class Dst, int PREC = 0>
 __device__ __forceinline__ void trace_persistent(const DevScene& S, int count, int* work, Src src, Dst dst,
-                                                 bool* overflow, int steps = STEPS) {
+                                                 bool* overflow, int steps = STEPS, int min_lanes = 1) {
+  const int warps = gridDim.x * (blockDim.x / 32);
+  const int width = min(32, max(min_lanes, (count + warps - 1) / warps));
   if constexpr (PREC == 2)
-    trace_persistent_wide<ANY, STEPS>(S, count, work, src, dst, overflow, steps);
+    trace_persistent_wide<ANY, STEPS>(S, count, work, src, dst, overflow, steps, width);
   else
-    trace_persistent_binary<ANY, STEPS, Src, Dst, PREC>(S, count, work, src, dst, overflow, steps);
+    trace_persistent_binary<ANY, STEPS, Src, Dst, PREC>(S, count, work, src, dst, overflow, steps, width);
 }
 
 

@@ -136,16 +136,17 @@ int mt_bvh_import(mt_scene* scene, const int32_t* nodes, const float* bounds, in
 /* Traversal format: 0 = FP32 child boxes (default, 64-byte records, the
  * reference's visit order); 1 = FP16 child boxes rounded outward (32-byte
  * records); 2 = a wide BVH of up to eight children with 8-bit boxes rounded
- * outward (96-byte nodes); 3 = 4-wide nodes holding a record's grandchildren with
- * FP16 boxes rounded outward (64-byte nodes, leaves tested in warp-wide batches).
+ * outward (96-byte nodes); 3 = 4-wide nodes with FP16 boxes rounded outward
+ * (64-byte nodes, leaves tested in warp-wide batches) over a tree of its own,
+ * split by the surface-area heuristic on the GPU (1M triangles: 2.2 ms).
  * Formats 1-3 are kept beside the FP32 records and rebuilt with every BVH build
  * or import. Outward-rounded boxes contain the FP32 boxes, so closest hits are
  * the same triangles at the same distances; only which of two triangles hit at
  * exactly the same distance is reported can change with the visit order, and
  * among coplanar triangles hit within a few ulps of each other format 2 keeps
- * the nearer and format 3 either (its choice may change between runs, since
- * its leaf tests wait for the warp). Any-hit answers are the same in every
- * format. */
+ * the nearer and format 3 the one that 4-wide nodes over the FP32 records' tree
+ * meet first (its leaf tests wait for the warp, which can change that choice
+ * between runs). Any-hit answers are the same in every format. */
 int mt_scene_set_bvh_precision(mt_scene* scene, int precision);
 /* Replace the material table (TracerAPI material edits, src/cl/ui/fx/main/TracerAPI.java:371). */
 int mt_scene_set_materials(mt_scene* scene, const void* materials, int nmaterials);

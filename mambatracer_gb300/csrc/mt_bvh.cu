@@ -543,8 +543,9 @@ __global__ void k_quantize_fp16(const float4* __restrict__ recs, int nrec, uint4
 
 // 4-wide FP16 nodes from FP32 records: node r holds, for each child of record r,
 // that child's two children when it is interior, else the child (a leaf), with
-// the same outward rounding as the FP16 records.
-__global__ void k_quad_fp16(const float4* __restrict__ recs, int nrec, uint4* q) {
+// the same outward rounding as the FP16 records. The tree's nodes start at node
+// `first` of q.
+__global__ void k_quad_fp16(const float4* __restrict__ recs, int nrec, int first, uint4* q) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nrec) return;
   auto pair = [](float lo, float hi) {
@@ -574,7 +575,7 @@ __global__ void k_quad_fp16(const float4* __restrict__ recs, int nrec, uint4* q)
       kids(ref[c], gb, gr);
       for (int g = 0; g < 2; ++g, ++n) {
         for (int a = 0; a < 3; ++a) w[3 * n + a] = pair(gb[g][2 * a], gb[g][2 * a + 1]);
-        w[12 + n] = (unsigned)gr[g];
+        w[12 + n] = (unsigned)(gr[g] >= 0 ? first + gr[g] : gr[g]);
       }
     } else {
       for (int a = 0; a < 3; ++a) w[3 * n + a] = pair(box[c][2 * a], box[c][2 * a + 1]);
@@ -586,7 +587,7 @@ __global__ void k_quad_fp16(const float4* __restrict__ recs, int nrec, uint4* q)
     for (int a = 0; a < 3; ++a) w[3 * n + a] = empty_box;
     w[12 + n] = (unsigned)kQuadEmpty;
   }
-  uint4* o = q + 4 * (size_t)i;
+  uint4* o = q + 4 * ((size_t)first + i);
   o[0] = make_uint4(w[0], w[1], w[2], w[3]);
   o[1] = make_uint4(w[4], w[5], w[6], w[7]);
   o[2] = make_uint4(w[8], w[9], w[10], w[11]);
@@ -732,13 +733,23 @@ int refresh_qnodes(mt_scene* s) {
   }
   if (int w = refresh_wide(s)) return w;
   if (s->precision == 3 && s->has_bvh && s->nrec > 0) {
-    int r = dalloc(&s->d_quad, 4 * (size_t)s->nrec);
-    if (r) return r;
-    cudaStream_t st = s->ctx->stream;
-    k_quad_fp16<<<blocks(s->nrec), kT, 0, st>>>(s->d_nodes, s->nrec, s->d_quad);
-    if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) {
+    float4* sah = nullptr;
+    int r = build_sah_records(s, &sah);
+    if (!r) r = dalloc(&s->d_quad, (sah ? 8 : 4) * (size_t)s->nrec);
+    cudaError_t e = cudaSuccess;
+    if (!r) {
+      cudaStream_t st = s->ctx->stream;
+      s->quad_again = sah ? s->nrec : 0;
+      if (sah) k_quad_fp16<<<blocks(s->nrec), kT, 0, st>>>(sah, s->nrec, 0, s->d_quad);
+      k_quad_fp16<<<blocks(s->nrec), kT, 0, st>>>(s->d_nodes, s->nrec, s->quad_again, s->d_quad);
+      e = cudaGetLastError();
+      const cudaError_t w = cudaStreamSynchronize(st);
+      if (e == cudaSuccess) e = w;
+    }
+    dfree(sah);
+    if (r || e != cudaSuccess) {
       dfree(s->d_quad);
-      return fail(MT_ERR_CUDA, "4-wide FP16 nodes: %s", cudaGetErrorString(cudaGetLastError()));
+      return r ? r : fail(MT_ERR_CUDA, "4-wide FP16 nodes: %s", cudaGetErrorString(e));
     }
     return MT_OK;
   }

@@ -62,8 +62,10 @@ static_assert(sizeof(Material) == 144, "Material layout");
 //     w4 = (hi.y .., hi.z ..): one quantised plane per byte, plane = origin + q 2^(e-127);
 //          an empty slot holds lo = 255, hi = 0 (never hit)
 //   wtris: the triangles in wide-leaf order, 3 float4 each as in tris.
-//   quad: 4-wide FP16 nodes (precision 3), 4 uint4 = 64 B, indexed like nodes: the
-//     node of record r holds the grandchildren of r where a child of r is
+//   quad: 4-wide FP16 nodes (precision 3), 4 uint4 = 64 B, first over the records of
+//     the surface-area tree (mt_sah.cu), then, from quad_again on, over nodes (the
+//     reference's tree, for rays with near ties; alone where the other would be too
+//     deep): the node of record r holds the grandchildren of r where a child of r is
 //     interior and the child itself where it is a leaf, in the order left's
 //     children, right's children; words 3c .. 3c + 2 = child c's x, y, z extents
 //     as (lo rounded down, hi rounded up) half2 pairs, words 12 + c = child c's
@@ -80,6 +82,7 @@ struct DevScene {
   const int2* up;
   int bitstack;  // binary formats: 1 = the stackless traversal (bitstack and parent links)
   int root_ref;
+  int quad_again;  // 4-wide nodes: the root of those over the reference's tree
   int ntri;
   int nrec;
   int precision;  // traversal format: 0 FP32 records, 1 FP16 records, 2 the wide BVH, 3 4-wide FP16 nodes

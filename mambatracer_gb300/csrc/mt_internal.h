@@ -96,7 +96,8 @@ struct mt_scene {
   float4* d_tris = nullptr;
   uint4* d_qnodes = nullptr;  // FP16 records (precision 1)
   uint4* d_wnodes = nullptr;  // wide BVH with 8-bit child boxes (precision 2)
-  uint4* d_quad = nullptr;    // 4-wide FP16 nodes (precision 3)
+  uint4* d_quad = nullptr;    // 4-wide FP16 nodes (precision 3): the surface-area tree's, the reference's
+  int quad_again = 0;         // the first node of the latter
   int2* d_up = nullptr;       // parent links of the records (the stackless traversal)
   float4* d_wtris = nullptr;
   int nwide = 0, wdepth = 0;
@@ -133,6 +134,7 @@ struct mt_scene {
     s.wnodes = d_wnodes;
     s.wtris = d_wtris;
     s.quad = d_quad;
+    s.quad_again = quad_again;
     s.up = d_up;
     s.bitstack = d_up && traversal_bitstack();
     s.precision = (precision == 1 && d_qnodes) ? 1
@@ -261,6 +263,10 @@ void servers_sync(mt_context* ctx);
 // FP16 records (precision 1), 4-wide FP16 nodes (precision 3), and the wide BVH
 // (precision 2, refresh_wide).
 int refresh_qnodes(mt_scene* s);
+// FP32 records of a surface-area-heuristic tree over the scene's triangle slots
+// (mt_sah.cu; cudaFree'd by the caller), or NULL where that tree would be deeper
+// than the traversal stack holds. Two triangles or more.
+int build_sah_records(mt_scene* s, float4** recs_out);
 int refresh_wide(mt_scene* s);
 // MT_CDF_TABLES=0 turns the CDF tables of environment sampling off (the samplers
 // then search the SATs directly; the tables hold the same values).

@@ -983,7 +983,17 @@ __global__ void __launch_bounds__(kTraceThreads) k_count(DevScene S, const float
       }
     } else if constexpr (PREC == 3) {
       int leaf = kQuadEmpty, cnt[2] = {0, 0};
-      while (!tr::quad_steps<ANY>(S, r, ref, leaf, sp, hit, finite, stack, top, 1, &overflow, cnt)) {
+      int tie = tr::kTieNone;
+      const float tmax = r.tmax;
+      for (;;) {
+        if (!tr::quad_steps<ANY>(S, r, ref, leaf, sp, hit, finite, stack, top, 1, &overflow, tie, cnt)) continue;
+        if (tie != tr::kTieSeen || overflow) break;
+        r.tmax = tmax;
+        ref = S.quad_again;
+        leaf = kQuadEmpty;
+        sp = 0;
+        hit = -1;
+        tie = tr::kTieAgain;
       }
       visits = cnt[0];
       tests = cnt[1];

@@ -301,10 +301,10 @@ __device__ __forceinline__ bool bitstack_steps(const DevScene& S, RayT& r, int& 
 }
 
 // ------------------------------------------------------------------ 4-wide FP16
-// Precision 3: the node of record r holds the children of r's two children
-// (a leaf child stands for itself), so one 64-byte node read replaces the two
-// dependent record reads of two binary levels. The boxes are the FP32 records'
-// child boxes rounded outward to FP16 as in precision 1, tested with the same
+// Precision 3: the node of record r (of the surface-area tree of mt_sah.cu) holds
+// the children of r's two children (a leaf child stands for itself), so one 64-byte
+// node read replaces the two dependent record reads of two binary levels. The boxes
+// are the FP32 child boxes rounded outward to FP16 as in precision 1, tested with the same
 // slab arithmetic, so the boxes entered contain those the binary traversal
 // enters (a grandchild's box nests in its parent's) and every triangle it tests
 // is tested here with the same FP32 Moller-Trumbore: the closest hit is the same
@@ -356,12 +356,25 @@ __device__ __forceinline__ float2 sub_mul2(unsigned long long p, unsigned long l
 // ref: the next entry (a node >= 0, a leaf < 0, kQuadEmpty: nothing left);
 // leaf: the waiting leaf or kQuadEmpty. cnt (or NULL): [0] += node visits,
 // [1] += triangle tests.
+// Near ties of closest hits: boxes are culled only beyond near_hi(closest hit),
+// so every triangle within kNear of the closest is tested, and tie becomes
+// kTieSeen when a second one was. Which of two such triangles is kept follows from
+// the order of the tests, hence from the tree: such a ray (about one in 10^6 of the
+// stadium's) is traced once more from its start with tie = kTieAgain, from the
+// root of the nodes that follow the reference's tree (DevScene::quad_again) and
+// culling at the closest hit itself, so the tie falls as it does on that tree
+// whatever tree the nodes from root_ref follow.
+enum { kTieNone = 0, kTieSeen = 1, kTieAgain = 2 };
+constexpr float kNear = 0x1p-19f;  // 16 ulps: the triangle test's own rounding on coplanar neighbours is a few
+__device__ __forceinline__ float near_hi(float t) { return t * (1.f + kNear); }
 template <bool ANY>
 __device__ __forceinline__ bool quad_steps(const DevScene& S, RayT& r, int& ref, int& leaf, int& sp, int& hit_face,
                                            bool finite, typename StackEntry<ANY>::type* stack,
-                                           typename StackEntry<ANY>::type& top, int steps, bool* overflow,
+                                           typename StackEntry<ANY>::type& top, int steps, bool* overflow, int& tie,
                                            int* cnt = nullptr) {
   const float4* __restrict__ tris = S.tris;
+  // entries beyond this are culled
+  float thi = !ANY && tie != kTieAgain && hit_face >= 0 ? near_hi(r.tmax) : r.tmax;
   // (lo, hi) half pairs swapped to (near, far) by the direction's sign
   const unsigned selx = r.sx ? 0x1032u : 0x3210u, sely = r.sy ? 0x1032u : 0x3210u, selz = r.sz ? 0x1032u : 0x3210u;
   const unsigned long long oxy = pack2(r.ox, r.oy), ixy = pack2(r.ix, r.iy);
@@ -376,7 +389,7 @@ __device__ __forceinline__ bool quad_steps(const DevScene& S, RayT& r, int& ref,
       for (;;) {
         if (sp == 0) return kQuadEmpty;
         const int2 e = stack[--sp];
-        if (!finite || e.x < 0 || __int_as_float(e.y) < r.tmax) return e.x;
+        if (!finite || e.x < 0 || __int_as_float(e.y) < thi) return e.x;
       }
     }
   };
@@ -393,11 +406,29 @@ __device__ __forceinline__ bool quad_steps(const DevScene& S, RayT& r, int& ref,
         const float4* tp = tris + 3 * (size_t)(~leaf);
         const float4 p1 = __ldg(tp + 0), e1 = __ldg(tp + 1), e2 = __ldg(tp + 2);
         leaf = kQuadEmpty;
-        const float t = tri_t(r, p1, e1, e2);
-        if ((r.tmin < t) && (t < r.tmax)) {
-          hit_face = __float_as_int(p1.w);
-          if (ANY) return true;
-          r.tmax = t;
+        if constexpr (ANY) {
+          const float t = tri_t(r, p1, e1, e2);
+          if ((r.tmin < t) && (t < r.tmax)) {
+            hit_face = __float_as_int(p1.w);
+            return true;
+          }
+        } else {
+          const float best = r.tmax;
+          r.tmax = thi;
+          const float t = tri_t(r, p1, e1, e2);
+          r.tmax = best;
+          if ((r.tmin < t) && (t < thi)) {
+            if (tie != kTieAgain) {
+              // a tie with a triangle that is no longer among the nearest does not count
+              if (hit_face >= 0 && near_hi(t) >= best) tie = kTieSeen;
+              else if (t < best) tie = kTieNone;
+            }
+            if (t < best) {
+              hit_face = __float_as_int(p1.w);
+              r.tmax = t;
+              thi = tie != kTieAgain ? near_hi(t) : t;
+            }
+          }
         }
       }
       continue;
@@ -426,10 +457,13 @@ __device__ __forceinline__ bool quad_steps(const DevScene& S, RayT& r, int& ref,
         const float2 nxy = sub_mul2(pack2(x.x, y.x), oxy, ixy), fxy = sub_mul2(pack2(x.y, y.y), oxy, ixy);
         tn = max3f(nxy.x, nxy.y, (z.x - r.oz) * r.iz);
         const float tf = min3f(fxy.x, fxy.y, (z.y - r.oz) * r.iz);
-        h = (tn <= tf) && (tn < r.tmax) && (tf * 1.00000024f > r.tmin);
+        h = (tn <= tf) && (tn < thi) && (tf * 1.00000024f > r.tmin);
       } else {
         const float2 x = half2_bits(wv[3 * k]), y = half2_bits(wv[3 * k + 1]), z = half2_bits(wv[3 * k + 2]);
+        const float best = r.tmax;
+        r.tmax = thi;
         h = slab(r, x.x, x.y, y.x, y.y, z.x, z.y, &tn) && cr[k] != kQuadEmpty;
+        r.tmax = best;
         if (tn != tn) tn = -INFINITY;  // order only: a NaN entry distance sorts first
       }
       key[k] = h ? tn : INFINITY;
@@ -672,6 +706,7 @@ __device__ __forceinline__ void trace_persistent_binary(const DevScene& S, int c
   int ref = 0, sp = 0, hit = -1, leaf = kQuadEmpty, par = -1, sib = -1;
   unsigned long long bits = 0;
   bool finite = true;
+  int tie = kTieNone;
   for (;;) {
     const bool need = (i < 0) && !exhausted;
     const unsigned m = __ballot_sync(0xffffffffu, need);
@@ -692,6 +727,7 @@ __device__ __forceinline__ void trace_persistent_binary(const DevScene& S, int c
           bits = 0;
           par = sib = -1;
           hit = -1;
+          tie = kTieNone;
         }
       }
       if (base + __popc(m) >= count) exhausted = true;
@@ -701,13 +737,24 @@ __device__ __forceinline__ void trace_persistent_binary(const DevScene& S, int c
     bool done = false;
     if (active) {
       if constexpr (PREC == 3)
-        done = quad_steps<ANY>(S, r, ref, leaf, sp, hit, finite, stack, top, steps, overflow);
+        done = quad_steps<ANY>(S, r, ref, leaf, sp, hit, finite, stack, top, steps, overflow, tie);
       else if constexpr (PREC >= 4)
         done = bitstack_steps<ANY, PREC - 4>(S, r, ref, bits, par, sib, hit, finite, steps);
       else
         done = trav_steps<ANY, PREC>(S, r, ref, sp, hit, finite, stack, top, steps, overflow);
     }
     if (done) {
+      if constexpr (PREC == 3 && !ANY) {
+        if (tie == kTieSeen) {
+          r.tmax = src(i).tmax;
+          ref = S.quad_again;
+          leaf = kQuadEmpty;
+          sp = 0;
+          hit = -1;
+          tie = kTieAgain;
+          continue;
+        }
+      }
       dst(i, r, hit);
       i = -1;
     }

@@ -317,8 +317,8 @@ __device__ __forceinline__ float D_H(V wh, float ax, float ay) {
 }
 __device__ __forceinline__ float G_Atten(V w1, V w2, float ax, float ay) { return 1.f / (1.f + lambda_(w1, ax, ay) + lambda_(w2, ax, ay)); }
 __device__ __forceinline__ float G1_(V w, float ax, float ay) { return 1.f / (1.f + lambda_(w, ax, ay)); }
-// Bsdf.cl:270-294
-__device__ __forceinline__ V sample_vndf(V v, float ax, float ay, float r1, float r2) {
+// Bsdf.cl:270-294 with r1 and the cosine and sine of phi = 2 pi r2
+__device__ __forceinline__ V sample_vndf(V v, float ax, float ay, float r1, float cphi, float sphi) {
   V Vh = normalize4(mk(ax * v.x, ay * v.y, v.z, 0.f));
   float lensq = Vh.x * Vh.x + Vh.y * Vh.y;
   V T1 = mk(1.f, 0.f, 0.f, 0.f);
@@ -328,9 +328,8 @@ __device__ __forceinline__ V sample_vndf(V v, float ax, float ay, float r1, floa
   }
   V T2 = cross4(Vh, T1);
   float r = sqrtf(r1);
-  float phi = 2.0f * kPi * r2;
-  float t1 = r * cosf(phi);
-  float t2 = r * sinf(phi);
+  float t1 = r * cphi;
+  float t2 = r * sphi;
   float s = 0.5f * (1.0f + Vh.z);
   t2 = (1.0f - s) * sqrtf(1.0f - t1 * t1) + s * t2;
   V Nh = add(add(smul(t1, T1), smul(t2, T2)), smul(sqrtf(maxf_(0.f, 1.f - t1 * t1 - t2 * t2)), Vh));
@@ -347,87 +346,92 @@ __device__ __forceinline__ V schlick3(float c, V f0) {
   float ex = powf(1.f - c, 5.0f);
   return mk(f0.x + (1.f - f0.x) * ex, f0.y + (1.f - f0.y) * ex, f0.z + (1.f - f0.z) * ex, 0.f);
 }
-// Bsdf.cl:380-394 with Sampling.cl:129-148
-__device__ __forceinline__ V sample_diffuse(const DevScene& S, const Bsdf& b, float sx, float sy, V* gen, float* pdfW) {
-  if (b.fix.z < kEpsCos) return zero4();
-  float term1 = 2.f * kPi * sx;
-  float term2 = sqrtf(1.f - sy);
-  V ret = mk(cosf(term1) * term2, sinf(term1) * term2, sqrtf(sy), 0.f);
-  float un = ret.z * 1.f / kPi;
-  *gen = ret;
-  *pdfW += un * b.pd;
-  V c = b.pm->diffuse_color;
-  return mk(c.x * 1.f / kPi, c.y * 1.f / kPi, c.z * 1.f / kPi, 1.f);
+// A local direction and the lobes to evaluate there: the light sample's direction or
+// the BSDF sample. A warp's lanes sample either lobe, and each then needs the other
+// lobe's value too; keeping the direction apart from the evaluation lets all of
+// them run one copy of the glossy terms together (Bsdf.cl inlined twice over held
+// 58 KB of code, and warps with lanes of both kinds ran both copies in turn).
+struct LobeDir {
+  V gen;  // local direction
+  V wh;   // glossy half vector (glo only)
+  bool dif, glo;
+};
+// evaluateBsdf's direction (Bsdf.cl:452-545): world in the hit's frame; below the
+// surface no lobe is evaluated and *cosGen stays.
+__device__ __forceinline__ LobeDir eval_dir(const Bsdf& b, V world, float* cosGen) {
+  LobeDir d;
+  d.gen = local_coord(b.frame, world);
+  d.dif = d.glo = false;
+  if (d.gen.z * b.fix.z < 0.f) return d;
+  *cosGen = d.gen.z;
+  const bool up = !(b.fix.z < kEpsCos || d.gen.z < kEpsCos);
+  d.dif = up && !(b.pd == 0.f);
+  d.glo = up && !(b.pg == 0.f);
+  if (d.glo) d.wh = normalize4(add(b.fix, d.gen));
+  return d;
 }
-// Bsdf.cl:396-432
-__device__ __forceinline__ V sample_glossy(const DevScene& S, const Bsdf& b, float sx, float sy, V* gen, float* pdfW) {
-  if (b.fix.z < kEpsCos) return zero4();
-  const Material& M = *b.pm;
-  float ax = M.glossy_param.y, ay = M.glossy_param.z;
-  V wh = sample_vndf(b.fix, ax, ay, sx, sy);
-  V wo = add(neg(b.fix), smul(2.f * dot4(b.fix, wh), wh));
-  *gen = wo;
-  float cI = fabsf(b.fix.z), cO = fabsf(wo.z);
-  *pdfW += b.pg * pdf_vndf(wo, wh, ax, ay);
-  float fr = G_Atten(b.fix, wo, ax, ay) * D_H(wh, ax, ay) / (4.f * cI * cO);
-  float whdot = fabsf(dot4(wh, wo));
-  V Fc = schlick3(whdot, M.glossy_color);
-  if (cI == 0.f || cO == 0.f) Fc = zero4();
-  if (wh.x == 0.f && wh.y == 0.f && wh.z == 0.f) Fc = zero4();
-  return mk(Fc.x * fr, Fc.y * fr, Fc.z * fr, 0.f);
+// sampleBsdf's direction (Bsdf.cl:380-432, :555-606, Sampling.cl:129-148): a cosine
+// sample with probability pd, else a visible GGX normal.
+__device__ __forceinline__ LobeDir sample_dir(const Bsdf& b, float s0, float s1, float s2) {
+  LobeDir d;
+  d.gen = zero4();
+  d.dif = d.glo = false;
+  const bool diffuse = s2 < b.pd;
+  if (b.fix.z < kEpsCos) return d;
+  const float phi = 2.f * kPi * (diffuse ? s0 : s1);
+  const float c = cosf(phi), s = sinf(phi);
+  if (diffuse) {
+    const float r = sqrtf(1.f - s1);
+    d.gen = mk(c * r, s * r, sqrtf(s1), 0.f);
+    d.dif = true;
+    d.glo = !(b.pg == 0.f) && !(d.gen.z < kEpsCos);
+    if (d.glo) d.wh = normalize4(add(b.fix, d.gen));
+  } else {
+    d.wh = sample_vndf(b.fix, b.pm->glossy_param.y, b.pm->glossy_param.z, s0, c, s);
+    d.gen = add(neg(b.fix), smul(2.f * dot4(b.fix, d.wh), d.wh));
+    d.glo = true;
+    d.dif = !(b.pd == 0.f) && !(d.gen.z < kEpsCos);
+  }
+  return d;
 }
-// Bsdf.cl:452-467
-__device__ __forceinline__ V eval_diffuse(const DevScene& S, const Bsdf& b, V gen, float* pdfW) {
-  if (b.pd == 0.f) return zero4();
-  if (b.fix.z < kEpsCos || gen.z < kEpsCos) return zero4();
-  *pdfW += b.pd * fmaxf(0.f, gen.z * 1.f / kPi);
-  V c = b.pm->diffuse_color;
-  return mk(c.x * 1.f / kPi, c.y * 1.f / kPi, c.z * 1.f / kPi, 1.f);
-}
-// Bsdf.cl:469-507
-__device__ __forceinline__ V eval_glossy(const DevScene& S, const Bsdf& b, V gen, float* pdfW) {
-  if (b.pg == 0.f) return zero4();
-  if (b.fix.z < kEpsCos || gen.z < kEpsCos) return zero4();
-  const Material& M = *b.pm;
-  float ax = M.glossy_param.y, ay = M.glossy_param.z;
-  V wh = normalize4(add(b.fix, gen));
-  float cI = fabsf(b.fix.z), cO = fabsf(gen.z);
-  *pdfW += b.pg * pdf_vndf(gen, wh, ax, ay);
-  float fr = G_Atten(b.fix, gen, ax, ay) * D_H(wh, ax, ay) / (4.f * cI * cO);
-  float whdot = fabsf(dot4(wh, gen));
-  V Fc = schlick3(whdot, M.glossy_color);
-  if (cI == 0.f || cO == 0.f) Fc = zero4();
-  if (wh.x == 0.f && wh.y == 0.f && wh.z == 0.f) Fc = zero4();
-  return mk(Fc.x * fr, Fc.y * fr, Fc.z * fr, 0.f);
-}
-// Bsdf.cl:525-545
-__device__ __forceinline__ V eval_bsdf(const DevScene& S, const Bsdf& b, V world, float* pdfW, float* cosGen) {
+// The lobes' values and probabilities at d (Bsdf.cl:380-507; sums of two terms, so
+// their order does not matter).
+__device__ __forceinline__ V lobes(const Bsdf& b, const LobeDir& d, float* pdfW) {
   V result = mk(0.f, 0.f, 0.f, 1.f);
-  V gen = local_coord(b.frame, world);
-  if (gen.z * b.fix.z < 0.f) return result;
-  *cosGen = gen.z;
-  result = add(result, eval_diffuse(S, b, gen, pdfW));
-  result = add(result, eval_glossy(S, b, gen, pdfW));
+  if (d.dif) {
+    *pdfW += b.pd * fmaxf(0.f, d.gen.z * 1.f / kPi);
+    const V c = b.pm->diffuse_color;
+    result = add(result, mk(c.x * 1.f / kPi, c.y * 1.f / kPi, c.z * 1.f / kPi, 1.f));
+  }
+  if (d.glo) {
+    const Material& M = *b.pm;
+    const float ax = M.glossy_param.y, ay = M.glossy_param.z;
+    const float cI = fabsf(b.fix.z), cO = fabsf(d.gen.z);
+    *pdfW += b.pg * pdf_vndf(d.gen, d.wh, ax, ay);
+    const float fr = G_Atten(b.fix, d.gen, ax, ay) * D_H(d.wh, ax, ay) / (4.f * cI * cO);
+    const float whdot = fabsf(dot4(d.wh, d.gen));
+    V Fc = schlick3(whdot, M.glossy_color);
+    if (cI == 0.f || cO == 0.f) Fc = zero4();
+    if (d.wh.x == 0.f && d.wh.y == 0.f && d.wh.z == 0.f) Fc = zero4();
+    result = add(result, mk(Fc.x * fr, Fc.y * fr, Fc.z * fr, 0.f));
+  }
   return result;
 }
-// Bsdf.cl:555-606 (worldGen is left untouched when the sample is rejected)
+// The end of sampleBsdf: f, the lobes' value at d, or zero where the sample is
+// rejected (*world is then left untouched).
+__device__ __forceinline__ V sample_end(const Bsdf& b, const LobeDir& d, V f, V* world, float* cosGen) {
+  *cosGen = fabsf(d.gen.z);
+  if (*cosGen < kEpsCos) return zero4();
+  *world = world_coord(b.frame, d.gen);
+  return f;
+}
+__device__ __forceinline__ V eval_bsdf(const DevScene& S, const Bsdf& b, V world, float* pdfW, float* cosGen) {
+  return lobes(b, eval_dir(b, world, cosGen), pdfW);
+}
 __device__ __forceinline__ V sample_bsdf(const DevScene& S, const Bsdf& b, float s0, float s1, float s2, V* world,
                                          float* pdfW, float* cosGen) {
-  V result = mk(0.f, 0.f, 0.f, 1.f);
-  V gen = zero4();
-  if (s2 < b.pd) {
-    result = add(result, sample_diffuse(S, b, s0, s1, &gen, pdfW));
-    if (zero4(result)) return zero4();
-    result = add(result, eval_glossy(S, b, gen, pdfW));
-  } else {
-    result = add(result, sample_glossy(S, b, s0, s1, &gen, pdfW));
-    if (zero4(result)) return zero4();
-    result = add(result, eval_diffuse(S, b, gen, pdfW));
-  }
-  *cosGen = fabsf(gen.z);
-  if (*cosGen < kEpsCos) return zero4();
-  *world = world_coord(b.frame, gen);
-  return result;
+  const LobeDir d = sample_dir(b, s0, s1, s2);
+  return sample_end(b, d, lobes(b, d, pdfW), world, cosGen);
 }
 // Sampling.cl:212-235
 __device__ __forceinline__ float mis2(float a, float b) { return a / (a + b); }
@@ -616,13 +620,14 @@ __device__ __forceinline__ V sph_dir(float u, float v) {
   float theta = u * 2.f * kPi;
   return mk(-sinf(phi) * cosf(theta), cosf(phi), sinf(phi) * sinf(theta), 0.f);
 }
-// Light.cl:195-227
+// Light.cl:195-227. TAB: the CDF tables are there (else looked at when it runs).
+template <bool TAB = false>
 __device__ __forceinline__ V illuminate_env(const DevEnv& E, V s, V* dir, float* dist, float* pdfW) {
   Region r{E.w, E.h, 0, 0, E.w, E.h};
   float uv[2];
   int off[2];
   float pdf;
-  if (E.env_marg)  // tables of the map's CDFs
+  if (TAB || E.env_marg)  // tables of the map's CDFs
     sample_cont_tab(r, s.x, s.y, uv, off, &pdf, E.sat, E.lum, RegionTab{E.env_marg, E.env_cond});
   else
     sample_cont(r, s.x, s.y, uv, off, &pdf, E.sat, E.lum);
@@ -688,6 +693,7 @@ __device__ __forceinline__ Region env_tile_region(const DevEnv& E, int tx, int t
   const int x1 = (int)((float)E.w * ux1), y1 = (int)((float)E.h * uy1);
   return Region{E.w, E.h, x0, y0, x1 - x0, y1 - y0};
 }
+template <bool TAB = false>
 __device__ __forceinline__ V illuminate_env_grid(const DevEnv& E, const float* cam, V p, V s, V* dir, float* dist,
                                                  float* pdfW) {
   const int cell = grid_cell(E, cam, p);
@@ -695,7 +701,7 @@ __device__ __forceinline__ V illuminate_env_grid(const DevEnv& E, const float* c
   const Region rc{E.nu, E.nv, 0, 0, E.rx, E.ry};
   float uvLL[2], pdfLL, uvSS[2], pdfSS;
   int offLL[2], offSS[2];
-  if (E.cell_marg)  // tables of the cell's CDFs
+  if (TAB || E.cell_marg)  // tables of the cell's CDFs
     sample_cont_tab(rc, s.x, s.y, uvLL, offLL, &pdfLL, E.grid_sat + base, E.grid_func + base,
                     RegionTab{E.cell_marg + (size_t)cell * (E.ry + 2),
                               E.cell_cond + (size_t)cell * (E.ry + 1) * (E.rx + 2)});
@@ -705,7 +711,7 @@ __device__ __forceinline__ V illuminate_env_grid(const DevEnv& E, const float* c
   *pdfW = 0.f;
   if (!(pdfLL > 0.f)) return zero4();  // empty cell: the BSDF sample covers it alone
   const Region rt = env_tile_region(E, offLL[0], offLL[1]);
-  if (E.tile_marg) {  // tables of the tile's CDFs (tiles divide the map: every tile is tw x th)
+  if (TAB || E.tile_marg) {  // tables of the tile's CDFs (tiles divide the map: every tile is tw x th)
     const int tw = E.w / E.rx, th = E.h / E.ry, tile = offLL[1] * E.rx + offLL[0];
     sample_cont_tab(rt, s.z, s.w, uvSS, offSS, &pdfSS, E.sat, E.lum,
                     RegionTab{E.tile_marg + (size_t)tile * (th + 2), E.tile_cond + (size_t)tile * (th + 1) * (tw + 2)});

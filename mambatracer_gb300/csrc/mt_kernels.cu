@@ -19,71 +19,17 @@
 
 #include "mt_device.cuh"
 #include "mt_kernels.h"
-#include "mt_scan.cuh"
+#include "mt_shade.cuh"
 #include "mt_traverse.cuh"
 
 namespace mt {
 
 using namespace dv;
 
-namespace {
-
-using namespace scan;
-
-__device__ __forceinline__ void film_add(float4* __restrict__ acc, float4* __restrict__ comp, int pixel, V v, int kahan) {
-  if (!abs_valid4(v)) return;  // addAccum, src/cl/kernel/Render.cl:1-7
-  V a = acc[pixel];
-  if (!kahan) {
-    acc[pixel] = add(a, v);
-    return;
-  }
-  V c = comp[pixel];
-  V y = sub(v, c);
-  V t = add(a, y);
-  comp[pixel] = sub(sub(t, a), y);
-  acc[pixel] = t;
-}
-
-}  // namespace
-
 // ----------------------------------------------------------------- raygen
 // InitCameraRayDataJitter (src/cl/kernel/Initialize.cl:129-172) with the
 // per-frame camera constants precomputed on the host, plus the path and queue
 // resets of InitPathData / InitIntersection / InitIntDataToIndex.
-// The camera ray of pixel id (InitCameraRayDataJitter): origin, world direction.
-__device__ __forceinline__ void camera_ray(const PassParams* __restrict__ pp, int id, V* o_out, V* d_out) {
-  int32_t sx, sy;
-  if (pp->mode == 0) {
-    sx = pp->seeds[0];
-    sy = pp->seeds[1];
-  } else {
-    stage_seed(0, 0, &sx, &sy);
-  }
-  Seed s = gen_seed(sx, sy, pp->frame_count, pp->mode == 0 ? id : pixel_gid(id));
-  float r0 = rnd(s), r1 = rnd(s);
-  const int W = pp->width;
-  float px = (float)(id % W), py = (float)(id / W);
-  float j1 = pp->inv_w * (2.f * r0 - 1.f);
-  float j2 = pp->inv_h * (2.f * r1 - 1.f);
-  V d = normalize4(mk(pp->cam_a * (2.f * px / pp->dim_w - 1.f + j1), -2.f * py / pp->dim_h + 1.f + j2, -pp->cam_d, 0.f));
-  const float* m = pp->cam_m;
-  V z = zero4();
-  V m0 = mk(m[0], m[1], m[2], m[3]), m1 = mk(m[4], m[5], m[6], m[7]), m2 = mk(m[8], m[9], m[10], m[11]),
-    m3 = mk(m[12], m[13], m[14], m[15]);
-  V o = mk(dot3(m0, z) + m0.w, dot3(m1, z) + m1.w, dot3(m2, z) + m2.w, dot3(m3, z) + m3.w);
-  if (!(o.w == 1.f)) o = mk(o.x / o.w, o.y / o.w, o.z / o.w, 0.f);
-  V dw = mk(dot4(m0, d), dot4(m1, d), dot4(m2, d), 0.f);
-  *o_out = o;
-  *d_out = dw;
-}
-// Queue slot and path state g of a new path (InitPathData).
-__device__ __forceinline__ void start_path(FrameBufs& fb, int g, V o, V dw) {
-  fb.q_o[0][g] = mk(o.x, o.y, o.z, __int_as_float(g));
-  fb.q_d[0][g] = mk(dw.x, dw.y, dw.z, 0.f);
-  fb.thr[g] = mk(1.f, 1.f, 1.f, 1.f);
-  fb.ps[g] = mk(0.f, 0.f, 0.f, 1.f);  // hitpoint.xyz, lastPdfW
-  fb.flag[g] = 1;                     // lastSpecular
-}
 __global__ void k_raygen(const PassParams* __restrict__ pp, Ctrl* ctrl, FrameBufs fb) {
   const int N = pp->width * pp->height;
   const int id = blockIdx.x * blockDim.x + threadIdx.x;
@@ -177,420 +123,6 @@ __global__ void __launch_bounds__(kTraceThreads, MINB) k_trace_shadow(DevScene S
   if (overflow) atomicExch(&ctrl->error, kDevErrStack);
 }
 
-// ----------------------------------------------------------------- shade
-// The per-path work, in two phases around the reference's compaction:
-//   shade_hit       IntersectPrimitives' hit record, SetupBSDFPath and
-//                   LightHitPass (emitter or environment contribution);
-//   shade_continue  the texture pass, DirectLight (light sample, BSDF
-//                   evaluation, shadow ray) and SampleBSDFRayDirection, then
-//                   Russian roulette in benchmark semantics.
-struct PathState {
-  bool alive;
-  int pixel;                // queue slot's path index (path state)
-  int fidx;                 // film index of its pixel
-  int local;                // its pixel within its frame (the samples' key)
-  const PassParams* pp;     // its frame's parameters
-  V thr, ps;
-  int spec;
-  Hit H;
-  Bsdf B;
-};
-struct ShadeOut {
-  bool has_shadow;
-  V sho, shd, shc, ndir;
-};
-// LEAN: an instance for scenes without mesh lights (hence without emitters) lit
-// by an environment map through the light grid, the benchmark scenes' case; it
-// leaves out the code of the other cases, which keeps the shading kernel's
-// instruction footprint small.
-template <int LEAN> __device__ __forceinline__ bool mesh_lights(const DevScene& S) { return !LEAN && S.nlights > 0; }
-template <int LEAN> __device__ __forceinline__ bool env_present(const DevEnv& E) { return LEAN || E.present; }
-template <int LEAN> __device__ __forceinline__ bool grid_on(const DevEnv& E) { return LEAN || E.grid_on; }
-
-// Which frame a path belongs to: one frame (its parameters, film index = path
-// index), or a batch of frames sharing the queues (BatchFrames).
-struct OneFrame {
-  const PassParams* pp;
-  __device__ __forceinline__ void operator()(int g, PathState& P) const {
-    P.pp = pp;
-    P.fidx = g;
-    P.local = g;
-  }
-};
-// Frames of a merged batch pass: frame k holds the paths start[k] .. start[k+1]-1
-// (pixel g - start[k] of that frame), its film at film[k] .. and its parameters
-// at pp[k].
-struct BatchFrames {
-  const int* start;  // n + 1
-  const int* film;   // n
-  const PassParams* pp;
-  int n;
-  __device__ __forceinline__ void operator()(int g, PathState& P) const {
-    int lo = 0, hi = n - 1;  // the last frame with start <= g
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (__ldg(start + mid) <= g) lo = mid;
-      else hi = mid - 1;
-    }
-    P.pp = pp + lo;
-    P.local = g - __ldg(start + lo);
-    P.fidx = __ldg(film + lo) + P.local;
-  }
-};
-
-template <int MODE, int LEAN = 0, class Res = OneFrame>
-__device__ __forceinline__ void shade_hit(const DevScene& S, const DevEnv& E, Res res, int b, const FrameBufs& fb,
-                                          int j, int count, PathState& P) {
-  P.alive = false;
-  P.pixel = 0;
-  P.thr = zero4();
-  P.ps = zero4();
-  P.spec = 0;
-  P.B.mat = -1;
-  if (j >= count) return;
-  float4 qo = __ldg(fb.q_o[(b + 1) & 1] + j);
-  float4 qd = __ldg(fb.q_d[(b + 1) & 1] + j);
-  const int pixel = __float_as_int(qo.w);
-  P.pixel = pixel;
-  res(pixel, P);
-  const PassParams* __restrict__ pp = P.pp;
-  const int kahan = pp->kahan;
-  V o = mk(qo.x, qo.y, qo.z, 0.f), d = mk(qd.x, qd.y, qd.z, 0.f);
-  const float t = fb.hit_t[j];
-  const int prim = fb.hit_prim[j];
-  P.thr = fb.thr[pixel];
-  P.ps = fb.ps[pixel];
-  P.spec = fb.flag[pixel];
-  if (prim >= 0) {
-    hit_record(S, o, d, t, prim, P.H);
-    P.B = setup_bsdf(S, d, P.H.n, P.H.mat);
-    if (P.B.mat >= 0) {
-      const Material& M = S.materials[P.B.mat];
-      if (!LEAN && is_emitter(M)) {  // LightHitPass emitter branch, Render.cl:76-104
-        float pick = 1.f / (float)S.nlights;
-        if (MODE == 1 && E.present && S.nlights > 0) pick = pick * 0.5f;
-        AreaLight L = get_area_light(S, M, prim);
-        float pdfA = 0.f;
-        V c = radiance_area(L, d, &pdfA);
-        if (zero3(c)) {
-          P.alive = true;  // Render.cl:88-89 returns with isect->hit still set
-        } else {
-          float w = 1.f;
-          if (!P.spec) {
-            float pdfW = pdf_a_to_w(pdfA, t, P.B.fix.z);
-            w = mis2(P.ps.w, pdfW * pick);
-          }
-          film_add(fb.film, fb.film_c, P.fidx, muls(mul(P.thr, c), w), kahan);
-        }
-      } else {
-        P.alive = true;
-      }
-    }
-  } else if (env_present<LEAN>(E)) {  // LightHitPass environment branch, Render.cl:106-123
-    float pdfW = 0.f;
-    V c;
-    if (MODE == 1 && grid_on<LEAN>(E))
-      c = radiance_env_grid(E, pp->cam_pos, P.ps, d, &pdfW, pp->grid_accum && !P.spec);
-    else
-      c = radiance_env(E, d, &pdfW);
-    if (!zero3(c)) {
-      if (MODE == 1 && mesh_lights<LEAN>(S)) pdfW = pdfW * 0.5f;
-      float w = 1.f;
-      if (!P.spec) w = mis2(P.ps.w, pdfW);
-      film_add(fb.film, fb.film_c, P.fidx, muls(mul(P.thr, c), w), kahan);
-    }
-  }
-}
-
-// A path that shade_hit kept going (benchmark semantics), loaded again from its
-// queue slot j: the hit record and BSDF set-up are recomputed from the same
-// inputs by the same code, so they equal what shade_hit computed.
-template <class Res>
-__device__ __forceinline__ void shade_load(const DevScene& S, Res res, int b, const FrameBufs& fb, int j,
-                                           PathState& P) {
-  const float4 qo = __ldg(fb.q_o[(b + 1) & 1] + j);
-  const float4 qd = __ldg(fb.q_d[(b + 1) & 1] + j);
-  const int pixel = __float_as_int(qo.w);
-  P.alive = true;
-  P.pixel = pixel;
-  res(pixel, P);
-  const V o = mk(qo.x, qo.y, qo.z, 0.f), d = mk(qd.x, qd.y, qd.z, 0.f);
-  P.thr = fb.thr[pixel];
-  P.ps = fb.ps[pixel];
-  P.spec = fb.flag[pixel];
-  hit_record(S, o, d, __ldg(fb.hit_t + j), __ldg(fb.hit_prim + j), P.H);
-  P.B = setup_bsdf(S, d, P.H.n, P.H.mat);
-}
-
-// gid: the work-item id the samples are keyed on (mode 0: the compacted slot,
-// mode 1: the pixel's id). Writes the path state back; P.alive turns false when
-// Russian roulette ends the path.
-template <int MODE, bool TEX, int LEAN = 0>
-__device__ __forceinline__ void shade_continue(const DevScene& S, const DevEnv& E, int b, const FrameBufs& fb,
-                                               int gid, PathState& P, ShadeOut& R) {
-  const PassParams* __restrict__ pp = P.pp;
-  const float fc = pp->frame_count;
-  R.has_shadow = false;
-  R.ndir = zero4();
-  Bsdf B = P.B;
-  Material tm;  // the path's textured copy of its material
-  if (TEX && has_textures(*B.pm)) {
-    tm = *B.pm;
-    apply_textures(S, B.mat, P.H.u, P.H.v, tm);
-    B.pm = &tm;
-  }
-  int32_t lx, ly, bx, by;
-  if (MODE == 0) {
-    lx = pp->seeds[2 * (2 * b)];
-    ly = pp->seeds[2 * (2 * b) + 1];
-    bx = lx;
-    by = ly;
-  } else {
-    stage_seed(b, 1, &lx, &ly);
-    stage_seed(b, 2, &bx, &by);
-  }
-  Seed s = gen_seed(lx, ly, fc, gid);
-  V dir = zero4();
-  float dist = 0.f, pdfW = 0.f, pick = 1.f;
-  V smp;
-  smp.x = rnd(s);
-  smp.y = rnd(s);
-  smp.z = rnd(s);
-  smp.w = rnd(s);
-  V rad = zero4();
-  bool smesh = false, senv = false;
-  if (env_present<LEAN>(E) && mesh_lights<LEAN>(S)) {
-    float r = rnd(s);
-    pick = pick * 0.5f;
-    if (r < 0.5f) smesh = true; else senv = true;
-  } else if (env_present<LEAN>(E)) {
-    senv = true;
-  } else if (mesh_lights<LEAN>(S)) {
-    smesh = true;
-  }
-  if (smesh) {
-    int li = (int)(rnd(s) * (float)S.nlights);
-    li = li < S.nlights ? li : S.nlights - 1;  // rounding of rnd * n for n > 2^22
-    int tri = S.light_faces[MODE == 0 ? 0 : li];  // Render.cl:305 reads light 0
-    pick = pick * (1.f / (float)S.nlights);
-    const Material& Ml = S.materials[__ldg(reinterpret_cast<const int*>(S.faces + tri) + 9) & 0xFFFF];
-    AreaLight L = get_area_light(S, Ml, tri);
-    rad = illuminate_area(L, P.H.p, smp.x, smp.y, &dir, &dist, &pdfW);
-  } else if (senv) {
-    if (MODE == 1 && grid_on<LEAN>(E))
-      rad = illuminate_env_grid(E, pp->cam_pos, P.H.p, smp, &dir, &dist, &pdfW);
-    else
-      rad = illuminate_env(E, smp, &dir, &dist, &pdfW);
-  }
-  if (!zero3(rad)) {
-    float bpdf = 0.f, cosO = 0.f;
-    V f = eval_bsdf(S, B, dir, &bpdf, &cosO);
-    if (!zero3(f)) {
-      float w = mis2(pdfW, bpdf);
-      float sc = (w * cosO / (pick * pdfW));
-      R.shc = mk(sc * (rad.x * f.x) * P.thr.x, sc * (rad.y * f.y) * P.thr.y, sc * (rad.z * f.z) * P.thr.z, 1.f);
-      R.sho = mk(P.H.p.x, P.H.p.y, P.H.p.z, __int_as_float(P.fidx));
-      R.shd = mk(dir.x, dir.y, dir.z, dist - 2.f * 1e-3f);
-      R.has_shadow = true;
-    }
-  }
-  // BSDF sample
-  Seed s2 = gen_seed(bx, by, fc, gid);
-  float s0 = rnd(s2), s1 = rnd(s2), sz = rnd(s2);
-  float pdf = 0.f, cosO = 0.f;
-  V f = sample_bsdf(S, B, s0, s1, sz, &R.ndir, &pdf, &cosO);
-  float q = cosO / pdf;
-  V thr = mul(P.thr, muls(f, q));
-  V ps = mk(P.H.p.x, P.H.p.y, P.H.p.z, pdf);
-  if (MODE == 1 && pp->rr_depth > 0 && b >= pp->rr_depth) {
-    int32_t rx, ry;
-    stage_seed(b, 3, &rx, &ry);
-    Seed rs = gen_seed(rx, ry, fc, gid);
-    float u = rnd(rs);
-    float mx = maxf_(thr.x, maxf_(thr.y, thr.z));
-    float cont = minf_(0.95f, mx);
-    if (!(u < cont)) P.alive = false;
-    else thr = divs(thr, cont);
-  }
-  fb.thr[P.pixel] = thr;
-  fb.ps[P.pixel] = ps;
-  fb.flag[P.pixel] = 0;
-}
-
-// Benchmark semantics: a warp appends its survivors to the next queue and its
-// shadow rays to the shadow queue, one atomic per queue (ranks by ballot).
-__device__ __forceinline__ void append_warp(Ctrl* ctrl, int b, const FrameBufs& fb, const PathState& P,
-                                            const ShadeOut& R) {
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  const int nq = b & 1;  // queue written for bounce b + 1
-  const unsigned am = __ballot_sync(0xffffffffu, P.alive), sm = __ballot_sync(0xffffffffu, R.has_shadow);
-  int qa = 0, qs = 0;
-  if (lane == 0) {
-    if (am) qa = atomicAdd(&ctrl->count[b + 1], __popc(am));
-    if (sm) qs = atomicAdd(&ctrl->shadow[b], __popc(sm));
-  }
-  qa = __shfl_sync(0xffffffffu, qa, 0);
-  qs = __shfl_sync(0xffffffffu, qs, 0);
-  if (P.alive) {
-    const int slot = qa + __popc(am & lt);
-    fb.q_o[nq][slot] = mk(P.H.p.x, P.H.p.y, P.H.p.z, __int_as_float(P.pixel));
-    fb.q_d[nq][slot] = mk(R.ndir.x, R.ndir.y, R.ndir.z, 0.f);
-  }
-  if (R.has_shadow) {
-    const int sslot = qs + __popc(sm & lt);
-    fb.s_o[sslot] = R.sho;
-    fb.s_d[sslot] = R.shd;
-    fb.s_c[sslot] = R.shc;
-  }
-}
-
-// Reference semantics (mode 0), one 256-path tile per block: survivors are
-// compacted in order (block scan + decoupled look-back) between the two phases,
-// and the light and BSDF samples of a survivor are keyed on its compacted slot
-// as DirectLight and SampleBSDFRayDirection key them on get_global_id; the
-// shadow ray of survivor j' sits at shadow slot j' (pixel -1: none).
-// TEX: the scene has textures (a separate instance keeps the untextured one lean).
-template <int MINB, bool TEX = false>
-__global__ void __launch_bounds__(kShadeThreads, MINB) k_shade_ref(DevScene S, DevEnv E, const PassParams* __restrict__ pp,
-                                                             Ctrl* ctrl, int b, FrameBufs fb,
-                                                             unsigned long long* status) {
-  __shared__ unsigned long long sh[kShadeThreads / 32 + 1];
-  __shared__ int s_tile;
-  __shared__ unsigned long long s_base;
-  const int count = ctrl->count[b];
-  const int ntiles = (count + kShadeThreads - 1) / kShadeThreads;
-  if (threadIdx.x == 0) s_tile = atomicAdd(&ctrl->tiles[b], 1);
-  __syncthreads();
-  const int tile = s_tile;
-  if (tile >= ntiles) return;
-  const int j = tile * kShadeThreads + threadIdx.x;
-  PathState P;
-  shade_hit<0>(S, E, OneFrame{pp}, b, fb, j, count, P);
-  unsigned long long tot = 0;
-  unsigned long long excl = block_rank2<kShadeThreads>(P.alive, false, &tot, sh);
-  if (threadIdx.x == 0) s_base = lookback(status, tile, tot, &ctrl->error);
-  __syncthreads();
-  const int slot = (int)(s_base + excl);
-  if (tile == ntiles - 1 && threadIdx.x == 0) {
-    ctrl->count[b + 1] = (int)(s_base + tot);
-    ctrl->shadow[b] = (int)(s_base + tot);
-  }
-  if (!P.alive) return;
-  ShadeOut R;
-  shade_continue<0, TEX>(S, E, b, fb, slot, P, R);
-  const int nq = b & 1;  // queue written for bounce b + 1
-  fb.q_o[nq][slot] = mk(P.H.p.x, P.H.p.y, P.H.p.z, __int_as_float(P.pixel));
-  fb.q_d[nq][slot] = mk(R.ndir.x, R.ndir.y, R.ndir.z, 0.f);
-  if (R.has_shadow) {
-    fb.s_o[slot] = R.sho;
-    fb.s_d[slot] = R.shd;
-    fb.s_c[slot] = R.shc;
-  } else {
-    fb.s_o[slot] = mk(0.f, 0.f, 0.f, __int_as_float(-1));
-  }
-}
-
-// Benchmark semantics (mode 1): samples are keyed on the pixel, so the order of
-// the queues carries no meaning and no block ever waits for another. Warps run
-// persistently over 32-path chunks (a chunk counter per bounce); each warp
-// appends its survivors and its shadow rays to the next queues with one atomic
-// per queue per chunk (ballot ranks inside the warp). Russian roulette runs after
-// the BSDF sample.
-// Res: OneFrame (pp = the frame's parameters) or BatchFrames (a merged batch pass).
-template <int MINB, bool TEX = false, int LEAN = 0, class Res = OneFrame>
-__global__ void __launch_bounds__(kShadeThreads, MINB) k_shade(DevScene S, DevEnv E, Res res, Ctrl* ctrl, int b,
-                                                         FrameBufs fb) {
-  const int count = ctrl->count[b];
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  const int nq = b & 1;  // queue written for bounce b + 1
-  for (;;) {
-    int chunk = 0;
-    if (lane == 0) chunk = atomicAdd(&ctrl->tiles[b], 1);
-    chunk = __shfl_sync(0xffffffffu, chunk, 0);
-    if (chunk * 32 >= count) break;
-    const int j = chunk * 32 + lane;
-    PathState P;
-    shade_hit<1, LEAN>(S, E, res, b, fb, j, count, P);
-    ShadeOut R;
-    R.has_shadow = false;
-    if (P.alive) shade_continue<1, TEX, LEAN>(S, E, b, fb, pixel_gid(P.local), P, R);
-    const unsigned am = __ballot_sync(0xffffffffu, P.alive), sm = __ballot_sync(0xffffffffu, R.has_shadow);
-    int qa = 0, qs = 0;
-    if (lane == 0) {
-      if (am) qa = atomicAdd(&ctrl->count[b + 1], __popc(am));
-      if (sm) qs = atomicAdd(&ctrl->shadow[b], __popc(sm));
-    }
-    qa = __shfl_sync(0xffffffffu, qa, 0);
-    qs = __shfl_sync(0xffffffffu, qs, 0);
-    if (P.alive) {
-      const int slot = qa + __popc(am & lt);
-      fb.q_o[nq][slot] = mk(P.H.p.x, P.H.p.y, P.H.p.z, __int_as_float(P.pixel));
-      fb.q_d[nq][slot] = mk(R.ndir.x, R.ndir.y, R.ndir.z, 0.f);
-    }
-    if (R.has_shadow) {
-      const int sslot = qs + __popc(sm & lt);
-      fb.s_o[sslot] = R.sho;
-      fb.s_d[sslot] = R.shd;
-      fb.s_c[sslot] = R.shc;
-    }
-  }
-}
-
-// Benchmark semantics in two launches (the default; MT_SHADE_SPLIT=0 runs the
-// single kernel above). k_shade_hit runs the hit record, the BSDF set-up and
-// LightHitPass over the whole queue and lists the slots of the paths that go
-// on; k_shade_cont runs the texture pass, DirectLight, SampleBSDFRayDirection
-// and Russian roulette over that list alone. Each is half the code (less
-// instruction fetch), and the second runs on full warps instead of warps whose
-// terminated paths idle through the light and BSDF samples. Samples are keyed on
-// the pixel, so the list's order carries no meaning.
-template <int MINB, int LEAN = 0, class Res = OneFrame>
-__global__ void __launch_bounds__(kShadeThreads, MINB) k_shade_hit(DevScene S, DevEnv E, Res res, Ctrl* ctrl, int b,
-                                                             FrameBufs fb) {
-  const int count = ctrl->count[b];
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  for (;;) {
-    int chunk = 0;
-    if (lane == 0) chunk = atomicAdd(&ctrl->tiles[b], 1);
-    chunk = __shfl_sync(0xffffffffu, chunk, 0);
-    if (chunk * 32 >= count) break;
-    const int j = chunk * 32 + lane;
-    PathState P;
-    shade_hit<1, LEAN>(S, E, res, b, fb, j, count, P);
-    const unsigned am = __ballot_sync(0xffffffffu, P.alive);
-    int base = 0;
-    if (lane == 0 && am) base = atomicAdd(&ctrl->live[b], __popc(am));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (P.alive) fb.live[base + __popc(am & lt)] = j;
-  }
-}
-
-template <int MINB, bool TEX = false, int LEAN = 0, class Res = OneFrame>
-__global__ void __launch_bounds__(kShadeThreads, MINB) k_shade_cont(DevScene S, DevEnv E, Res res, Ctrl* ctrl, int b,
-                                                              FrameBufs fb) {
-  const int count = ctrl->live[b];
-  const int lane = threadIdx.x & 31;
-  for (;;) {
-    int chunk = 0;
-    if (lane == 0) chunk = atomicAdd(&ctrl->tiles2[b], 1);
-    chunk = __shfl_sync(0xffffffffu, chunk, 0);
-    if (chunk * 32 >= count) break;
-    const int k = chunk * 32 + lane;
-    PathState P;
-    P.alive = false;
-    ShadeOut R;
-    R.has_shadow = false;
-    if (k < count) {
-      shade_load(S, res, b, fb, __ldg(fb.live + k), P);
-      shade_continue<1, TEX, LEAN>(S, E, b, fb, pixel_gid(P.local), P, R);
-    }
-    append_warp(ctrl, b, fb, P, R);
-  }
-}
-
 // Adds a finished pass's ray counts into the job's running totals
 // [primary, extension, shadow].
 __global__ void k_accumulate(const Ctrl* ctrl, int max_depth, int n_pixels, unsigned long long* totals) {
@@ -664,15 +196,6 @@ int shadow_grid_bps() { return tuning_ref().shadow_grid; }
 int trace_minb() { return tuning_ref().closest_minb; }
 int shadow_minb() { return tuning_ref().shadow_minb; }
 int shade_minb() { return tuning_ref().shade_minb; }
-// Resident blocks per SM of the benchmark-semantics shading kernel (its grid is
-// one resident wave of persistent warps).
-int shade_blocks_per_sm(int minb) {
-  int n = 0;
-  if (minb == 4) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_shade<4>, kShadeThreads, 0);
-  else if (minb == 5) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_shade<5>, kShadeThreads, 0);
-  else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_shade<3>, kShadeThreads, 0);
-  return n > 0 ? n : 1;
-}
 template <int MINB>
 int trace_blocks_per_sm() {
   int n = 0;
@@ -785,7 +308,6 @@ int launch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const PassP
                 cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, int shade_split_req, int min_lanes) {
   const bool two_launches = shade_split_req < 0 ? shade_split() : shade_split_req != 0;
   const int N = width * height;
-  static int shade_bps[6] = {};
   // shadow rays of bounce b beside the extension rays of bounce b + 1 (no
   // per-kernel events): both read only what shading b wrote (in reference
   // semantics both read its survivor count), and shading b + 1, which rewrites
@@ -796,7 +318,6 @@ int launch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const PassP
   auto trace = [&](bool closest, int b) { launch_trace(st, S, ctrl, b, mode, fb, kahan, closest, N, num_sms, shared, min_lanes); };
   // persistent traversal: one resident wave, or fewer blocks for a small frame
   // (a queue never exceeds the frame's pixels), leaving SMs to other streams
-  const int tiles = (N + kShadeThreads - 1) / kShadeThreads;
   int e = 0;
   if (ev) cudaEventRecord(ev[e++], st);
   k_raygen<<<(N + 255) / 256, 256, 0, st>>>(d_pp, ctrl, fb);
@@ -806,47 +327,8 @@ int launch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const PassP
     if (ev) cudaEventRecord(ev[e++], st);
     if (split && b > 1) cudaStreamWaitEvent(st, join, 0);
     unsigned long long* stb = status + (size_t)(b - 1) * status_stride;
-    if (mode == 0) {
-      if (S.tex_on)
-        k_shade_ref<3, true><<<tiles, kShadeThreads, 0, st>>>(S, E, d_pp, ctrl, b, fb, stb);
-      else
-        k_shade_ref<3><<<tiles, kShadeThreads, 0, st>>>(S, E, d_pp, ctrl, b, fb, stb);
-    } else if (two_launches) {
-      const int sm = shade_minb();
-      if (shade_bps[sm] == 0) shade_bps[sm] = shade_blocks_per_sm(sm);
-      const int sgrid = std::max(1, std::min(num_sms * shade_bps[sm], tiles));
-      const bool lean = S.nlights == 0 && E.present && E.grid_on && !S.tex_on;
-      const OneFrame R1{d_pp};
-      if (lean)
-        k_shade_hit<4, 1><<<sgrid, kShadeThreads, 0, st>>>(S, E, R1, ctrl, b, fb);
-      else
-        k_shade_hit<4><<<sgrid, kShadeThreads, 0, st>>>(S, E, R1, ctrl, b, fb);
-      if (S.tex_on)
-        k_shade_cont<4, true><<<sgrid, kShadeThreads, 0, st>>>(S, E, R1, ctrl, b, fb);
-      else if (lean && sm == 4)
-        k_shade_cont<4, false, 1><<<sgrid, kShadeThreads, 0, st>>>(S, E, R1, ctrl, b, fb);
-      else if (sm == 4)
-        k_shade_cont<4><<<sgrid, kShadeThreads, 0, st>>>(S, E, R1, ctrl, b, fb);
-      else if (sm == 5)
-        k_shade_cont<5><<<sgrid, kShadeThreads, 0, st>>>(S, E, R1, ctrl, b, fb);
-      else
-        k_shade_cont<3><<<sgrid, kShadeThreads, 0, st>>>(S, E, R1, ctrl, b, fb);
-    } else {
-      const int sm = shade_minb();
-      if (shade_bps[sm] == 0) shade_bps[sm] = shade_blocks_per_sm(sm);
-      const int sgrid = std::max(1, std::min(num_sms * shade_bps[sm], tiles));
-      const bool lean = S.nlights == 0 && E.present && E.grid_on;
-      if (S.tex_on)
-        k_shade<4, true><<<sgrid, kShadeThreads, 0, st>>>(S, E, OneFrame{d_pp}, ctrl, b, fb);
-      else if (lean && sm == 4)
-        k_shade<4, false, 1><<<sgrid, kShadeThreads, 0, st>>>(S, E, OneFrame{d_pp}, ctrl, b, fb);
-      else if (sm == 4)
-        k_shade<4><<<sgrid, kShadeThreads, 0, st>>>(S, E, OneFrame{d_pp}, ctrl, b, fb);
-      else if (sm == 5)
-        k_shade<5><<<sgrid, kShadeThreads, 0, st>>>(S, E, OneFrame{d_pp}, ctrl, b, fb);
-      else
-        k_shade<3><<<sgrid, kShadeThreads, 0, st>>>(S, E, OneFrame{d_pp}, ctrl, b, fb);
-    }
+    if (mode == 0) launch_shade_ref(st, S, E, d_pp, N, ctrl, b, fb, stb);
+    else launch_shade(st, S, E, d_pp, two_launches, shade_minb(), num_sms, N, ctrl, b, fb);
     if (ev) cudaEventRecord(ev[e++], st);
     if (split) {
       cudaEventRecord(fork, st);
@@ -881,23 +363,10 @@ int launch_batch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const
                       const PassParams* d_pp, int nframes, int total, int max_depth, int kahan, Ctrl* ctrl,
                       FrameBufs fb, int num_sms, unsigned long long* totals, bool shared, int min_lanes) {
   const BatchFrames B{d_start, d_film, d_pp, nframes};
-  static int shade_bps = 0;
-  if (shade_bps == 0) shade_bps = shade_blocks_per_sm(4);
-  const int tiles = (total + kShadeThreads - 1) / kShadeThreads;
-  const int sgrid = std::max(1, std::min(num_sms * shade_bps, tiles));
   k_raygen_batch<<<(total + 255) / 256, 256, 0, st>>>(B, total, ctrl, fb);
   for (int b = 1; b <= max_depth; ++b) {
     launch_trace(st, S, ctrl, b, 1, fb, kahan, true, total, num_sms, shared, min_lanes);
-    if (shade_split()) {
-      k_shade_hit<4, 0, BatchFrames><<<sgrid, kShadeThreads, 0, st>>>(S, E, B, ctrl, b, fb);
-      if (S.tex_on)
-        k_shade_cont<4, true, 0, BatchFrames><<<sgrid, kShadeThreads, 0, st>>>(S, E, B, ctrl, b, fb);
-      else
-        k_shade_cont<4, false, 0, BatchFrames><<<sgrid, kShadeThreads, 0, st>>>(S, E, B, ctrl, b, fb);
-    } else if (S.tex_on)
-      k_shade<4, true, 0, BatchFrames><<<sgrid, kShadeThreads, 0, st>>>(S, E, B, ctrl, b, fb);
-    else
-      k_shade<4, false, 0, BatchFrames><<<sgrid, kShadeThreads, 0, st>>>(S, E, B, ctrl, b, fb);
+    launch_shade_batch(st, S, E, d_start, d_film, d_pp, nframes, shade_split(), num_sms, total, ctrl, b, fb);
     launch_trace(st, S, ctrl, b, 1, fb, kahan, false, total, num_sms, shared, min_lanes);
   }
   if (totals) k_accumulate<<<1, 32, 0, st>>>(ctrl, max_depth, total, totals);

@@ -69,6 +69,16 @@ int launch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const PassP
                 unsigned long long* status, size_t status_stride, int num_sms, cudaEvent_t* events,
                 unsigned long long* totals, bool shared = false, cudaStream_t side = nullptr,
                 cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr, int shade_split = -1, int min_lanes = 1);
+// Shading of one bounce (mt_shade.cu): reference semantics; benchmark semantics of
+// one frame (in one launch or two) and of a merged batch pass. N, total: paths a
+// queue holds at most.
+void launch_shade_ref(cudaStream_t st, const DevScene& S, const DevEnv& E, const PassParams* pp, int N, Ctrl* ctrl, int b,
+                      FrameBufs fb, unsigned long long* status);
+void launch_shade(cudaStream_t st, const DevScene& S, const DevEnv& E, const PassParams* pp, bool two, int minb,
+                  int num_sms, int N, Ctrl* ctrl, int b, FrameBufs fb);
+void launch_shade_batch(cudaStream_t st, const DevScene& S, const DevEnv& E, const int* d_start, const int* d_film,
+                        const PassParams* d_pp, int nframes, bool two, int num_sms, int total, Ctrl* ctrl, int b,
+                        FrameBufs fb);
 // The process's benchmark-semantics shading setting (MT_SHADE_SPLIT): -1 render
 // jobs choose per frame (shade_split_for) and other passes run two launches; 0
 // always one launch; 1 always two.

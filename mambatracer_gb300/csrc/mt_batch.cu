@@ -19,23 +19,21 @@
 namespace {
 
 void free_bufs(FrameBufs& fb) {
-  for (auto* p : {&fb.q_o[0], &fb.q_o[1], &fb.q_d[0], &fb.q_d[1], &fb.thr, &fb.ps, &fb.s_o, &fb.s_d, &fb.s_c,
+  for (auto* p : {&fb.q_o[0], &fb.q_o[1], &fb.q_d[0], &fb.q_d[1], &fb.q_t[0], &fb.q_t[1], &fb.s_o, &fb.s_d, &fb.s_c,
                   &fb.film, &fb.film_c})
     dfree(*p);
   dfree(fb.hit_t);
   dfree(fb.hit_prim);
-  dfree(fb.flag);
   dfree(fb.live);
 }
 
 int alloc_bufs(FrameBufs& fb, size_t n) {
   int r = MT_OK;
-  for (auto* p : {&fb.q_o[0], &fb.q_o[1], &fb.q_d[0], &fb.q_d[1], &fb.thr, &fb.ps, &fb.s_o, &fb.s_d, &fb.s_c,
+  for (auto* p : {&fb.q_o[0], &fb.q_o[1], &fb.q_d[0], &fb.q_d[1], &fb.q_t[0], &fb.q_t[1], &fb.s_o, &fb.s_d, &fb.s_c,
                   &fb.film, &fb.film_c})
     if (!r) r = dalloc(p, n);
   if (!r) r = dalloc(&fb.hit_t, n);
   if (!r) r = dalloc(&fb.hit_prim, n);
-  if (!r) r = dalloc(&fb.flag, n);
   if (!r) r = dalloc(&fb.live, n);
   return r;
 }

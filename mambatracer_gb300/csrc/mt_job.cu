@@ -91,12 +91,10 @@ void free_slot(JobSlot& s) {
   for (int k = 0; k < 2; ++k) {
     dfree(s.fb.q_o[k]);
     dfree(s.fb.q_d[k]);
+    dfree(s.fb.q_t[k]);
   }
   dfree(s.fb.hit_t);
   dfree(s.fb.hit_prim);
-  dfree(s.fb.thr);
-  dfree(s.fb.ps);
-  dfree(s.fb.flag);
   dfree(s.fb.s_o);
   dfree(s.fb.s_d);
   dfree(s.fb.s_c);
@@ -174,12 +172,10 @@ int alloc_slot(JobSlot& s, size_t N, int spp, int max_depth, size_t status_strid
   for (int k = 0; k < 2 && !r; ++k) {
     r = dalloc(&s.fb.q_o[k], N);
     if (!r) r = dalloc(&s.fb.q_d[k], N);
+    if (!r) r = dalloc(&s.fb.q_t[k], N);
   }
   if (!r) r = dalloc(&s.fb.hit_t, N);
   if (!r) r = dalloc(&s.fb.hit_prim, N);
-  if (!r) r = dalloc(&s.fb.thr, N);
-  if (!r) r = dalloc(&s.fb.ps, N);
-  if (!r) r = dalloc(&s.fb.flag, N);
   if (!r) r = dalloc(&s.fb.s_o, N);
   if (!r) r = dalloc(&s.fb.s_d, N);
   if (!r) r = dalloc(&s.fb.s_c, N);

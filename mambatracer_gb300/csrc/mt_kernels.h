@@ -9,12 +9,10 @@ namespace mt {
 // Per-job frame buffers (structure of arrays).
 struct FrameBufs {
   float4* q_o[2];   // ray queue: origin.xyz, bits(pixel)  (ping-pong by bounce parity)
-  float4* q_d[2];   // ray queue: direction.xyz, 0
+  float4* q_d[2];   // ray queue: direction.xyz, lastPdfW
+  float4* q_t[2];   // ray queue: throughput (4 lanes as the reference); bounce 1 has none
   float* hit_t;     // closest-hit distance per queue slot
   int* hit_prim;    // closest-hit face id per queue slot (-1 = miss)
-  float4* thr;      // path throughput per pixel (4 lanes as the reference)
-  float4* ps;       // path: hitpoint.xyz, lastPdfW
-  int* flag;        // path: lastSpecular
   float4* s_o;      // shadow queue: origin.xyz, bits(pixel or -1)
   float4* s_d;      // shadow queue: direction.xyz, tMax
   float4* s_c;      // shadow queue: contribution.xyz

@@ -171,9 +171,8 @@ void free_lane(Lane& L) {
   }
   dfree(L.fb.hit_t);
   dfree(L.fb.hit_prim);
-  dfree(L.fb.thr);
-  dfree(L.fb.ps);
-  dfree(L.fb.flag);
+  dfree(L.fb.q_t[0]);
+  dfree(L.fb.q_t[1]);
   dfree(L.fb.s_o);
   dfree(L.fb.s_d);
   dfree(L.fb.s_c);
@@ -205,9 +204,8 @@ int alloc_lane(Lane& L, size_t N, int spp, int depth, size_t stride) {
   }
   if (!r) r = dalloc(&L.fb.hit_t, N);
   if (!r) r = dalloc(&L.fb.hit_prim, N);
-  if (!r) r = dalloc(&L.fb.thr, N);
-  if (!r) r = dalloc(&L.fb.ps, N);
-  if (!r) r = dalloc(&L.fb.flag, N);
+  if (!r) r = dalloc(&L.fb.q_t[0], N);
+  if (!r) r = dalloc(&L.fb.q_t[1], N);
   if (!r) r = dalloc(&L.fb.s_o, N);
   if (!r) r = dalloc(&L.fb.s_d, N);
   if (!r) r = dalloc(&L.fb.s_c, N);
@@ -272,12 +270,11 @@ void release_scene(Request* R) {
 }
 
 void free_merged(mt_server* s) {
-  for (auto* p : {&s->mfb.q_o[0], &s->mfb.q_o[1], &s->mfb.q_d[0], &s->mfb.q_d[1], &s->mfb.thr, &s->mfb.ps,
+  for (auto* p : {&s->mfb.q_o[0], &s->mfb.q_o[1], &s->mfb.q_d[0], &s->mfb.q_d[1], &s->mfb.q_t[0], &s->mfb.q_t[1],
                   &s->mfb.s_o, &s->mfb.s_d, &s->mfb.s_c, &s->mfb.film, &s->mfb.film_c})
     dfree(*p);
   dfree(s->mfb.hit_t);
   dfree(s->mfb.hit_prim);
-  dfree(s->mfb.flag);
   dfree(s->mfb.live);
   for (MergeGroup& G : s->groups) {
     for (Round& Rd : G.rounds) {
@@ -311,12 +308,11 @@ int alloc_merged(mt_server* s, size_t N, int m) {
     s->groups[k % m].slots.push_back(k);
   }
   int r = MT_OK;
-  for (auto* p : {&s->mfb.q_o[0], &s->mfb.q_o[1], &s->mfb.q_d[0], &s->mfb.q_d[1], &s->mfb.thr, &s->mfb.ps,
+  for (auto* p : {&s->mfb.q_o[0], &s->mfb.q_o[1], &s->mfb.q_d[0], &s->mfb.q_d[1], &s->mfb.q_t[0], &s->mfb.q_t[1],
                   &s->mfb.s_o, &s->mfb.s_d, &s->mfb.s_c, &s->mfb.film, &s->mfb.film_c})
     if (!r) r = dalloc(p, P);
   if (!r) r = dalloc(&s->mfb.hit_t, P);
   if (!r) r = dalloc(&s->mfb.hit_prim, P);
-  if (!r) r = dalloc(&s->mfb.flag, P);
   if (!r) r = dalloc(&s->mfb.live, P);
   for (Lane& L : s->lanes)
     if (!r && cudaMallocHost((void**)&L.h_stage, sizeof(float4) * N) != cudaSuccess)
@@ -343,12 +339,10 @@ int alloc_merged(mt_server* s, size_t N, int m) {
     for (int q = 0; q < 2; ++q) {
       G.fb.q_o[q] += base;
       G.fb.q_d[q] += base;
+      G.fb.q_t[q] += base;
     }
     G.fb.hit_t += base;
     G.fb.hit_prim += base;
-    G.fb.thr += base;
-    G.fb.ps += base;
-    G.fb.flag += base;
     G.fb.s_o += base;
     G.fb.s_d += base;
     G.fb.s_c += base;

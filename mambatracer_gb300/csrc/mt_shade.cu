@@ -34,7 +34,8 @@ __device__ __forceinline__ void append_warp(Ctrl* ctrl, int b, const FrameBufs& 
   if (P.alive) {
     const int slot = qa + __popc(am & lt);
     fb.q_o[nq][slot] = mk(P.H.p.x, P.H.p.y, P.H.p.z, __int_as_float(P.pixel));
-    fb.q_d[nq][slot] = mk(R.ndir.x, R.ndir.y, R.ndir.z, 0.f);
+    fb.q_d[nq][slot] = mk(R.ndir.x, R.ndir.y, R.ndir.z, P.ps.w);
+    fb.q_t[nq][slot] = P.thr;
   }
   if (R.has_shadow) {
     const int sslot = qs + __popc(sm & lt);
@@ -80,7 +81,8 @@ __global__ void __launch_bounds__(kShadeThreads, MINB) k_shade_ref(DevScene S, D
   shade_continue<0, TEX, L>(S, E, b, fb, slot, P, R);
   const int nq = b & 1;  // queue written for bounce b + 1
   fb.q_o[nq][slot] = mk(P.H.p.x, P.H.p.y, P.H.p.z, __int_as_float(P.pixel));
-  fb.q_d[nq][slot] = mk(R.ndir.x, R.ndir.y, R.ndir.z, 0.f);
+  fb.q_d[nq][slot] = mk(R.ndir.x, R.ndir.y, R.ndir.z, P.ps.w);
+  fb.q_t[nq][slot] = P.thr;
   if (R.has_shadow) {
     fb.s_o[slot] = R.sho;
     fb.s_d[slot] = R.shd;
@@ -126,7 +128,8 @@ __global__ void __launch_bounds__(kShadeThreads, MINB) k_shade(DevScene S, DevEn
     if (P.alive) {
       const int slot = qa + __popc(am & lt);
       fb.q_o[nq][slot] = mk(P.H.p.x, P.H.p.y, P.H.p.z, __int_as_float(P.pixel));
-      fb.q_d[nq][slot] = mk(R.ndir.x, R.ndir.y, R.ndir.z, 0.f);
+      fb.q_d[nq][slot] = mk(R.ndir.x, R.ndir.y, R.ndir.z, P.ps.w);
+      fb.q_t[nq][slot] = P.thr;
     }
     if (R.has_shadow) {
       const int sslot = qs + __popc(sm & lt);

@@ -51,13 +51,11 @@ __device__ __forceinline__ void camera_ray(const PassParams* __restrict__ pp, in
   *o_out = o;
   *d_out = dw;
 }
-// Queue slot and path state g of a new path (InitPathData).
+// Queue slot g of a new path. Its state is InitPathData's constants, which bounce 1
+// knows (queue_state).
 __device__ __forceinline__ void start_path(FrameBufs& fb, int g, V o, V dw) {
   fb.q_o[0][g] = mk(o.x, o.y, o.z, __int_as_float(g));
-  fb.q_d[0][g] = mk(dw.x, dw.y, dw.z, 0.f);
-  fb.thr[g] = mk(1.f, 1.f, 1.f, 1.f);
-  fb.ps[g] = mk(0.f, 0.f, 0.f, 1.f);  // hitpoint.xyz, lastPdfW
-  fb.flag[g] = 1;                     // lastSpecular
+  fb.q_d[0][g] = mk(dw.x, dw.y, dw.z, 1.f);
 }
 
 // ----------------------------------------------------------------- shade
@@ -69,12 +67,14 @@ __device__ __forceinline__ void start_path(FrameBufs& fb, int g, V o, V dw) {
 //                   Russian roulette in benchmark semantics.
 struct PathState {
   bool alive;
-  int pixel;                // queue slot's path index (path state)
+  int slot;                 // its queue slot
+  int pixel;                // its path index: which pixel of which frame
   int fidx;                 // film index of its pixel
   int local;                // its pixel within its frame (the samples' key)
   const PassParams* pp;     // its frame's parameters
-  V thr, ps;
-  int spec;
+  V thr;                    // throughput (from shade_continue on)
+  V ps;                     // hitpoint.xyz of the last bounce, lastPdfW
+  int spec;                 // lastSpecular: only the camera's ray
   Hit H;
   Bsdf B;
 };
@@ -133,12 +133,23 @@ struct BatchFrames {
   }
 };
 
+// A path's state in queue slot j at bounce b. It travels with the queue (q_d.w the
+// last pdf, q_t the throughput; the last hitpoint is the ray's origin), so a bounce
+// reads and writes it in slot order; bounce 1 starts from InitPathData's constants.
+__device__ __forceinline__ void queue_state(int b, float4 qo, float4 qd, PathState& P) {
+  P.ps = b == 1 ? mk(0.f, 0.f, 0.f, 1.f) : mk(qo.x, qo.y, qo.z, qd.w);
+  P.spec = b == 1;
+}
+__device__ __forceinline__ V queue_thr(const FrameBufs& fb, int b, int j) {
+  return b == 1 ? mk(1.f, 1.f, 1.f, 1.f) : __ldg(fb.q_t[(b + 1) & 1] + j);
+}
+
 template <int MODE, int L = kAnyLights, class Res = OneFrame>
 __device__ __forceinline__ void shade_hit(const DevScene& S, const DevEnv& E, Res res, int b, const FrameBufs& fb,
                                           int j, int count, PathState& P) {
   P.alive = false;
+  P.slot = j;
   P.pixel = 0;
-  P.thr = zero4();
   P.ps = zero4();
   P.spec = 0;
   P.B.mat = -1;
@@ -153,9 +164,7 @@ __device__ __forceinline__ void shade_hit(const DevScene& S, const DevEnv& E, Re
   V o = mk(qo.x, qo.y, qo.z, 0.f), d = mk(qd.x, qd.y, qd.z, 0.f);
   const float t = fb.hit_t[j];
   const int prim = fb.hit_prim[j];
-  P.thr = fb.thr[pixel];
-  P.ps = fb.ps[pixel];
-  P.spec = fb.flag[pixel];
+  queue_state(b, qo, qd, P);
   if (prim >= 0) {
     hit_record(S, o, d, t, prim, P.H);
     P.B = setup_bsdf(S, d, P.H.n, P.H.mat);
@@ -175,7 +184,7 @@ __device__ __forceinline__ void shade_hit(const DevScene& S, const DevEnv& E, Re
             float pdfW = pdf_a_to_w(pdfA, t, P.B.fix.z);
             w = mis2(P.ps.w, pdfW * pick);
           }
-          film_add(fb.film, fb.film_c, P.fidx, muls(mul(P.thr, c), w), kahan);
+          film_add(fb.film, fb.film_c, P.fidx, muls(mul(queue_thr(fb, b, j), c), w), kahan);
         }
       } else {
         P.alive = true;
@@ -192,7 +201,7 @@ __device__ __forceinline__ void shade_hit(const DevScene& S, const DevEnv& E, Re
       if (MODE == 1 && mesh_lights<L>(S)) pdfW = pdfW * 0.5f;
       float w = 1.f;
       if (!P.spec) w = mis2(P.ps.w, pdfW);
-      film_add(fb.film, fb.film_c, P.fidx, muls(mul(P.thr, c), w), kahan);
+      film_add(fb.film, fb.film_c, P.fidx, muls(mul(queue_thr(fb, b, j), c), w), kahan);
     }
   }
 }
@@ -207,24 +216,23 @@ __device__ __forceinline__ void shade_load(const DevScene& S, Res res, int b, co
   const float4 qd = __ldg(fb.q_d[(b + 1) & 1] + j);
   const int pixel = __float_as_int(qo.w);
   P.alive = true;
+  P.slot = j;
   P.pixel = pixel;
   res(pixel, P);
   const V o = mk(qo.x, qo.y, qo.z, 0.f), d = mk(qd.x, qd.y, qd.z, 0.f);
-  P.thr = fb.thr[pixel];
-  P.ps = fb.ps[pixel];
-  P.spec = fb.flag[pixel];
   hit_record(S, o, d, __ldg(fb.hit_t + j), __ldg(fb.hit_prim + j), P.H);
   P.B = setup_bsdf(S, d, P.H.n, P.H.mat);
 }
 
 // gid: the work-item id the samples are keyed on (mode 0: the compacted slot,
-// mode 1: the pixel's id). Writes the path state back; P.alive turns false when
+// mode 1: the pixel's id). P ends with the next bounce's state; P.alive turns false when
 // Russian roulette ends the path.
 template <int MODE, bool TEX, int L = kAnyLights>
 __device__ __forceinline__ void shade_continue(const DevScene& S, const DevEnv& E, int b, const FrameBufs& fb,
                                                int gid, PathState& P, ShadeOut& R) {
   const PassParams* __restrict__ pp = P.pp;
   const float fc = pp->frame_count;
+  P.thr = queue_thr(fb, b, P.slot);
   R.has_shadow = false;
   R.ndir = zero4();
   Bsdf B = P.B;
@@ -310,7 +318,6 @@ __device__ __forceinline__ void shade_continue(const DevScene& S, const DevEnv& 
   f = sample_end(B, ds, f, &R.ndir, &cosO);
   float q = cosO / pdf;
   V thr = mul(P.thr, muls(f, q));
-  V ps = mk(P.H.p.x, P.H.p.y, P.H.p.z, pdf);
   if (MODE == 1 && pp->rr_depth > 0 && b >= pp->rr_depth) {
     int32_t rx, ry;
     stage_seed(b, 3, &rx, &ry);
@@ -321,9 +328,8 @@ __device__ __forceinline__ void shade_continue(const DevScene& S, const DevEnv& 
     if (!(u < cont)) P.alive = false;
     else thr = divs(thr, cont);
   }
-  fb.thr[P.pixel] = thr;
-  fb.ps[P.pixel] = ps;
-  fb.flag[P.pixel] = 0;
+  P.thr = thr;
+  P.ps.w = pdf;
 }
 
 }  // namespace mt

@@ -39,7 +39,10 @@ __global__ void __launch_bounds__(kCompactThreads)
   if (i < n) keep = __ldg(reinterpret_cast<const int*>(in + 6 * (size_t)i) + 20) != 0;
   unsigned long long tot;
   const unsigned long long excl = block_rank2<kCompactThreads>(keep, false, &tot, sh);
-  if (threadIdx.x == 0) s_excl = lookback(status, tile, tot, err);
+  if (threadIdx.x < 32) {
+    const unsigned long long e = lookback(status, tile, tot, err);
+    if (threadIdx.x == 0) s_excl = e;
+  }
   __syncthreads();
   const int b0 = *base;
   if (keep) {

@@ -28,33 +28,43 @@ __device__ __forceinline__ void st_release(unsigned long long* p, unsigned long 
 }
 
 // Decoupled look-back over tile aggregates (single-pass stable compaction).
-// Returns the exclusive prefix of `tile`. Every wait is bounded: after
-// kSpinLimit polls the error is latched and the partial prefix is used.
+// Called by one whole warp; returns the exclusive prefix of `tile`. The warp reads
+// 32 tiles before it at a time (one dependent read of L2 each, tiles finishing side
+// by side would otherwise walk over one another's aggregates one by one). Every
+// wait is bounded: after kSpinLimit polls the error is latched and the partial
+// prefix is used.
 __device__ __forceinline__ unsigned long long lookback(unsigned long long* status, int tile, unsigned long long agg, int* err) {
+  const int lane = threadIdx.x & 31;
   if (tile == 0) {
-    st_release(&status[0], kFlagPfx | agg);
+    if (lane == 0) st_release(&status[0], kFlagPfx | agg);
     return 0;
   }
-  st_release(&status[tile], kFlagAgg | agg);
+  if (lane == 0) st_release(&status[tile], kFlagAgg | agg);
   unsigned long long excl = 0;
-  int t = tile - 1;
-  while (t >= 0) {
-    unsigned long long s = 0;
+  for (int t = tile - 1; t >= 0; t -= 32) {
+    const int mine = t - lane;  // lane 0 the nearest
+    unsigned long long s = kFlagPfx;  // before the first tile: an empty prefix
     int it = 0;
-    for (; it < kSpinLimit; ++it) {
-      s = ld_acquire(&status[t]);
-      if (s >> 62) break;
-      __nanosleep(32);
-    }
-    if (it == kSpinLimit) {
-      atomicExch(err, kDevErrLookback);
+    if (mine >= 0)
+      for (; it < kSpinLimit; ++it) {
+        s = ld_acquire(&status[mine]);
+        if (s >> 62) break;
+        __nanosleep(32);
+      }
+    if (__any_sync(0xffffffffu, it == kSpinLimit)) {
+      if (lane == 0) atomicExch(err, kDevErrLookback);
       break;
     }
-    excl += s & kValMask;
-    if ((s >> 62) == 2) break;
-    --t;
+    // the nearest complete prefix ends the walk
+    const unsigned pfx = __ballot_sync(0xffffffffu, (s >> 62) == 2);
+    const int last = pfx ? __ffs(pfx) - 1 : 31;
+    unsigned long long v = lane <= last ? s & kValMask : 0ull;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    excl += v;
+    if (pfx) break;
   }
-  st_release(&status[tile], kFlagPfx | (excl + agg));
+  if (lane == 0) st_release(&status[tile], kFlagPfx | (excl + agg));
   return excl;
 }
 

@@ -69,7 +69,10 @@ __global__ void __launch_bounds__(kShadeThreads, MINB) k_shade_ref(DevScene S, D
   shade_hit<0, L>(S, E, OneFrame{pp}, b, fb, j, count, P);
   unsigned long long tot = 0;
   unsigned long long excl = block_rank2<kShadeThreads>(P.alive, false, &tot, sh);
-  if (threadIdx.x == 0) s_base = lookback(status, tile, tot, &ctrl->error);
+  if (threadIdx.x < 32) {
+    const unsigned long long base = lookback(status, tile, tot, &ctrl->error);
+    if (threadIdx.x == 0) s_base = base;
+  }
   __syncthreads();
   const int slot = (int)(s_base + excl);
   if (tile == ntiles - 1 && threadIdx.x == 0) {
@@ -262,7 +265,7 @@ void launch_shade_ref(cudaStream_t st, const DevScene& S, const DevEnv& E, const
   else if (S.tex_on)
     k_shade_ref<3, true><<<tiles, kShadeThreads, 0, st>>>(S, E, pp, ctrl, b, fb, status);
   else if (l == kMeshLights)
-    k_shade_ref<3, false, kMeshLights><<<tiles, kShadeThreads, 0, st>>>(S, E, pp, ctrl, b, fb, status);
+    k_shade_ref<4, false, kMeshLights><<<tiles, kShadeThreads, 0, st>>>(S, E, pp, ctrl, b, fb, status);
   else if (l == kMapLights)
     k_shade_ref<3, false, kMapLights><<<tiles, kShadeThreads, 0, st>>>(S, E, pp, ctrl, b, fb, status);
   else

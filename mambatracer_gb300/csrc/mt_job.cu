@@ -384,7 +384,7 @@ int enqueue_frame(mt_job* j, JobSlot& s) {
     cudaEvent_t* ev = j->kev.empty() ? nullptr : j->kev.data() + per_pass_events * p;
     if (launch_pass(s.stream, S, E, s.d_pp + p, c.mode, c.max_depth, c.film_kahan, c.width, c.height, s.d_ctrl + p,
                     s.fb, s.d_status + j->status_stride * (size_t)c.max_depth * p, j->status_stride, ctx->num_sms,
-                    ev, j->d_totals, j->nslots > 1, s.side, s.sfork, s.sjoin, j->shade_split, tail_lanes(j->nslots)))
+                    ev, j->d_totals, j->nslots > 1, s.side, s.sfork, s.sjoin, j->shade_split != 0, tail_lanes(j->nslots)))
       return fail(MT_ERR_CUDA, "pass launch: %s", cudaGetErrorString(cudaGetLastError()));
   }
   return MT_OK;
@@ -430,6 +430,8 @@ extern "C" int mt_render_frame(mt_job* j, const int32_t* seeds, float frame_coun
   const int split_setting = shade_split_setting();
   if (split_setting >= 0) {
     j->shade_split = split_setting;
+  } else if (j->nslots == 1 && c.width * c.height < kSplitPaths) {
+    j->shade_split = 0;
   } else if (c.mode == 1 && c.max_depth >= 2) {
     // One launch or two for the shading of the next frames: a finished frame's
     // share of bounce-1 paths that went on decides (shade_split_for): this slot's
@@ -474,7 +476,7 @@ extern "C" int mt_render_frame(mt_job* j, const int32_t* seeds, float frame_coun
   CU(cudaEventRecord(s.ev0, s.stream));
   if (c.use_graph && !c.profile) {
     const int form = j->shade_split == 0 ? 0 : 1;
-    const bool both = split_setting < 0 && c.mode == 1;  // the job may switch forms later
+    const bool both = split_setting < 0 && c.mode == 1 && (j->nslots > 1 || c.width * c.height >= kSplitPaths);  // may switch later
     for (int f = 0; f < 2; ++f) {
       if (s.graphs[f] || (f != form && !both)) continue;
       const int keep = j->shade_split;
@@ -499,7 +501,7 @@ extern "C" int mt_render_frame(mt_job* j, const int32_t* seeds, float frame_coun
   {
     // per pass: raygen, per bounce closest hits + shading (one launch or two) +
     // shadow rays, the ray totals; then the film merge
-    const int two = c.mode == 1 && (j->shade_split < 0 ? shade_split_setting() != 0 : j->shade_split != 0);
+    const int two = c.mode == 1 && j->shade_split != 0;
     j->launches += (int64_t)c.spp * (2 + (int64_t)c.max_depth * (3 + two)) + (j->nslots > 1 ? 1 : 0);
   }
   CU(cudaEventRecord(s.ev1, s.stream));

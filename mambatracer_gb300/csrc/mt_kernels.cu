@@ -166,7 +166,7 @@ int env_shade_minb() {
   return (x == 3 || x == 4 || x == 5) ? x : kShadeMinBlocks;
 }
 // MT_SHADE_SPLIT: unset, render jobs choose one or two shading launches frame by
-// frame (shade_split_for) and other passes take two; 0 always one; 1 always two.
+// frame (shade_split_for) and other passes by their size; 0 always one; 1 always two.
 int shade_split_mode() {
   static const int m = [] {
     const char* e = std::getenv("MT_SHADE_SPLIT");
@@ -175,7 +175,7 @@ int shade_split_mode() {
   }();
   return m;
 }
-bool shade_split() { return shade_split_mode() != 0; }
+bool shade_split(int n) { return shade_split_mode() < 0 ? n >= kSplitPaths : shade_split_mode() != 0; }
 
 int env_steps() {
   const char* e = std::getenv("MT_REFILL_STEPS");
@@ -306,7 +306,7 @@ int launch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const PassP
                 int kahan, int width, int height, Ctrl* ctrl, FrameBufs fb, unsigned long long* status,
                 size_t status_stride, int num_sms, cudaEvent_t* ev, unsigned long long* totals, bool shared,
                 cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, int shade_split_req, int min_lanes) {
-  const bool two_launches = shade_split_req < 0 ? shade_split() : shade_split_req != 0;
+  const bool two_launches = shade_split_req < 0 ? shade_split(width * height) : shade_split_req != 0;
   const int N = width * height;
   // shadow rays of bounce b beside the extension rays of bounce b + 1 (no
   // per-kernel events): both read only what shading b wrote (in reference
@@ -366,7 +366,7 @@ int launch_batch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const
   k_raygen_batch<<<(total + 255) / 256, 256, 0, st>>>(B, total, ctrl, fb);
   for (int b = 1; b <= max_depth; ++b) {
     launch_trace(st, S, ctrl, b, 1, fb, kahan, true, total, num_sms, shared, min_lanes);
-    launch_shade_batch(st, S, E, d_start, d_film, d_pp, nframes, shade_split(), num_sms, total, ctrl, b, fb);
+    launch_shade_batch(st, S, E, d_start, d_film, d_pp, nframes, shade_split(total), num_sms, total, ctrl, b, fb);
     launch_trace(st, S, ctrl, b, 1, fb, kahan, false, total, num_sms, shared, min_lanes);
   }
   if (totals) k_accumulate<<<1, 32, 0, st>>>(ctrl, max_depth, total, totals);

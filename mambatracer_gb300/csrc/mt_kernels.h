@@ -77,10 +77,18 @@ void launch_shade(cudaStream_t st, const DevScene& S, const DevEnv& E, const Pas
 void launch_shade_batch(cudaStream_t st, const DevScene& S, const DevEnv& E, const int* d_start, const int* d_film,
                         const PassParams* d_pp, int nframes, bool two, int num_sms, int total, Ctrl* ctrl, int b,
                         FrameBufs fb);
-// The process's benchmark-semantics shading setting (MT_SHADE_SPLIT): -1 render
-// jobs choose per frame (shade_split_for) and other passes run two launches; 0
-// always one launch; 1 always two.
+// The process's benchmark-semantics shading setting (MT_SHADE_SPLIT): -1 by size
+// and, in render jobs, per frame (shade_split_for); 0 always one launch; 1 always
+// two.
 int shade_split_setting();
+// Paths from which a pass that runs alone may shade in two launches. Below, the
+// second launch costs more than its full warps gain, whatever share of the paths
+// goes on (4 passes, one launch against two: room 256 x 256, 99 % going on, 944 and
+// 1061 us, 39 % 857 and 959, 6 % 743 and 840; textured room 640 x 360, 64 %, 1345 and
+// 1512; 200k soup 800 x 600, 70 %, 10.16 and 10.20 ms; room 1280 x 720, 64 %, 2.63 and
+// 2.82); above, two pay (textured room 1920 x 1080, 64 %, 5.84 and 5.71 ms; 200k soup
+// 1920 x 1080, 52 %, 22.16 and 21.80).
+constexpr int kSplitPaths = 1 << 20;
 // Whether shading in two launches pays for a frame whose bounce-1 queue of
 // `queued` paths left `went_on` going on (two launches pay when many paths end at
 // their first hit: their lanes would idle through the light and BSDF samples);

@@ -226,7 +226,7 @@ int mt_film_read(mt_job* job, float* rgba, int resolve);
  * so the next frames can be submitted while this one finishes. Up to eight
  * reads stay pending; a ninth first completes the oldest. rgba must stay valid
  * until its read completes (mt_film_wait, mt_film_read, mt_film_clear, or the
- * ninth read after it); resolve is applied then. No counterpart in the
+ * ninth read after it); resolve is applied on the device before the copy. No counterpart in the
  * reference, whose image read (CImage.processImage/readImage) blocks. */
 int mt_film_read_async(mt_job* job, float* rgba, int resolve);
 int mt_film_wait(mt_job* job);

@@ -208,8 +208,6 @@ struct mt_job {
   static constexpr int kMaxReads = 8;
   struct Read {
     float* host = nullptr;
-    int resolve = 0;
-    double frames = 0;
     cudaEvent_t ev = nullptr;
   };
   cudaStream_t rstream = nullptr;
@@ -217,6 +215,7 @@ struct mt_job {
   cudaEvent_t rdone = nullptr;  // the latest read's event: one of reads[].ev
   Read reads[kMaxReads];        // pending reads, oldest at r_head
   int r_head = 0, r_count = 0;
+  float4* d_resolved = nullptr;  // the film divided by its frames, for resolved reads (first one on)
   const float4* film() const { return nslots > 1 ? d_film : slots[0].fb.film; }
   // adaptive light grid (mode 1, scene grid on, environment present)
   unsigned scene_version = 0;

@@ -16,6 +16,7 @@ constexpr int kQuadEmpty = (int)0x80000000;  // an unused child slot of a 4-wide
 // most three children, so a tree within the 64-level bound needs 3 * 32 entries.
 constexpr int kQuadStack = 3 * (kStackDepth / 2);
 constexpr int kWideWords = 6;        // uint4 per wide-BVH node: 80 bytes used, padded to 96 (three 32-byte loads)
+constexpr int kTinyRecords = 512;    // a tree that fits an SM's L1 (32 KB of 64-byte records)
 constexpr int kTraceThreads = 128;   // threads per traversal CTA
 constexpr int kTraceMinBlocksClosest = 12;  // register bounds of the traversal kernels (CTAs per SM)
 constexpr int kTraceMinBlocksShadow = 8;

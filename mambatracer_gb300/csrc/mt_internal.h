@@ -168,19 +168,28 @@ struct mt_scene {
   }
 };
 
-// One in-flight frame's resources: path state, queues, film, parameters,
-// control blocks, and the stream its frames run on.
-struct JobSlot {
+// What one pass in flight needs: path state and queues, its stream and the stream of
+// its shadow rays.
+struct PassBuf {
   FrameBufs fb{};
+  cudaStream_t stream = nullptr;  // the slot's own for its first buffer
+  cudaStream_t side = nullptr;    // shadow rays beside the next bounce's extension rays
+  cudaEvent_t sfork = nullptr, sjoin = nullptr, done = nullptr;
+};
+// One in-flight frame's resources: pass buffers, film, parameters, control blocks,
+// and the stream its frames run on.
+struct JobSlot {
+  char* slab = nullptr;                    // the device arrays below, one allocation
+  std::vector<PassBuf> bufs;               // passes of a frame that overlap
+  float4 *film = nullptr, *film_c = nullptr;  // the slot's own film (not when passes go to the job's)
   Ctrl* d_ctrl = nullptr;                  // one per pass
-  unsigned long long* d_status = nullptr;  // compaction tile status, per pass and bounce
+  unsigned long long* d_status = nullptr;  // mode 0: compaction tile status, per pass and bounce
   PassParams* h_pp = nullptr;              // pinned, one per pass
   PassParams* d_pp = nullptr;
   cudaStream_t stream = nullptr;
-  cudaStream_t side = nullptr;  // shadow rays beside the next bounce's extension rays
-  cudaEvent_t sfork = nullptr, sjoin = nullptr;
+  cudaEvent_t pfork = nullptr;  // the other buffers' streams start after the frame's set-up
   cudaEvent_t fork = nullptr, ev0 = nullptr, ev1 = nullptr, done = nullptr;
-  cudaGraphExec_t graphs[2] = {nullptr, nullptr};  // per shading form: one launch, two launches
+  cudaGraphExec_t graphs[2] = {nullptr, nullptr};  // of a frame among others, and of one alone (logged jobs)
   unsigned graph_version = 0;  // scene version the graph was captured against
   bool ran = false;            // a frame has run on this slot (its control blocks hold its counts)
 };
@@ -189,7 +198,11 @@ struct mt_job {
   mt_context* ctx;
   mt_scene* scene;
   mt_render_config cfg;
+  // Passes of one frame, and frames rendered one after the other, run side by side
+  // in `logged` jobs: each logs its contributions, and they are added to the film in
+  // pass order. merge: the caller's own frames in flight (cfg.inflight > 1).
   int nslots = 1;
+  bool logged = false, merge = false;
   std::vector<JobSlot> slots;
   int next = 0;   // slot of the next frame
   int last = -1;  // slot of the last frame
@@ -197,8 +210,9 @@ struct mt_job {
   unsigned char camera[64];
   int has_camera = 0;
   double frames = 0;                       // passes accumulated in the film
-  // nslots > 1: each frame renders into its slot's film from zero, and a merge
-  // on the slot's stream adds it into this film in frame order
+  // merge: each frame renders into its slot's film from zero, and a merge on the
+  // slot's stream adds it into this film in frame order; logged without merge: the
+  // film itself
   float4* d_film = nullptr;
   float4* d_film_c = nullptr;
   std::vector<cudaEvent_t> kev;            // profile: 2 + 3 * max_depth per pass
@@ -216,13 +230,10 @@ struct mt_job {
   Read reads[kMaxReads];        // pending reads, oldest at r_head
   int r_head = 0, r_count = 0;
   float4* d_resolved = nullptr;  // the film divided by its frames, for resolved reads (first one on)
-  const float4* film() const { return nslots > 1 ? d_film : slots[0].fb.film; }
+  const float4* film() const { return d_film ? d_film : slots[0].film; }
   // adaptive light grid (mode 1, scene grid on, environment present)
   unsigned scene_version = 0;
   unsigned tune_version = 0;  // launch-shape version the graphs were captured with
-  // benchmark-semantics shading form of the next frames (1 two launches, 0 one),
-  // chosen from the last finished frame's bounce-1 survivors; -1 not yet known
-  int shade_split = -1;
   int64_t launches = 0;  // kernels of the render passes and film merges issued (mt_job_launches)
   int grid_on = 0, grid_fp64 = 0;
   int nu = 0, nv = 0, rx = 0, ry = 0;

@@ -65,6 +65,18 @@ void camera_constants(const void* cam64, int W, int H, PassParams& pp) {
 
 namespace {
 
+// Passes of a job that run side by side: a pass alone leaves most of the GPU idle
+// from its third bounce on, when few paths are left. 1, 2, 4, 8 at once: the room at
+// 500 x 500, 15 bounces, four frames 3.76, 2.59, 2.32, 2.16 ms; the textured room at
+// 641 x 359, 8 passes, 2.61, 1.79, 1.58, 1.46; the 200k soup at 800 x 600, 4 passes,
+// 11.1, 8.1, 6.9, 6.9; the stadium at 1080p, 4 passes, 11.9 and (4) 8.2. More than
+// four cost memory and gain little; where the caller keeps frames in flight, a few
+// more keep each frame's own passes together (stadium, two frames of 4 passes, one
+// submitted: 8.8 ms with two at once, 7.7 with four).
+constexpr int kOverlap = 4;
+constexpr int kOverlapMerged = 8;
+constexpr size_t kOverlapBytes = 8ull << 30;  // the memory their buffers may take
+
 // Adds one frame's film (rendered from zero into its slot's film) into the
 // job's film. With Kahan adds on, the slot film's value is film - film_c and
 // the add into the job's film is compensated too.
@@ -88,36 +100,28 @@ __global__ void k_film_merge(const float4* __restrict__ f, const float4* __restr
 }
 
 void free_slot(JobSlot& s) {
-  for (int k = 0; k < 2; ++k) {
-    dfree(s.fb.q_o[k]);
-    dfree(s.fb.q_d[k]);
-    dfree(s.fb.q_t[k]);
+  for (PassBuf& B : s.bufs) {
+    for (cudaEvent_t* e : {&B.sfork, &B.sjoin, &B.done}) {
+      if (*e) cudaEventDestroy(*e);
+      *e = nullptr;
+    }
+    if (B.side) cudaStreamDestroy(B.side);
+    if (B.stream && B.stream != s.stream) cudaStreamDestroy(B.stream);
   }
-  dfree(s.fb.hit_t);
-  dfree(s.fb.hit_prim);
-  dfree(s.fb.s_o);
-  dfree(s.fb.s_d);
-  dfree(s.fb.s_c);
-  dfree(s.fb.film);
-  dfree(s.fb.film_c);
-  dfree(s.fb.live);
-  dfree(s.d_ctrl);
-  dfree(s.d_status);
-  dfree(s.d_pp);
+  s.bufs.clear();
+  dfree(s.slab);
   if (s.h_pp) cudaFreeHost(s.h_pp);
   s.h_pp = nullptr;
   for (cudaGraphExec_t& g : s.graphs) {
     if (g) cudaGraphExecDestroy(g);
     g = nullptr;
   }
-  for (cudaEvent_t* e : {&s.fork, &s.ev0, &s.ev1, &s.done, &s.sfork, &s.sjoin}) {
+  for (cudaEvent_t* e : {&s.pfork, &s.fork, &s.ev0, &s.ev1, &s.done}) {
     if (*e) cudaEventDestroy(*e);
     *e = nullptr;
   }
   if (s.stream) cudaStreamDestroy(s.stream);
   s.stream = nullptr;
-  if (s.side) cudaStreamDestroy(s.side);
-  s.side = nullptr;
 }
 
 void free_job(mt_job* j) {
@@ -168,36 +172,78 @@ int check_cfg(const mt_render_config* c) {
   return MT_OK;
 }
 
-int alloc_slot(JobSlot& s, size_t N, int spp, int max_depth, size_t status_stride) {
+// Bytes of one pass buffer per pixel: queues and hits, and the log of a path's
+// contributions (two a bounce at most).
+size_t pass_bytes(int max_depth) { return 6 * 16 + 8 + 48 + 4 + 4 + 32 * (size_t)max_depth; }
+
+// A slot's device memory is one allocation (an allocation costs 40 us and more, whatever
+// its size up to some MB): sized in a first walk over the arrays, handed out in a second.
+int alloc_slot(JobSlot& s, const mt_render_config& c, int nbuf, bool logged, bool own_film, size_t status_stride) {
+  const size_t N = (size_t)c.width * c.height;
   int r = MT_OK;
-  for (int k = 0; k < 2 && !r; ++k) {
-    r = dalloc(&s.fb.q_o[k], N);
-    if (!r) r = dalloc(&s.fb.q_d[k], N);
-    if (!r) r = dalloc(&s.fb.q_t[k], N);
+  if (cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking) != cudaSuccess)
+    r = fail(MT_ERR_CUDA, "stream create");
+  s.bufs.resize(nbuf);
+  size_t at = 0;
+  auto take = [&](auto** p, size_t count) {
+    if (s.slab) *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(s.slab + at);
+    at += (count * sizeof(**p) + 255) / 256 * 256;
+  };
+  for (int walk = 0; walk < 2 && !r; ++walk) {
+    at = 0;
+    for (PassBuf& B : s.bufs) {
+      for (auto* p : {&B.fb.q_o[0], &B.fb.q_o[1], &B.fb.q_d[0], &B.fb.q_d[1], &B.fb.q_t[0], &B.fb.q_t[1], &B.fb.s_o,
+                      &B.fb.s_d, &B.fb.s_c})
+        take(p, N);
+      take(&B.fb.hit_t, N);
+      take(&B.fb.hit_prim, N);
+      take(&B.fb.live, N);
+      if (logged) {
+        take(&B.fb.log, 2 * (size_t)c.max_depth * N);
+        take(&B.fb.log_n, N);
+        B.fb.log_stride = (int)N;
+      }
+    }
+    if (own_film) {
+      take(&s.film, N);
+      take(&s.film_c, N);
+    }
+    take(&s.d_ctrl, (size_t)c.spp);
+    if (c.mode == 0) take(&s.d_status, status_stride * (size_t)c.max_depth * c.spp);
+    take(&s.d_pp, (size_t)c.spp);
+    if (walk == 0) r = dalloc(&s.slab, at);
   }
-  if (!r) r = dalloc(&s.fb.hit_t, N);
-  if (!r) r = dalloc(&s.fb.hit_prim, N);
-  if (!r) r = dalloc(&s.fb.s_o, N);
-  if (!r) r = dalloc(&s.fb.s_d, N);
-  if (!r) r = dalloc(&s.fb.s_c, N);
-  if (!r) r = dalloc(&s.fb.film, N);
-  if (!r) r = dalloc(&s.fb.film_c, N);
-  if (!r) r = dalloc(&s.fb.live, N);
-  if (!r) r = dalloc(&s.d_ctrl, (size_t)spp);
-  if (!r) r = dalloc(&s.d_status, status_stride * (size_t)max_depth * spp);
-  if (!r) r = dalloc(&s.d_pp, (size_t)spp);
-  if (!r && cudaMallocHost((void**)&s.h_pp, sizeof(PassParams) * spp) != cudaSuccess)
+  for (PassBuf& B : s.bufs) {
+    B.fb.film = s.film;
+    B.fb.film_c = s.film_c;
+    if (&B == &s.bufs[0]) B.stream = s.stream;
+    else if (!r && cudaStreamCreateWithFlags(&B.stream, cudaStreamNonBlocking) != cudaSuccess)
+      r = fail(MT_ERR_CUDA, "stream create");
+    if (!r && cudaStreamCreateWithFlags(&B.side, cudaStreamNonBlocking) != cudaSuccess)
+      r = fail(MT_ERR_CUDA, "stream create");
+    for (cudaEvent_t* e : {&B.sfork, &B.sjoin, &B.done})
+      if (!r && cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess)
+        r = fail(MT_ERR_CUDA, "event create");
+  }
+  if (!r && cudaMallocHost((void**)&s.h_pp, sizeof(PassParams) * c.spp) != cudaSuccess)
     r = fail(MT_ERR_NOMEM, "pinned pass parameters");
-  if (!r && cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking) != cudaSuccess)
-    r = fail(MT_ERR_CUDA, "stream create");
-  if (!r && cudaStreamCreateWithFlags(&s.side, cudaStreamNonBlocking) != cudaSuccess)
-    r = fail(MT_ERR_CUDA, "stream create");
   for (cudaEvent_t* e : {&s.fork, &s.ev0, &s.ev1, &s.done})
     if (!r && cudaEventCreate(e) != cudaSuccess) r = fail(MT_ERR_CUDA, "event create");
-  for (cudaEvent_t* e : {&s.sfork, &s.sjoin})
-    if (!r && cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) r = fail(MT_ERR_CUDA, "event create");
-  if (!r) std::memset(s.h_pp, 0, sizeof(PassParams) * spp);
+  if (!r && cudaEventCreateWithFlags(&s.pfork, cudaEventDisableTiming) != cudaSuccess)
+    r = fail(MT_ERR_CUDA, "event create");
+  if (!r) std::memset(s.h_pp, 0, sizeof(PassParams) * c.spp);
   return r;
+}
+
+// Zeroes the job's film (a slot's film of a merge job is zeroed by each frame) on the
+// context stream.
+int clear_films(mt_job* j) {
+  const size_t N = (size_t)j->cfg.width * j->cfg.height;
+  float4* f = j->d_film ? j->d_film : j->slots[0].film;
+  float4* c = j->d_film ? j->d_film_c : j->slots[0].film_c;
+  CU(cudaMemsetAsync(f, 0, N * 16, j->ctx->stream));
+  CU(cudaMemsetAsync(c, 0, N * 16, j->ctx->stream));
+  return MT_OK;
 }
 
 // Sets up the job's light grid from the scene (CAdaptiveEnvironment.setHDRLuminance,
@@ -274,15 +320,24 @@ extern "C" int mt_job_create(mt_context* ctx, mt_scene* scene, const mt_render_c
   j->ctx = ctx;
   j->scene = scene;
   j->cfg = *cfg;
-  j->nslots = (cfg->profile || cfg->inflight < 1) ? 1 : cfg->inflight;
   const size_t N = (size_t)cfg->width * cfg->height;
   j->status_stride = (N + kShadeThreads - 1) / kShadeThreads;
+  // How many passes overlap, shared out over the caller's frames in flight; without
+  // those, over the passes of a frame first and then over frames.
+  const int frames = (cfg->profile || cfg->inflight < 1) ? 1 : cfg->inflight;
+  const size_t fit = kOverlapBytes / (N * pass_bytes(cfg->max_depth));
+  const int overlap =
+      cfg->profile ? 1 : (int)std::min<size_t>(frames > 1 ? kOverlapMerged : kOverlap, std::max<size_t>(fit, 1));
+  const int nbuf = std::max(1, std::min({cfg->spp, kOverlap, overlap / frames}));
+  j->merge = frames > 1;
+  j->nslots = j->merge ? frames : std::max(1, overlap / nbuf);
+  j->logged = nbuf > 1 || (!j->merge && j->nslots > 1);
   j->slots.resize(j->nslots);
   for (JobSlot& s : j->slots)
-    if (!r) r = alloc_slot(s, N, cfg->spp, cfg->max_depth, j->status_stride);
+    if (!r) r = alloc_slot(s, *cfg, nbuf, j->logged, j->merge || !j->logged, j->status_stride);
   if (!r) r = dalloc(&j->d_totals, 4);
-  if (!r && j->nslots > 1) r = dalloc(&j->d_film, N);
-  if (!r && j->nslots > 1) r = dalloc(&j->d_film_c, N);
+  if (!r && (j->merge || j->logged)) r = dalloc(&j->d_film, N);
+  if (!r && (j->merge || j->logged)) r = dalloc(&j->d_film_c, N);
   if (!r && cudaStreamCreateWithFlags(&j->rstream, cudaStreamNonBlocking) != cudaSuccess)
     r = fail(MT_ERR_CUDA, "stream create");
   if (!r && cudaEventCreateWithFlags(&j->rfork, cudaEventDisableTiming) != cudaSuccess)
@@ -310,14 +365,7 @@ extern "C" int mt_job_create(mt_context* ctx, mt_scene* scene, const mt_render_c
     return r;
   }
   j->h_ctrl.resize(cfg->spp);
-  for (JobSlot& s : j->slots) {
-    cudaMemsetAsync(s.fb.film, 0, N * 16, ctx->stream);
-    cudaMemsetAsync(s.fb.film_c, 0, N * 16, ctx->stream);
-  }
-  if (j->nslots > 1) {
-    cudaMemsetAsync(j->d_film, 0, N * 16, ctx->stream);
-    cudaMemsetAsync(j->d_film_c, 0, N * 16, ctx->stream);
-  }
+  clear_films(j);
   cudaMemsetAsync(j->d_totals, 0, 32, ctx->stream);
   CU(cudaStreamSynchronize(ctx->stream));
   ctx->jobs.push_back(j);
@@ -349,8 +397,28 @@ extern "C" int mt_job_set_camera(mt_job* j, const void* camera) {
 }
 
 namespace {
-// Enqueue one frame's passes on the slot's stream.
-int enqueue_frame(mt_job* j, JobSlot& s) {
+// Logged jobs: whether a frame's passes are added to the film among its launches (its
+// slot's own film, or the job's when no other frame is in flight) or after them.
+bool replay_inside(const mt_job* j) { return j->merge || j->nslots == 1; }
+// Adds passes p .. p + n - 1 of the slot's frame to the film they go to.
+int replay(mt_job* j, JobSlot& s, cudaStream_t st, int p, int n) {
+  Replay R{};
+  R.passes = n;
+  R.stride = j->cfg.width * j->cfg.height;
+  R.max_depth = j->cfg.max_depth;
+  R.kahan = j->cfg.film_kahan;
+  for (int i = 0; i < n; ++i) {
+    const FrameBufs& fb = s.bufs[(p + i) % s.bufs.size()].fb;
+    R.log[i] = fb.log;
+    R.n[i] = fb.log_n;
+    R.ctrl[i] = s.d_ctrl + p + i;
+  }
+  return j->merge ? launch_replay(st, R, s.film, s.film_c, j->d_totals)
+                  : launch_replay(st, R, j->d_film, j->d_film_c, j->d_totals);
+}
+// Enqueue one frame's passes on the slot's streams. direct: a one-pass frame of a
+// logged job with nothing else in flight adds to the job's film as it goes.
+int enqueue_frame(mt_job* j, JobSlot& s, bool direct) {
   mt_context* ctx = j->ctx;
   const mt_render_config& c = j->cfg;
   DevScene S = j->scene->view();
@@ -372,22 +440,40 @@ int enqueue_frame(mt_job* j, JobSlot& s) {
     }
   }
   const size_t per_pass_events = 2 + 3 * (size_t)c.max_depth;
-  if (j->nslots > 1) {
-    const size_t N = (size_t)c.width * c.height;
-    CU(cudaMemsetAsync(s.fb.film, 0, N * 16, s.stream));
-    CU(cudaMemsetAsync(s.fb.film_c, 0, N * 16, s.stream));
+  const size_t N = (size_t)c.width * c.height, status = j->status_stride * (size_t)c.max_depth;
+  if (j->merge) {
+    CU(cudaMemsetAsync(s.film, 0, N * 16, s.stream));
+    CU(cudaMemsetAsync(s.film_c, 0, N * 16, s.stream));
   }
+  CU(cudaMemcpyAsync(s.d_pp, s.h_pp, sizeof(PassParams) * c.spp, cudaMemcpyHostToDevice, s.stream));
+  CU(cudaMemsetAsync(s.d_ctrl, 0, sizeof(Ctrl) * c.spp, s.stream));
+  if (c.mode == 0) CU(cudaMemsetAsync(s.d_status, 0, status * c.spp * 8, s.stream));
+  const int nbuf = (int)s.bufs.size();
+  if (nbuf > 1) CU(cudaEventRecord(s.pfork, s.stream));
   for (int p = 0; p < c.spp; ++p) {
-    CU(cudaMemcpyAsync(s.d_pp + p, s.h_pp + p, sizeof(PassParams), cudaMemcpyHostToDevice, s.stream));
-    CU(cudaMemsetAsync(s.d_ctrl + p, 0, sizeof(Ctrl), s.stream));
-    CU(cudaMemsetAsync(s.d_status + j->status_stride * (size_t)c.max_depth * p, 0,
-                       j->status_stride * (size_t)c.max_depth * 8, s.stream));
+    PassBuf& B = s.bufs[p % nbuf];
+    if (p > 0 && p < nbuf) CU(cudaStreamWaitEvent(B.stream, s.pfork, 0));
     cudaEvent_t* ev = j->kev.empty() ? nullptr : j->kev.data() + per_pass_events * p;
-    if (launch_pass(s.stream, S, E, s.d_pp + p, c.mode, c.max_depth, c.film_kahan, c.width, c.height, s.d_ctrl + p,
-                    s.fb, s.d_status + j->status_stride * (size_t)c.max_depth * p, j->status_stride, ctx->num_sms,
-                    ev, j->d_totals, j->nslots > 1, s.side, s.sfork, s.sjoin, j->shade_split != 0, tail_lanes(j->nslots)))
+    FrameBufs fb = B.fb;
+    if (direct) {
+      fb.log = nullptr;
+      fb.film = j->d_film;
+      fb.film_c = j->d_film_c;
+    }
+    const int beside = direct ? 1 : std::max(j->nslots, nbuf);
+    if (launch_pass(B.stream, S, E, s.d_pp + p, c.mode, c.max_depth, c.film_kahan, c.width, c.height, s.d_ctrl + p, fb,
+                    s.d_status ? s.d_status + status * p : nullptr, j->status_stride, ctx->num_sms, ev,
+                    j->logged && !direct ? nullptr : j->d_totals, beside > 1, B.side, B.sfork, B.sjoin,
+                    shade_split((int)N, nbuf > 1 || j->merge), tail_lanes(S, beside)))
       return fail(MT_ERR_CUDA, "pass launch: %s", cudaGetErrorString(cudaGetLastError()));
+    if (j->logged && replay_inside(j)) {
+      // the pass before has been added
+      if (p > 0) CU(cudaStreamWaitEvent(B.stream, s.bufs[(p - 1) % nbuf].done, 0));
+      if (replay(j, s, B.stream, p, 1)) return fail(MT_ERR_CUDA, "film: %s", cudaGetErrorString(cudaGetLastError()));
+    }
+    if (nbuf > 1) CU(cudaEventRecord(B.done, B.stream));
   }
+  for (int k = 1; k < std::min(nbuf, c.spp); ++k) CU(cudaStreamWaitEvent(s.stream, s.bufs[k].done, 0));
   return MT_OK;
 }
 }  // namespace
@@ -428,30 +514,6 @@ extern "C" int mt_render_frame(mt_job* j, const int32_t* seeds, float frame_coun
   // The slot's previous frame must have consumed its pinned parameters; frames
   // on the other slots keep running meanwhile.
   CU(cudaEventSynchronize(s.done));
-  const int split_setting = shade_split_setting();
-  if (split_setting >= 0) {
-    j->shade_split = split_setting;
-  } else if (j->nslots == 1 && c.width * c.height < kSplitPaths) {
-    j->shade_split = 0;
-  } else if (c.mode == 1 && c.max_depth >= 2) {
-    // One launch or two for the shading of the next frames: a finished frame's
-    // share of bounce-1 paths that went on decides (shade_split_for): this slot's
-    // last frame, or, while nothing is decided yet, the job's latest frame once it
-    // has finished. Both forms render the same film, and each slot holds a graph
-    // of each (both captured at its first frame), so a change costs nothing.
-    JobSlot* src = s.ran ? &s : nullptr;
-    if (!src && j->shade_split < 0 && j->last >= 0 && j->slots[j->last].ran) {
-      const cudaError_t q = cudaEventQuery(j->slots[j->last].done);
-      if (q == cudaSuccess) src = &j->slots[j->last];
-      else if (q != cudaErrorNotReady) return fail(MT_ERR_CUDA, "frame event: %s", cudaGetErrorString(q));
-    }
-    if (src) {
-      int counts[3] = {0, 0, 0};
-      CU(cudaMemcpyAsync(counts, src->d_ctrl, sizeof(counts), cudaMemcpyDeviceToHost, src->stream));
-      CU(cudaStreamSynchronize(src->stream));
-      j->shade_split = shade_split_for(counts[1], counts[2], j->shade_split < 0 ? 1 : j->shade_split);
-    }
-  }
   // CDeviceGI.loop updates the grid after each of its first frames
   // (src/cl/device/CDeviceGI.java:263-264): those frames accumulate.
   const int accumulate = j->grid_on && j->grid_frames < c.grid_updates;
@@ -472,38 +534,42 @@ extern "C" int mt_render_frame(mt_job* j, const int32_t* seeds, float frame_coun
   // order after work already on the context stream (film clears, uploads)
   CU(cudaEventRecord(s.fork, ctx->stream));
   CU(cudaStreamWaitEvent(s.stream, s.fork, 0));
-  if (j->nslots == 1) CU(cudaStreamWaitEvent(s.stream, j->rdone, 0));
+  bool direct = false;
+  if (j->logged && !replay_inside(j) && c.spp == 1) {
+    const cudaError_t q = j->last < 0 ? cudaSuccess : cudaEventQuery(j->slots[j->last].done);
+    if (q == cudaErrorNotReady) cudaGetLastError();
+    else if (q != cudaSuccess) return fail(MT_ERR_CUDA, "frame event: %s", cudaGetErrorString(q));
+    direct = q == cudaSuccess;
+  }
+  // a frame that adds to the film as it goes starts after the film's last read
+  if (j->nslots == 1 || direct) CU(cudaStreamWaitEvent(s.stream, j->rdone, 0));
   if (j->grid_on) CU(cudaStreamWaitEvent(s.stream, j->grid_ev, 0));  // the last grid update
   CU(cudaEventRecord(s.ev0, s.stream));
   if (c.use_graph && !c.profile) {
-    const int form = j->shade_split == 0 ? 0 : 1;
-    const bool both = split_setting < 0 && c.mode == 1 && (j->nslots > 1 || c.width * c.height >= kSplitPaths);  // may switch later
-    for (int f = 0; f < 2; ++f) {
-      if (s.graphs[f] || (f != form && !both)) continue;
-      const int keep = j->shade_split;
-      j->shade_split = f;
+    cudaGraphExec_t& graph = s.graphs[direct];
+    if (!graph) {
       cudaGraph_t g;
       CU(cudaStreamBeginCapture(s.stream, cudaStreamCaptureModeThreadLocal));
-      int r = enqueue_frame(j, s);
+      int r = enqueue_frame(j, s, direct);
       cudaError_t e = cudaStreamEndCapture(s.stream, &g);
-      j->shade_split = keep;
       if (r) return r;
       if (e != cudaSuccess) return fail(MT_ERR_CUDA, "graph capture: %s", cudaGetErrorString(e));
-      e = cudaGraphInstantiate(&s.graphs[f], g, 0);
+      e = cudaGraphInstantiate(&graph, g, 0);
       cudaGraphDestroy(g);
       if (e != cudaSuccess) return fail(MT_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(e));
     }
-    CU(cudaGraphLaunch(s.graphs[form], s.stream));
+    CU(cudaGraphLaunch(graph, s.stream));
   } else {
-    int r = enqueue_frame(j, s);
+    int r = enqueue_frame(j, s, direct);
     if (r) return r;
   }
   s.ran = true;
   {
     // per pass: raygen, per bounce closest hits + shading (one launch or two) +
     // shadow rays, the ray totals; then the film merge
-    const int two = c.mode == 1 && j->shade_split != 0;
-    j->launches += (int64_t)c.spp * (2 + (int64_t)c.max_depth * (3 + two)) + (j->nslots > 1 ? 1 : 0);
+    const int two = c.mode == 1 && shade_split(c.width * c.height, s.bufs.size() > 1 || j->merge);
+    j->launches += (int64_t)c.spp * (2 + (int64_t)c.max_depth * (3 + two)) + (j->merge ? 1 : 0);
+    if (j->logged && !replay_inside(j)) j->launches -= c.spp - 1;  // all its passes in one
   }
   CU(cudaEventRecord(s.ev1, s.stream));
   if (accumulate) {
@@ -524,8 +590,11 @@ extern "C" int mt_render_frame(mt_job* j, const int32_t* seeds, float frame_coun
     if (j->last >= 0) CU(cudaStreamWaitEvent(s.stream, j->slots[j->last].done, 0));
     CU(cudaStreamWaitEvent(s.stream, j->rdone, 0));
     const size_t N = (size_t)c.width * c.height;
-    k_film_merge<<<(unsigned)((N + 255) / 256), 256, 0, s.stream>>>(s.fb.film, s.fb.film_c, c.film_kahan, N,
-                                                                    j->d_film, j->d_film_c);
+    if (j->merge)
+      k_film_merge<<<(unsigned)((N + 255) / 256), 256, 0, s.stream>>>(s.film, s.film_c, c.film_kahan, N, j->d_film,
+                                                                      j->d_film_c);
+    else if (!direct)
+      replay(j, s, s.stream, 0, c.spp);
     CU(cudaGetLastError());
   }
   CU(cudaEventRecord(s.done, s.stream));
@@ -703,15 +772,8 @@ extern "C" int mt_film_clear(mt_job* j) {
   int r = finish_reads(j);
   if (r) return r;
   join_jobs(ctx);
-  const size_t N = (size_t)j->cfg.width * j->cfg.height;
-  for (JobSlot& s : j->slots) {
-    CU(cudaMemsetAsync(s.fb.film, 0, N * 16, ctx->stream));
-    CU(cudaMemsetAsync(s.fb.film_c, 0, N * 16, ctx->stream));
-  }
-  if (j->nslots > 1) {
-    CU(cudaMemsetAsync(j->d_film, 0, N * 16, ctx->stream));
-    CU(cudaMemsetAsync(j->d_film_c, 0, N * 16, ctx->stream));
-  }
+  r = clear_films(j);
+  if (r) return r;
   CU(cudaMemsetAsync(j->d_totals, 0, 32, ctx->stream));
   image_reset(j);
   j->frames = 0;

@@ -70,8 +70,7 @@ struct ShadowRays {
 struct ShadowResolve {
   const float4* so;
   const float4* sc;
-  float4* film;
-  float4* film_c;
+  FrameBufs fb;
   int kahan;
   unsigned* traced;
   __device__ __forceinline__ void operator()(int i, const tr::RayT&, int hit) const {
@@ -80,7 +79,7 @@ struct ShadowResolve {
     ++*traced;
     if (hit < 0) {  // unoccluded: addAccum(&accum[pixel], contrib), Render.cl:456-461
       float4 c = __ldg(sc + i);
-      film_add(film, film_c, pixel, mk(c.x, c.y, c.z, 1.f), kahan);
+      contribute(fb, pixel, pixel, mk(c.x, c.y, c.z, 1.f), kahan);
     }
   }
 };
@@ -115,7 +114,7 @@ __global__ void __launch_bounds__(kTraceThreads, MINB) k_trace_shadow(DevScene S
   unsigned traced = 0;
   tr::trace_persistent<true, kSteps, ShadowRays, ShadowResolve, PREC>(
       S, count, &ctrl->work[2 * b + 1], ShadowRays{fb.s_o, fb.s_d},
-      ShadowResolve{fb.s_o, fb.s_c, fb.film, fb.film_c, kahan, &traced}, &overflow, steps, min_lanes);
+      ShadowResolve{fb.s_o, fb.s_c, fb, kahan, &traced}, &overflow, steps, min_lanes);
   unsigned long long tot = traced;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) tot += __shfl_down_sync(0xffffffffu, tot, o);
@@ -134,6 +133,48 @@ __global__ void k_accumulate(const Ctrl* ctrl, int max_depth, int n_pixels, unsi
   atomicAdd(totals + 1, ext);
   atomicAdd(totals + 2, (unsigned long long)ctrl->rays[2]);
   if (ctrl->error) atomicExch(totals + 3, (unsigned long long)ctrl->error);
+}
+
+// Adds logged contributions to the film, one thread per pixel: reads what was
+// logged and the film once, coalesced.
+__global__ void k_replay(Replay R, float4* __restrict__ film, float4* __restrict__ film_c, unsigned long long* totals) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < R.passes) {
+    const Ctrl& c = *R.ctrl[i];
+    unsigned long long ext = 0;
+    for (int b = 2; b <= R.max_depth; ++b) ext += (unsigned long long)c.count[b];
+    atomicAdd(totals + 0, (unsigned long long)R.stride);
+    atomicAdd(totals + 1, ext);
+    atomicAdd(totals + 2, c.rays[2]);
+    if (c.error) atomicExch(totals + 3, (unsigned long long)c.error);
+  }
+  if (i >= R.stride) return;
+  int n[kReplayPasses], any = 0;
+#pragma unroll
+  for (int p = 0; p < kReplayPasses; ++p) {
+    n[p] = p < R.passes ? R.n[p][i] : 0;
+    any |= n[p];
+  }
+  if (!any) return;
+  V a = film[i], c = R.kahan ? film_c[i] : zero4();
+#pragma unroll
+  for (int p = 0; p < kReplayPasses; ++p)
+    for (int k = 0; k < n[p]; ++k) {
+      const V v = R.log[p][(size_t)k * R.stride + i];
+      if (!R.kahan) {
+        a = add(a, v);
+        continue;
+      }
+      const V y = sub(v, c), t = add(a, y);
+      c = sub(sub(t, a), y);
+      a = t;
+    }
+  film[i] = a;
+  if (R.kahan) film_c[i] = c;
+}
+int launch_replay(cudaStream_t st, const Replay& R, float4* film, float4* film_c, unsigned long long* totals) {
+  k_replay<<<(R.stride + 255) / 256, 256, 0, st>>>(R, film, film_c, totals);
+  return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
 // ---------------------------------------------------------------- launchers
@@ -165,18 +206,6 @@ int env_shade_minb() {
   int x = e ? std::atoi(e) : kShadeMinBlocks;
   return (x == 3 || x == 4 || x == 5) ? x : kShadeMinBlocks;
 }
-// MT_SHADE_SPLIT: unset, render jobs choose one or two shading launches frame by
-// frame (shade_split_for) and other passes by their size; 0 always one; 1 always two.
-int shade_split_mode() {
-  static const int m = [] {
-    const char* e = std::getenv("MT_SHADE_SPLIT");
-    if (!e) return -1;
-    return std::atoi(e) == 0 ? 0 : 1;
-  }();
-  return m;
-}
-bool shade_split(int n) { return shade_split_mode() < 0 ? n >= kSplitPaths : shade_split_mode() != 0; }
-
 int env_steps() {
   const char* e = std::getenv("MT_REFILL_STEPS");
   int x = e ? std::atoi(e) : kSteps;
@@ -258,17 +287,13 @@ void launch_traces(cudaStream_t st, int grid, const DevScene& S, Ctrl* ctrl, int
 
 Tuning get_tuning() { return tuning_ref(); }
 
-int shade_split_setting() { return shade_split_mode(); }
-
-// Measured with six frames in flight: the 1M soup (53 % of bounce-1 paths go
-// on) 915 Mrays/s in two launches against 861 in one; the stadium (71 % go on)
-// 2588 against 2743. A band around the crossover keeps the current choice.
-int shade_split_for(int queued, int went_on, int current) {
-  if (queued <= 0) return current;
-  const double f = (double)went_on / queued;
-  if (f < 0.58) return 1;
-  if (f > 0.66) return 0;
-  return current;
+bool shade_split(int n, bool beside) {
+  static const int m = [] {
+    const char* e = std::getenv("MT_SHADE_SPLIT");
+    if (!e) return -1;
+    return std::atoi(e) == 0 ? 0 : 1;
+  }();
+  return m < 0 ? n >= (beside ? 1 << 18 : 1 << 20) : m != 0;
 }
 
 bool set_tuning(const Tuning& t) {
@@ -305,8 +330,7 @@ void launch_trace(cudaStream_t st, const DevScene& S, Ctrl* ctrl, int b, int mod
 int launch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const PassParams* d_pp, int mode, int max_depth,
                 int kahan, int width, int height, Ctrl* ctrl, FrameBufs fb, unsigned long long* status,
                 size_t status_stride, int num_sms, cudaEvent_t* ev, unsigned long long* totals, bool shared,
-                cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, int shade_split_req, int min_lanes) {
-  const bool two_launches = shade_split_req < 0 ? shade_split(width * height) : shade_split_req != 0;
+                cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, bool two_launches, int min_lanes) {
   const int N = width * height;
   // shadow rays of bounce b beside the extension rays of bounce b + 1 (no
   // per-kernel events): both read only what shading b wrote (in reference
@@ -326,8 +350,7 @@ int launch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const PassP
     trace(true, b);
     if (ev) cudaEventRecord(ev[e++], st);
     if (split && b > 1) cudaStreamWaitEvent(st, join, 0);
-    unsigned long long* stb = status + (size_t)(b - 1) * status_stride;
-    if (mode == 0) launch_shade_ref(st, S, E, d_pp, N, ctrl, b, fb, stb);
+    if (mode == 0) launch_shade_ref(st, S, E, d_pp, N, ctrl, b, fb, status + (size_t)(b - 1) * status_stride);
     else launch_shade(st, S, E, d_pp, two_launches, shade_minb(), num_sms, N, ctrl, b, fb);
     if (ev) cudaEventRecord(ev[e++], st);
     if (split) {
@@ -366,7 +389,7 @@ int launch_batch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const
   k_raygen_batch<<<(total + 255) / 256, 256, 0, st>>>(B, total, ctrl, fb);
   for (int b = 1; b <= max_depth; ++b) {
     launch_trace(st, S, ctrl, b, 1, fb, kahan, true, total, num_sms, shared, min_lanes);
-    launch_shade_batch(st, S, E, d_start, d_film, d_pp, nframes, shade_split(total), num_sms, total, ctrl, b, fb);
+    launch_shade_batch(st, S, E, d_start, d_film, d_pp, nframes, shade_split(total, shared), num_sms, total, ctrl, b, fb);
     launch_trace(st, S, ctrl, b, 1, fb, kahan, false, total, num_sms, shared, min_lanes);
   }
   if (totals) k_accumulate<<<1, 32, 0, st>>>(ctrl, max_depth, total, totals);

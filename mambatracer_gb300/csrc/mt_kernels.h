@@ -19,16 +19,37 @@ struct FrameBufs {
   float4* film;     // accumulated radiance per pixel
   float4* film_c;   // Kahan compensation per pixel
   int* live;        // queue slots of the paths that go on after the hit phase (two-launch shading)
+  // Contributions kept for later (passes that overlap): path g's k-th one at
+  // log[k * log_stride + g], log_n[g] of them; log NULL: added to the film at once.
+  float4* log;
+  int* log_n;
+  int log_stride;
 };
 
-// Rays of a short queue kept together in a warp, by how many frames or streams
-// of passes run side by side. Alone, one ray to a warp is fastest (1, 2, 4, 8,
-// 16, 32: the 200k soup at 800 x 600 12.2, 12.3, 12.5, 12.7, 13.3, 14.2 ms); with
-// six 1080p frames of the 1M soup in flight the GPU's issue slots are taken and
-// the spread rays' instructions cost (46.8, 46.6, 46.4, 46.1, 45.5, 45.2 ms for
-// eight frames); a served mix on four streams lies between (12.5, 12.7, 12.8, 13.1,
-// 13.5, 14.3 ms).
-inline int tail_lanes(int beside) { return beside <= 1 ? 1 : beside <= 4 ? 8 : 32; }
+// Up to kReplayPasses finished passes' contributions, added to the film pass by
+// pass in the order they were made (what film_add does as they come), and the
+// passes' ray counts to the totals.
+constexpr int kReplayPasses = 4;
+struct Replay {
+  const float4* log[kReplayPasses];
+  const int* n[kReplayPasses];
+  const Ctrl* ctrl[kReplayPasses];
+  int passes, stride, max_depth, kahan;
+};
+int launch_replay(cudaStream_t st, const Replay& R, float4* film, float4* film_c, unsigned long long* totals);
+
+// Rays of a short queue kept together in a warp, by how many passes run side by
+// side. Alone, one ray to a warp is fastest (1, 2, 4, 8, 16, 32: the 200k soup at 800 x
+// 600, passes one by one, 12.2, 12.3, 12.5, 12.7, 13.3, 14.2 ms); with six 1080p frames of
+// the 1M soup in flight the GPU's issue slots are taken and the spread rays'
+// instructions cost (46.8, 46.6, 46.4, 46.1, 45.5, 45.2 ms for eight frames); a served
+// mix on four streams lies between (12.5, 12.7, 12.8, 13.1, 13.5, 14.3 ms), and so do
+// four passes at once (200k soup 6.70 ms with 8, 6.94 with 32). A tree of a few hundred
+// nodes is in L1 and its rays are short, so there is no latency to spread for beside
+// others (room 500 x 500, four frames at once, 2.32 ms with 8, 2.16 with 32).
+inline int tail_lanes(const DevScene& S, int beside) {
+  return beside <= 1 ? 1 : beside <= 4 && S.nrec > kTinyRecords ? 8 : 32;
+}
 
 // Launch shapes of the hot kernels, process-wide (one GPU per process):
 // closest_minb / shadow_minb: the traversal build, by the resident blocks per
@@ -66,7 +87,7 @@ int launch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const PassP
                 int max_depth, int kahan, int width, int height, Ctrl* ctrl, FrameBufs fb,
                 unsigned long long* status, size_t status_stride, int num_sms, cudaEvent_t* events,
                 unsigned long long* totals, bool shared = false, cudaStream_t side = nullptr,
-                cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr, int shade_split = -1, int min_lanes = 1);
+                cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr, bool two_launches = false, int min_lanes = 1);
 // Shading of one bounce (mt_shade.cu): reference semantics; benchmark semantics of
 // one frame (in one launch or two) and of a merged batch pass. N, total: paths a
 // queue holds at most.
@@ -77,23 +98,16 @@ void launch_shade(cudaStream_t st, const DevScene& S, const DevEnv& E, const Pas
 void launch_shade_batch(cudaStream_t st, const DevScene& S, const DevEnv& E, const int* d_start, const int* d_film,
                         const PassParams* d_pp, int nframes, bool two, int num_sms, int total, Ctrl* ctrl, int b,
                         FrameBufs fb);
-// The process's benchmark-semantics shading setting (MT_SHADE_SPLIT): -1 by size
-// and, in render jobs, per frame (shade_split_for); 0 always one launch; 1 always
-// two.
-int shade_split_setting();
-// Paths from which a pass that runs alone may shade in two launches. Below, the
-// second launch costs more than its full warps gain, whatever share of the paths
-// goes on (4 passes, one launch against two: room 256 x 256, 99 % going on, 944 and
-// 1061 us, 39 % 857 and 959, 6 % 743 and 840; textured room 640 x 360, 64 %, 1345 and
-// 1512; 200k soup 800 x 600, 70 %, 10.16 and 10.20 ms; room 1280 x 720, 64 %, 2.63 and
-// 2.82); above, two pay (textured room 1920 x 1080, 64 %, 5.84 and 5.71 ms; 200k soup
-// 1920 x 1080, 52 %, 22.16 and 21.80).
-constexpr int kSplitPaths = 1 << 20;
-// Whether shading in two launches pays for a frame whose bounce-1 queue of
-// `queued` paths left `went_on` going on (two launches pay when many paths end at
-// their first hit: their lanes would idle through the light and BSDF samples);
-// current: the choice so far, kept near the crossover.
-int shade_split_for(int queued, int went_on, int current);
+// Whether a pass of n paths shades in two launches (MT_SHADE_SPLIT in the environment:
+// 0 never, 1 always): beside, other passes or frames run beside it. The second
+// launch's full warps and smaller code gain with the paths; its fixed cost of a few
+// us a bounce matters below a million paths alone and, hidden behind the others,
+// below 2^18 beside others. One launch against two, alone: room 256 x 256, 4 passes,
+// 944 and 1061 us; 200k soup 800 x 600, 3.02 and 3.05 ms; textured room 1920 x 1080, 4
+// passes, 5.84 and 5.71 ms; overlapping: 200k soup 800 x 600, 4 passes, 6.89 and 6.70;
+// stadium 1080p, 4 passes, 8.17 and 7.55; eight frames of the stadium in flight 16.8 and
+// 15.2, of the 1M soup 44.2 and 40.7.
+bool shade_split(int n, bool beside);
 
 // Closest or any hit of reference-layout rays with the traversal work per ray
 // (interior-node visits, triangle tests), one ray per thread.

@@ -256,8 +256,8 @@ int start_request(mt_server* s, Lane& L, Request* R) {
   for (int p = 0; p < R->spp; ++p)
     if (launch_pass(L.stream, S, E, L.d_pp + p, 1, c.max_depth, c.film_kahan, R->width, R->height, L.d_ctrl + p,
                     L.fb, L.d_status + stride * (size_t)c.max_depth * p, stride, s->ctx->num_sms, nullptr,
-                    s->d_totals, s->lanes.size() > 1, L.side, L.sfork, L.sjoin, -1,
-                    tail_lanes((int)s->lanes.size())))
+                    s->d_totals, s->lanes.size() > 1, L.side, L.sfork, L.sjoin,
+                    shade_split((int)N, s->lanes.size() > 1), tail_lanes(S, (int)s->lanes.size())))
       return fail(MT_ERR_CUDA, "pass launch: %s", cudaGetErrorString(cudaGetLastError()));
   CU(cudaMemcpyAsync(L.h_stage, L.fb.film, N * 16, cudaMemcpyDeviceToHost, L.stream));
   CU(cudaLaunchHostFunc(L.stream, lane_done, &L));
@@ -440,7 +440,7 @@ int issue_round(mt_server* s, MergeGroup& G, const std::vector<int>& work, const
     const int lr = launch_batch_pass(st, S, E, Rd.d_tab + Gr.tab, Rd.d_tab + Gr.tab + Gr.n + 1, Rd.d_pp + Gr.pp,
                                      Gr.n, Gr.total, c.max_depth, c.film_kahan, Rd.d_ctrl + g, G.fb,
                                      s->ctx->num_sms, s->d_totals, s->groups.size() > 1,
-                                     tail_lanes((int)s->groups.size()));
+                                     tail_lanes(S, (int)s->groups.size()));
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(st, &graph);
     if (lr || e != cudaSuccess) {

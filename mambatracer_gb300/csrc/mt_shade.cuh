@@ -24,6 +24,18 @@ __device__ __forceinline__ void film_add(float4* __restrict__ acc, float4* __res
   acc[pixel] = t;
 }
 
+// A contribution of path g to pixel f: added to the film, or kept in the pass's log,
+// from which k_replay adds it once the passes before have been added. Either way a
+// pixel's sums see the same values in the same order.
+__device__ __forceinline__ void contribute(const FrameBufs& fb, int g, int f, V v, int kahan) {
+  if (!fb.log) {
+    film_add(fb.film, fb.film_c, f, v, kahan);
+  } else if (abs_valid4(v)) {
+    const int k = fb.log_n[g];
+    fb.log[(size_t)k * fb.log_stride + g] = v;
+    fb.log_n[g] = k + 1;
+  }
+}
 
 // The camera ray of pixel id (InitCameraRayDataJitter): origin, world direction.
 __device__ __forceinline__ void camera_ray(const PassParams* __restrict__ pp, int id, V* o_out, V* d_out) {
@@ -56,6 +68,7 @@ __device__ __forceinline__ void camera_ray(const PassParams* __restrict__ pp, in
 __device__ __forceinline__ void start_path(FrameBufs& fb, int g, V o, V dw) {
   fb.q_o[0][g] = mk(o.x, o.y, o.z, __int_as_float(g));
   fb.q_d[0][g] = mk(dw.x, dw.y, dw.z, 1.f);
+  if (fb.log) fb.log_n[g] = 0;
 }
 
 // ----------------------------------------------------------------- shade
@@ -184,7 +197,7 @@ __device__ __forceinline__ void shade_hit(const DevScene& S, const DevEnv& E, Re
             float pdfW = pdf_a_to_w(pdfA, t, P.B.fix.z);
             w = mis2(P.ps.w, pdfW * pick);
           }
-          film_add(fb.film, fb.film_c, P.fidx, muls(mul(queue_thr(fb, b, j), c), w), kahan);
+          contribute(fb, P.pixel, P.fidx, muls(mul(queue_thr(fb, b, j), c), w), kahan);
         }
       } else {
         P.alive = true;
@@ -201,7 +214,7 @@ __device__ __forceinline__ void shade_hit(const DevScene& S, const DevEnv& E, Re
       if (MODE == 1 && mesh_lights<L>(S)) pdfW = pdfW * 0.5f;
       float w = 1.f;
       if (!P.spec) w = mis2(P.ps.w, pdfW);
-      film_add(fb.film, fb.film_c, P.fidx, muls(mul(queue_thr(fb, b, j), c), w), kahan);
+      contribute(fb, P.pixel, P.fidx, muls(mul(queue_thr(fb, b, j), c), w), kahan);
     }
   }
 }
@@ -310,7 +323,7 @@ __device__ __forceinline__ void shade_continue(const DevScene& S, const DevEnv& 
     const float w = mis2(pdfW, bpdf);
     const float sc = (w * cosL / (pick * pdfW));
     R.shc = mk(sc * (rad.x * fl.x) * P.thr.x, sc * (rad.y * fl.y) * P.thr.y, sc * (rad.z * fl.z) * P.thr.z, 1.f);
-    R.sho = mk(P.H.p.x, P.H.p.y, P.H.p.z, __int_as_float(P.fidx));
+    R.sho = mk(P.H.p.x, P.H.p.y, P.H.p.z, __int_as_float(fb.log ? P.pixel : P.fidx));
     R.shd = mk(dir.x, dir.y, dir.z, dist - 2.f * 1e-3f);
     R.has_shadow = true;
   }

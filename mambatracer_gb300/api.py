@@ -143,8 +143,8 @@ class Scene:
         """The preview device's frame (CDeviceRT): ARGB ints and the material group per pixel."""
         cam = np.ascontiguousarray(camera)
         assert cam.dtype == layout.CAMERA
-        argb = np.zeros(width * height, np.int32)
-        group = np.zeros(width * height, np.int32)
+        argb = np.empty(width * height, np.int32)
+        group = np.empty(width * height, np.int32)
         check(lib().mt_preview_frame(self.h, _p(cam), width, height, _p(argb), _p(group)))
         return argb, group
 
@@ -155,15 +155,15 @@ class Scene:
     def trace_closest(self, rays: np.ndarray):
         rays = np.ascontiguousarray(rays)
         assert rays.dtype == layout.RAY
-        t = np.zeros(rays.shape[0], np.float32)
-        prim = np.zeros(rays.shape[0], np.int32)
+        t = np.empty(rays.shape[0], np.float32)
+        prim = np.empty(rays.shape[0], np.int32)
         check(lib().mt_trace_closest(self.h, _p(rays), rays.shape[0], _p(t), _p(prim)))
         return t, prim
 
     def trace_any(self, rays: np.ndarray):
         rays = np.ascontiguousarray(rays)
         assert rays.dtype == layout.RAY
-        occ = np.zeros(rays.shape[0], np.int32)
+        occ = np.empty(rays.shape[0], np.int32)
         check(lib().mt_trace_any(self.h, _p(rays), rays.shape[0], _p(occ)))
         return occ
 
@@ -210,7 +210,7 @@ class Job:
         check(lib().mt_render_frame(self.h, _p(seeds), float(frame_count)))
 
     def film(self, resolve: bool = False) -> np.ndarray:
-        out = np.zeros((self.width * self.height, 4), np.float32)
+        out = np.empty((self.width * self.height, 4), np.float32)
         check(lib().mt_film_read(self.h, _p(out), int(resolve)))
         return out
 
@@ -227,7 +227,7 @@ class Job:
 
     def image(self, exposure: float = 0.18, gamma: float = 2.2):
         """The displayed ARGB image (int32 per pixel) and the log-average luminance."""
-        out = np.zeros(self.width * self.height, np.int32)
+        out = np.empty(self.width * self.height, np.int32)
         la = C.c_float()
         check(lib().mt_image_argb(self.h, _p(out), float(exposure), float(gamma), C.byref(la)))
         return out, la.value
@@ -464,7 +464,7 @@ def batch_render(ctx: Context, scene: Scene, frames, max_depth: int = 8, rr_dept
         f.width, f.height, f.spp, f.frame_count = int(w), int(h), int(spp), float(fc)
         C.memmove(f.camera, np.frombuffer(c.tobytes(), np.uint8).ctypes.data, 64)
     sizes = [int(w) * int(h) for _, w, h, _, _ in frames]
-    out = np.zeros((sum(sizes), 4), np.float32)
+    out = np.empty((sum(sizes), 4), np.float32)
     rays = np.zeros(3, np.int64)
     check(lib().mt_batch_render(ctx.h, scene.h, C.cast(arr, C.c_void_p), len(frames), max_depth, rr_depth, film_kahan,
                                 _p(out), _p(rays)))

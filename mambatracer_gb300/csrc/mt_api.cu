@@ -51,6 +51,40 @@ void join_jobs(mt_context* ctx) {
   }
 }
 
+int Workspace::get(mt_context* c, size_t bytes) {
+  ctx = c;
+  at = 0;
+  own = bytes > kWorkspaceMax;
+  if (own) return dalloc(&base, bytes);
+  if (bytes > c->ws_bytes) {
+    // grown in steps, so calls of slowly growing sizes do not allocate each time
+    const size_t grown = std::min(kWorkspaceMax, std::max({bytes, 2 * c->ws_bytes, (size_t)1 << 20}));
+    cudaStreamSynchronize(c->stream);
+    dfree(c->ws);
+    c->ws_bytes = 0;
+    int r = dalloc(&c->ws, grown);
+    if (r) return r;
+    c->ws_bytes = grown;
+  }
+  base = c->ws;
+  return MT_OK;
+}
+
+void Workspace::release() {
+  if (own) dfree(base);
+  base = nullptr;
+}
+
+void prefault(void* p, size_t bytes, cudaEvent_t ready) {
+  constexpr size_t kPage = 4096, kStep = 64 * kPage;
+  auto* b = static_cast<volatile char*>(p);
+  for (size_t o = 0; o < bytes; o += kStep) {
+    if (cudaEventQuery(ready) != cudaErrorNotReady) return;
+    cudaGetLastError();  // not ready is not an error
+    for (size_t q = o; q < std::min(bytes, o + kStep); q += kPage) b[q] = 0;
+  }
+}
+
 extern "C" const char* mt_version(void) {
   return "mambatracer-gb300 sm_103a fmad=false prec-div prec-sqrt";
 }
@@ -82,6 +116,7 @@ extern "C" int mt_ctx_create(int device, mt_context** out) {
     return MT_ERR_NOMEM;
   }
   for (auto& ev : c->ev) cudaEventCreate(&ev);
+  cudaEventCreateWithFlags(&c->ready, cudaEventDisableTiming);
   *out = c;
   return MT_OK;
 }
@@ -91,11 +126,13 @@ extern "C" int mt_ctx_destroy(mt_context* ctx) {
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->stream);
   dfree(ctx->d_scratch);
+  dfree(ctx->ws);
   dfree(ctx->cs_status);
   dfree(ctx->cs_words);
   dfree(ctx->d_plain_err);
   for (auto& ev : ctx->ev)
     if (ev) cudaEventDestroy(ev);
+  if (ctx->ready) cudaEventDestroy(ctx->ready);
   cudaStreamDestroy(ctx->stream);
   delete ctx;
   return MT_OK;
@@ -840,36 +877,35 @@ int query(mt_scene* s, const void* rays, int n, int any, float* t_out, int32_t* 
   mt_context* ctx = s->ctx;
   std::lock_guard<std::recursive_mutex> lk(ctx->mu);
   CU(cudaSetDevice(ctx->device));
-  float4* d_rays = nullptr;
-  float* d_t = nullptr;
-  int* d_p = nullptr;
-  int* d_c = nullptr;
-  int r = dalloc(&d_rays, 5 * (size_t)n);
-  if (!r) r = dalloc(&d_t, (size_t)n);
-  if (!r) r = dalloc(&d_p, (size_t)n);
-  if (!r && counts_out) r = dalloc(&d_c, 2 * (size_t)n);
-  if (!r) {
-    cudaMemcpyAsync(d_rays, rays, 80 * (size_t)n, cudaMemcpyHostToDevice, ctx->stream);
-    cudaMemsetAsync(ctx->d_scratch, 0, 8, ctx->stream);
-    const int lr = counts_out ? launch_count(ctx->stream, s->view(), d_rays, n, any, d_t, d_p, d_c, ctx->d_scratch + 1)
-                              : launch_query(ctx->stream, s->view(), d_rays, n, any, d_t, d_p, ctx->d_scratch,
-                                             ctx->d_scratch + 1, ctx->num_sms);
-    if (lr) r = fail(MT_ERR_CUDA, "query launch: %s", cudaGetErrorString(cudaGetLastError()));
-  }
+  const size_t bytes = Workspace::round(80 * (size_t)n) + 2 * Workspace::round(4 * (size_t)n) +
+                       (counts_out ? Workspace::round(8 * (size_t)n) : 0);
+  Workspace ws;
+  int r = ws.get(ctx, bytes);
+  if (r) return r;
+  float4* d_rays = ws.take<float4>(5 * (size_t)n);
+  float* d_t = ws.take<float>((size_t)n);
+  int* d_p = ws.take<int>((size_t)n);
+  int* d_c = counts_out ? ws.take<int>(2 * (size_t)n) : nullptr;
+  cudaMemcpyAsync(d_rays, rays, 80 * (size_t)n, cudaMemcpyHostToDevice, ctx->stream);
+  cudaMemsetAsync(ctx->d_scratch, 0, 8, ctx->stream);
+  const int lr = counts_out ? launch_count(ctx->stream, s->view(), d_rays, n, any, d_t, d_p, d_c, ctx->d_scratch + 1)
+                            : launch_query(ctx->stream, s->view(), d_rays, n, any, d_t, d_p, ctx->d_scratch,
+                                           ctx->d_scratch + 1, ctx->num_sms);
+  if (lr) r = fail(MT_ERR_CUDA, "query launch: %s", cudaGetErrorString(cudaGetLastError()));
   int err = 0;
   if (!r) {
+    cudaEventRecord(ctx->ready, ctx->stream);
+    if (!any) prefault(t_out, 4 * (size_t)n, ctx->ready);
+    prefault(prim_out, 4 * (size_t)n, ctx->ready);
     if (!any) cudaMemcpyAsync(t_out, d_t, 4 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream);
     cudaMemcpyAsync(prim_out, d_p, 4 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream);
     if (counts_out) cudaMemcpyAsync(counts_out, d_c, 8 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream);
     cudaMemcpyAsync(&err, ctx->d_scratch + 1, 4, cudaMemcpyDeviceToHost, ctx->stream);
-    cudaError_t e = cudaStreamSynchronize(ctx->stream);
-    if (e != cudaSuccess) r = fail(MT_ERR_CUDA, "query: %s", cudaGetErrorString(e));
-    else if (err) r = fail(MT_ERR_DEVICE, "device error %d", err);
   }
-  dfree(d_rays);
-  dfree(d_t);
-  dfree(d_p);
-  dfree(d_c);
+  const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+  if (!r && e != cudaSuccess) r = fail(MT_ERR_CUDA, "query: %s", cudaGetErrorString(e));
+  else if (!r && err) r = fail(MT_ERR_DEVICE, "device error %d", err);
+  ws.release();
   return r;
 }
 }  // namespace

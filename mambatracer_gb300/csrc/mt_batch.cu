@@ -16,30 +16,6 @@
 
 #include "mt_internal.h"
 
-namespace {
-
-void free_bufs(FrameBufs& fb) {
-  for (auto* p : {&fb.q_o[0], &fb.q_o[1], &fb.q_d[0], &fb.q_d[1], &fb.q_t[0], &fb.q_t[1], &fb.s_o, &fb.s_d, &fb.s_c,
-                  &fb.film, &fb.film_c})
-    dfree(*p);
-  dfree(fb.hit_t);
-  dfree(fb.hit_prim);
-  dfree(fb.live);
-}
-
-int alloc_bufs(FrameBufs& fb, size_t n) {
-  int r = MT_OK;
-  for (auto* p : {&fb.q_o[0], &fb.q_o[1], &fb.q_d[0], &fb.q_d[1], &fb.q_t[0], &fb.q_t[1], &fb.s_o, &fb.s_d, &fb.s_c,
-                  &fb.film, &fb.film_c})
-    if (!r) r = dalloc(p, n);
-  if (!r) r = dalloc(&fb.hit_t, n);
-  if (!r) r = dalloc(&fb.hit_prim, n);
-  if (!r) r = dalloc(&fb.live, n);
-  return r;
-}
-
-}  // namespace
-
 extern "C" int mt_batch_render(mt_context* ctx, mt_scene* s, const mt_batch_frame* frames, int nframes, int max_depth,
                                int rr_depth, int film_kahan, float* films_out, int64_t* rays_out) {
   if (!ctx || !s || !frames || !films_out || nframes <= 0) return fail(MT_ERR_INVALID, "bad argument");
@@ -95,28 +71,28 @@ extern "C" int mt_batch_render(mt_context* ctx, mt_scene* s, const mt_batch_fram
     tot[p] = g;
   }
 
+  Workspace ws;
+  auto R = [](size_t b) { return Workspace::round(b); };
+  int r = ws.get(ctx, 11 * R(total * 16) + 3 * R(total * 4) + R(sizeof(Ctrl) * (size_t)max_spp) + R(h_start.size() * 4) +
+                          R(h_film.size() * 4) + R(h_pp.size() * sizeof(PassParams)) + R(32));
+  if (r) return r;
   FrameBufs fb{};
-  Ctrl* d_ctrl = nullptr;
-  int *d_start = nullptr, *d_film = nullptr;
-  PassParams* d_pp = nullptr;
-  unsigned long long* d_totals = nullptr;
-  int r = alloc_bufs(fb, total);
-  if (!r) r = dalloc(&d_ctrl, (size_t)max_spp);
-  if (!r) r = dalloc(&d_start, h_start.size());
-  if (!r) r = dalloc(&d_film, h_film.size());
-  if (!r) r = dalloc(&d_pp, h_pp.size());
-  if (!r) r = dalloc(&d_totals, 4);
+  for (auto* p : {&fb.q_o[0], &fb.q_o[1], &fb.q_d[0], &fb.q_d[1], &fb.q_t[0], &fb.q_t[1], &fb.s_o, &fb.s_d, &fb.s_c,
+                  &fb.film, &fb.film_c})
+    *p = ws.take<float4>(total);
+  fb.hit_t = ws.take<float>(total);
+  fb.hit_prim = ws.take<int>(total);
+  fb.live = ws.take<int>(total);
+  Ctrl* d_ctrl = ws.take<Ctrl>((size_t)max_spp);
+  int* d_start = ws.take<int>(h_start.size());
+  int* d_film = ws.take<int>(h_film.size());
+  PassParams* d_pp = ws.take<PassParams>(h_pp.size());
+  unsigned long long* d_totals = ws.take<unsigned long long>(4);
   auto done = [&](int code) {
     cudaStreamSynchronize(st);
-    free_bufs(fb);
-    dfree(d_ctrl);
-    dfree(d_start);
-    dfree(d_film);
-    dfree(d_pp);
-    dfree(d_totals);
+    ws.release();
     return code;
   };
-  if (r) return done(r);
   cudaError_t e = cudaMemsetAsync(fb.film, 0, total * 16, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(fb.film_c, 0, total * 16, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_ctrl, 0, sizeof(Ctrl) * (size_t)max_spp, st);
@@ -128,27 +104,14 @@ extern "C" int mt_batch_render(mt_context* ctx, mt_scene* s, const mt_batch_fram
   if (e != cudaSuccess) return done(fail(MT_ERR_CUDA, "batch set-up: %s", cudaGetErrorString(e)));
   const DevScene S = s->view();
   const DevEnv E = s->env_view();  // full-map environment sampling
-  // every pass of the batch (per pass: raygen, per bounce closest hits, shading
-  // and shadow rays, ray totals) captured into one CUDA graph and launched once
-  e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
-  if (e != cudaSuccess) return done(fail(MT_ERR_CUDA, "batch capture: %s", cudaGetErrorString(e)));
-  int lr = 0;
-  for (int p = 0; p < max_spp && !lr; ++p)
-    lr = launch_batch_pass(st, S, E, d_start + (size_t)p * (nframes + 1), d_film + (size_t)p * nframes,
-                           d_pp + (size_t)p * nframes, nact[p], tot[p], max_depth, film_kahan, d_ctrl + p, fb,
-                           ctx->num_sms, d_totals);
-  cudaGraph_t graph = nullptr;
-  e = cudaStreamEndCapture(st, &graph);
-  if (lr || e != cudaSuccess) {
-    if (graph) cudaGraphDestroy(graph);
-    return done(fail(MT_ERR_CUDA, "batch pass capture: %s", cudaGetErrorString(lr ? cudaGetLastError() : e)));
-  }
-  cudaGraphExec_t exec = nullptr;
-  e = cudaGraphInstantiate(&exec, graph, 0);
-  cudaGraphDestroy(graph);
-  if (e == cudaSuccess) e = cudaGraphLaunch(exec, st);
-  if (exec) cudaGraphExecDestroy(exec);  // released once the launch completes
-  if (e != cudaSuccess) return done(fail(MT_ERR_CUDA, "batch graph: %s", cudaGetErrorString(e)));
+  for (int p = 0; p < max_spp; ++p)
+    if (launch_batch_pass(st, S, E, d_start + (size_t)p * (nframes + 1), d_film + (size_t)p * nframes,
+                          d_pp + (size_t)p * nframes, nact[p], tot[p], max_depth, film_kahan, d_ctrl + p, fb,
+                          ctx->num_sms, d_totals))
+      return done(fail(MT_ERR_CUDA, "batch pass: %s", cudaGetErrorString(cudaGetLastError())));
+  e = cudaEventRecord(ctx->ready, st);
+  if (e != cudaSuccess) return done(fail(MT_ERR_CUDA, "batch: %s", cudaGetErrorString(e)));
+  prefault(films_out, total * 16, ctx->ready);
   unsigned long long h_tot[4] = {0, 0, 0, 0};
   e = cudaMemcpyAsync(films_out, fb.film, total * 16, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(h_tot, d_totals, 32, cudaMemcpyDeviceToHost, st);

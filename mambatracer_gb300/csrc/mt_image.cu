@@ -182,6 +182,8 @@ extern "C" int mt_image_argb(mt_job* j, int32_t* argb, float exposure, float gam
     k_tone_map<<<(n + 255) / 256, 256, 0, ctx->stream>>>(j->d_fb, n, j->d_tone_tot, exposure, gamma, j->d_argb);
     CU(cudaGetLastError());
   }
+  CU(cudaEventRecord(ctx->ready, ctx->stream));
+  prefault(argb, (size_t)n * 4, ctx->ready);
   float tot[2] = {0.f, 0.f};
   CU(cudaMemcpyAsync(argb, j->d_argb, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));
   if (log_average && j->frames > 0) CU(cudaMemcpyAsync(tot, j->d_tone_tot, 8, cudaMemcpyDeviceToHost, ctx->stream));

@@ -743,6 +743,7 @@ extern "C" int mt_film_read(mt_job* j, float* rgba, int resolve) {
   mt_context* ctx = j->ctx;
   std::lock_guard<std::recursive_mutex> lk(ctx->mu);
   CU(cudaSetDevice(ctx->device));
+  if (j->last >= 0) prefault(rgba, (size_t)j->cfg.width * j->cfg.height * 16, j->slots[j->last].done);
   mt_job::Read* rd = nullptr;
   int r = enqueue_read(j, rgba, resolve, &rd);
   return r ? r : finish_reads(j);

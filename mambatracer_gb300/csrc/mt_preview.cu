@@ -106,24 +106,30 @@ extern "C" int mt_preview_frame(mt_scene* s, const void* camera, int width, int 
   camera_constants(camera, width, height, pp);
   pp.width = width;
   pp.height = height;
-  int *d_argb = nullptr, *d_group = nullptr;
-  CU(cudaMallocAsync((void**)&d_argb, (size_t)n * 4, ctx->stream));
-  if (group) CU(cudaMallocAsync((void**)&d_group, (size_t)n * 4, ctx->stream));
-  CU(cudaMemsetAsync(ctx->d_scratch, 0, 8, ctx->stream));
+  Workspace ws;
+  if (int r = ws.get(ctx, 2 * Workspace::round((size_t)n * 4))) return r;
+  int* d_argb = ws.take<int>((size_t)n);
+  int* d_group = group ? ws.take<int>((size_t)n) : nullptr;
+  cudaError_t e = cudaMemsetAsync(ctx->d_scratch, 0, 8, ctx->stream);
   int bps = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, mt::k_preview, kTraceThreads, 0);
   const int grid = std::max(1, std::min(ctx->num_sms * std::max(bps, 1), (n + kTraceThreads - 1) / kTraceThreads));
   mt::k_preview<<<grid, kTraceThreads, 0, ctx->stream>>>(s->view(), s->env_view(), pp, n, d_argb, d_group,
                                                          ctx->d_scratch, ctx->d_scratch + 1);
-  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaGetLastError();
   int err = 0;
+  if (e == cudaSuccess) e = cudaEventRecord(ctx->ready, ctx->stream);
+  if (e == cudaSuccess) {
+    prefault(argb, (size_t)n * 4, ctx->ready);
+    if (group) prefault(group, (size_t)n * 4, ctx->ready);
+  }
   if (e == cudaSuccess) e = cudaMemcpyAsync(argb, d_argb, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess && group)
     e = cudaMemcpyAsync(group, d_group, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(&err, ctx->d_scratch + 1, 4, cudaMemcpyDeviceToHost, ctx->stream);
-  cudaFreeAsync(d_argb, ctx->stream);
-  if (d_group) cudaFreeAsync(d_group, ctx->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  const cudaError_t w = cudaStreamSynchronize(ctx->stream);
+  ws.release();
+  if (e == cudaSuccess) e = w;
   if (e != cudaSuccess) return fail(MT_ERR_CUDA, "preview: %s", cudaGetErrorString(e));
   if (err) return fail(MT_ERR_DEPTH, "BVH deeper than the traversal stack");
   return MT_OK;

@@ -127,6 +127,12 @@ extern "C" int mt_ctx_destroy(mt_context* ctx) {
   cudaStreamSynchronize(ctx->stream);
   dfree(ctx->d_scratch);
   dfree(ctx->ws);
+  for (auto& p : ctx->pass_streams) {
+    for (cudaEvent_t e : {p.fork, p.join, p.done})
+      if (e) cudaEventDestroy(e);
+    for (cudaStream_t q : {p.stream, p.side})
+      if (q) cudaStreamDestroy(q);
+  }
   dfree(ctx->cs_status);
   dfree(ctx->cs_words);
   dfree(ctx->d_plain_err);

@@ -71,30 +71,60 @@ extern "C" int mt_batch_render(mt_context* ctx, mt_scene* s, const mt_batch_fram
     tot[p] = g;
   }
 
-  Workspace ws;
+  // Passes overlap as a job's do (mt_job.cu), as far as the kept scratch holds them.
   auto R = [](size_t b) { return Workspace::round(b); };
-  int r = ws.get(ctx, 11 * R(total * 16) + 3 * R(total * 4) + R(sizeof(Ctrl) * (size_t)max_spp) + R(h_start.size() * 4) +
-                          R(h_film.size() * 4) + R(h_pp.size() * sizeof(PassParams)) + R(32));
+  const size_t fixed = 2 * R(total * 16) + R(sizeof(Ctrl) * (size_t)max_spp) + R(h_start.size() * 4) +
+                       R(h_film.size() * 4) + R(h_pp.size() * sizeof(PassParams)) + R(32);
+  const size_t queues = 9 * R(total * 16) + 3 * R(total * 4),
+               log = R(total * 16 * 2 * (size_t)max_depth) + R(total * 4);
+  const size_t room = kWorkspaceMax > fixed ? (kWorkspaceMax - fixed) / (queues + log) : 0;
+  const int nbuf = (int)std::max<size_t>(1, std::min<size_t>({room, (size_t)max_spp, 4}));
+  const bool logged = nbuf > 1;
+  while ((int)ctx->pass_streams.size() < nbuf) {
+    mt_context::PassStream p;
+    cudaError_t e = cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&p.side, cudaStreamNonBlocking);
+    for (cudaEvent_t* v : {&p.fork, &p.join, &p.done})
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(v, cudaEventDisableTiming);
+    ctx->pass_streams.push_back(p);  // also a half-made one: the context frees it
+    if (e != cudaSuccess) return fail(MT_ERR_CUDA, "batch streams: %s", cudaGetErrorString(e));
+  }
+  Workspace ws;
+  int r = ws.get(ctx, fixed + nbuf * (queues + (logged ? log : 0)));
   if (r) return r;
-  FrameBufs fb{};
-  for (auto* p : {&fb.q_o[0], &fb.q_o[1], &fb.q_d[0], &fb.q_d[1], &fb.q_t[0], &fb.q_t[1], &fb.s_o, &fb.s_d, &fb.s_c,
-                  &fb.film, &fb.film_c})
-    *p = ws.take<float4>(total);
-  fb.hit_t = ws.take<float>(total);
-  fb.hit_prim = ws.take<int>(total);
-  fb.live = ws.take<int>(total);
+  float4* film = ws.take<float4>(total);
+  float4* film_c = ws.take<float4>(total);
+  std::vector<FrameBufs> fbs(nbuf);
+  for (FrameBufs& fb : fbs) {
+    for (auto* p : {&fb.q_o[0], &fb.q_o[1], &fb.q_d[0], &fb.q_d[1], &fb.q_t[0], &fb.q_t[1], &fb.s_o, &fb.s_d, &fb.s_c})
+      *p = ws.take<float4>(total);
+    fb.hit_t = ws.take<float>(total);
+    fb.hit_prim = ws.take<int>(total);
+    fb.live = ws.take<int>(total);
+    fb.film = film;
+    fb.film_c = film_c;
+    if (logged) {
+      fb.log = ws.take<float4>(total * 2 * (size_t)max_depth);
+      fb.log_n = ws.take<int>(total);
+      fb.log_stride = (int)total;
+    }
+  }
   Ctrl* d_ctrl = ws.take<Ctrl>((size_t)max_spp);
   int* d_start = ws.take<int>(h_start.size());
   int* d_film = ws.take<int>(h_film.size());
   PassParams* d_pp = ws.take<PassParams>(h_pp.size());
   unsigned long long* d_totals = ws.take<unsigned long long>(4);
   auto done = [&](int code) {
+    for (int k = 0; k < nbuf; ++k) {
+      cudaStreamSynchronize(ctx->pass_streams[k].stream);
+      cudaStreamSynchronize(ctx->pass_streams[k].side);
+    }
     cudaStreamSynchronize(st);
     ws.release();
     return code;
   };
-  cudaError_t e = cudaMemsetAsync(fb.film, 0, total * 16, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(fb.film_c, 0, total * 16, st);
+  cudaError_t e = cudaMemsetAsync(film, 0, total * 16, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(film_c, 0, total * 16, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_ctrl, 0, sizeof(Ctrl) * (size_t)max_spp, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_totals, 0, 32, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_start, h_start.data(), h_start.size() * 4, cudaMemcpyHostToDevice, st);
@@ -104,16 +134,45 @@ extern "C" int mt_batch_render(mt_context* ctx, mt_scene* s, const mt_batch_fram
   if (e != cudaSuccess) return done(fail(MT_ERR_CUDA, "batch set-up: %s", cudaGetErrorString(e)));
   const DevScene S = s->view();
   const DevEnv E = s->env_view();  // full-map environment sampling
-  for (int p = 0; p < max_spp; ++p)
-    if (launch_batch_pass(st, S, E, d_start + (size_t)p * (nframes + 1), d_film + (size_t)p * nframes,
-                          d_pp + (size_t)p * nframes, nact[p], tot[p], max_depth, film_kahan, d_ctrl + p, fb,
-                          ctx->num_sms, d_totals))
+  e = cudaEventRecord(ctx->ready, st);  // the set-up
+  for (int k = 0; k < nbuf && e == cudaSuccess; ++k) e = cudaStreamWaitEvent(ctx->pass_streams[k].stream, ctx->ready, 0);
+  if (e != cudaSuccess) return done(fail(MT_ERR_CUDA, "batch set-up: %s", cudaGetErrorString(e)));
+  for (int p = 0; p < max_spp; ++p) {
+    const int k = p % nbuf;
+    mt_context::PassStream& P = ctx->pass_streams[k];
+    const int* start = d_start + (size_t)p * (nframes + 1);
+    const int* fmap = d_film + (size_t)p * nframes;
+    if (launch_batch_pass(P.stream, S, E, start, fmap, d_pp + (size_t)p * nframes, nact[p], tot[p], max_depth, film_kahan,
+                          d_ctrl + p, fbs[k], ctx->num_sms, logged ? nullptr : d_totals, P.side, P.fork, P.join, nbuf))
       return done(fail(MT_ERR_CUDA, "batch pass: %s", cudaGetErrorString(cudaGetLastError())));
+    if (logged) {
+      Replay Rp{};
+      Rp.log[0] = fbs[k].log;
+      Rp.count[0] = fbs[k].log_n;
+      Rp.ctrl[0] = d_ctrl + p;
+      Rp.passes = 1;
+      Rp.stride = (int)total;
+      Rp.n = tot[p];
+      Rp.max_depth = max_depth;
+      Rp.kahan = film_kahan;
+      Rp.start = start;
+      Rp.film = fmap;
+      Rp.frames = nact[p];
+      if (p > 0) e = cudaStreamWaitEvent(P.stream, ctx->pass_streams[(p - 1) % nbuf].done, 0);
+      if (e != cudaSuccess || launch_replay(P.stream, Rp, film, film_c, d_totals))
+        return done(fail(MT_ERR_CUDA, "batch film: %s", cudaGetErrorString(cudaGetLastError())));
+    }
+    e = cudaEventRecord(P.done, P.stream);
+    if (e != cudaSuccess) return done(fail(MT_ERR_CUDA, "batch: %s", cudaGetErrorString(e)));
+  }
+  for (int k = 0; k < std::min(nbuf, max_spp) && e == cudaSuccess; ++k)
+    e = cudaStreamWaitEvent(st, ctx->pass_streams[k].done, 0);
+  if (e != cudaSuccess) return done(fail(MT_ERR_CUDA, "batch: %s", cudaGetErrorString(e)));
   e = cudaEventRecord(ctx->ready, st);
   if (e != cudaSuccess) return done(fail(MT_ERR_CUDA, "batch: %s", cudaGetErrorString(e)));
   prefault(films_out, total * 16, ctx->ready);
   unsigned long long h_tot[4] = {0, 0, 0, 0};
-  e = cudaMemcpyAsync(films_out, fb.film, total * 16, cudaMemcpyDeviceToHost, st);
+  e = cudaMemcpyAsync(films_out, film, total * 16, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(h_tot, d_totals, 32, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return done(fail(MT_ERR_CUDA, "batch: %s", cudaGetErrorString(e)));

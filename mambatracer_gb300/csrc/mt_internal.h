@@ -68,6 +68,12 @@ struct mt_context {
   // previews, batches), kept between them: allocating and freeing it cost 80-280 us a
   // call. Used on `stream` under `mu`, so one call at a time; at most kWorkspaceMax
   // bytes are kept (a larger call allocates its own), and they go with the context.
+  // streams of a batch's overlapping passes, created by the first batch
+  struct PassStream {
+    cudaStream_t stream = nullptr, side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr, done = nullptr;
+  };
+  std::vector<PassStream> pass_streams;
   char* ws = nullptr;
   size_t ws_bytes = 0;
   std::vector<mt_job*> jobs;  // jobs whose streams join into `stream`

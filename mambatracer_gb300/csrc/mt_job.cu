@@ -404,13 +404,13 @@ bool replay_inside(const mt_job* j) { return j->merge || j->nslots == 1; }
 int replay(mt_job* j, JobSlot& s, cudaStream_t st, int p, int n) {
   Replay R{};
   R.passes = n;
-  R.stride = j->cfg.width * j->cfg.height;
+  R.n = R.stride = j->cfg.width * j->cfg.height;
   R.max_depth = j->cfg.max_depth;
   R.kahan = j->cfg.film_kahan;
   for (int i = 0; i < n; ++i) {
     const FrameBufs& fb = s.bufs[(p + i) % s.bufs.size()].fb;
     R.log[i] = fb.log;
-    R.n[i] = fb.log_n;
+    R.count[i] = fb.log_n;
     R.ctrl[i] = s.d_ctrl + p + i;
   }
   return j->merge ? launch_replay(st, R, s.film, s.film_c, j->d_totals)

@@ -143,20 +143,26 @@ __global__ void k_replay(Replay R, float4* __restrict__ film, float4* __restrict
     const Ctrl& c = *R.ctrl[i];
     unsigned long long ext = 0;
     for (int b = 2; b <= R.max_depth; ++b) ext += (unsigned long long)c.count[b];
-    atomicAdd(totals + 0, (unsigned long long)R.stride);
+    atomicAdd(totals + 0, (unsigned long long)R.n);
     atomicAdd(totals + 1, ext);
     atomicAdd(totals + 2, c.rays[2]);
     if (c.error) atomicExch(totals + 3, (unsigned long long)c.error);
   }
-  if (i >= R.stride) return;
+  if (i >= R.n) return;
   int n[kReplayPasses], any = 0;
 #pragma unroll
   for (int p = 0; p < kReplayPasses; ++p) {
-    n[p] = p < R.passes ? R.n[p][i] : 0;
+    n[p] = p < R.passes ? R.count[p][i] : 0;
     any |= n[p];
   }
   if (!any) return;
-  V a = film[i], c = R.kahan ? film_c[i] : zero4();
+  int px = i;
+  if (R.frames) {
+    PathState P;
+    BatchFrames{R.start, R.film, nullptr, R.frames}(i, P);
+    px = P.fidx;
+  }
+  V a = film[px], c = R.kahan ? film_c[px] : zero4();
 #pragma unroll
   for (int p = 0; p < kReplayPasses; ++p)
     for (int k = 0; k < n[p]; ++k) {
@@ -169,11 +175,11 @@ __global__ void k_replay(Replay R, float4* __restrict__ film, float4* __restrict
       c = sub(sub(t, a), y);
       a = t;
     }
-  film[i] = a;
-  if (R.kahan) film_c[i] = c;
+  film[px] = a;
+  if (R.kahan) film_c[px] = c;
 }
 int launch_replay(cudaStream_t st, const Replay& R, float4* film, float4* film_c, unsigned long long* totals) {
-  k_replay<<<(R.stride + 255) / 256, 256, 0, st>>>(R, film, film_c, totals);
+  k_replay<<<(R.n + 255) / 256, 256, 0, st>>>(R, film, film_c, totals);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -384,14 +390,25 @@ __global__ void k_raygen_batch(BatchFrames B, int total, Ctrl* ctrl, FrameBufs f
 
 int launch_batch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const int* d_start, const int* d_film,
                       const PassParams* d_pp, int nframes, int total, int max_depth, int kahan, Ctrl* ctrl,
-                      FrameBufs fb, int num_sms, unsigned long long* totals, bool shared, int min_lanes) {
+                      FrameBufs fb, int num_sms, unsigned long long* totals, cudaStream_t side, cudaEvent_t fork,
+                      cudaEvent_t join, int beside) {
   const BatchFrames B{d_start, d_film, d_pp, nframes};
+  const bool split = tuning_ref().shadow_stream, two = shade_split(total, beside > 1);
+  const int lanes = tail_lanes(S, beside);
   k_raygen_batch<<<(total + 255) / 256, 256, 0, st>>>(B, total, ctrl, fb);
+  // shadow rays beside the next bounce's extension rays, as in launch_pass
   for (int b = 1; b <= max_depth; ++b) {
-    launch_trace(st, S, ctrl, b, 1, fb, kahan, true, total, num_sms, shared, min_lanes);
-    launch_shade_batch(st, S, E, d_start, d_film, d_pp, nframes, shade_split(total, shared), num_sms, total, ctrl, b, fb);
-    launch_trace(st, S, ctrl, b, 1, fb, kahan, false, total, num_sms, shared, min_lanes);
+    launch_trace(st, S, ctrl, b, 1, fb, kahan, true, total, num_sms, split || beside > 1, lanes);
+    if (split && b > 1) cudaStreamWaitEvent(st, join, 0);
+    launch_shade_batch(st, S, E, d_start, d_film, d_pp, nframes, two, num_sms, total, ctrl, b, fb);
+    if (split) {
+      cudaEventRecord(fork, st);
+      cudaStreamWaitEvent(side, fork, 0);
+    }
+    launch_trace(split ? side : st, S, ctrl, b, 1, fb, kahan, false, total, num_sms, split || beside > 1, lanes);
+    if (split) cudaEventRecord(join, side);
   }
+  if (split) cudaStreamWaitEvent(st, join, 0);
   if (totals) k_accumulate<<<1, 32, 0, st>>>(ctrl, max_depth, total, totals);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

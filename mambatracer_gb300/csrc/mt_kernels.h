@@ -32,9 +32,13 @@ struct FrameBufs {
 constexpr int kReplayPasses = 4;
 struct Replay {
   const float4* log[kReplayPasses];
-  const int* n[kReplayPasses];
+  const int* count[kReplayPasses];
   const Ctrl* ctrl[kReplayPasses];
   int passes, stride, max_depth, kahan;
+  int n;  // paths of a pass
+  // merged batch passes: path to pixel as in launch_batch_pass; frames 0: pixel = path
+  const int *start, *film;
+  int frames;
 };
 int launch_replay(cudaStream_t st, const Replay& R, float4* film, float4* film_c, unsigned long long* totals);
 
@@ -82,7 +86,8 @@ unsigned tuning_version();         // bumped by every set_tuning (jobs recapture
 // d_film[k], its parameters are d_pp[k]. total = d_start[nframes].
 int launch_batch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const int* d_start, const int* d_film,
                       const PassParams* d_pp, int nframes, int total, int max_depth, int kahan, Ctrl* ctrl,
-                      FrameBufs fb, int num_sms, unsigned long long* totals, bool shared = false, int min_lanes = 1);
+                      FrameBufs fb, int num_sms, unsigned long long* totals, cudaStream_t side, cudaEvent_t fork,
+                      cudaEvent_t join, int beside);
 int launch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const PassParams* d_pp, int mode,
                 int max_depth, int kahan, int width, int height, Ctrl* ctrl, FrameBufs fb,
                 unsigned long long* status, size_t status_stride, int num_sms, cudaEvent_t* events,

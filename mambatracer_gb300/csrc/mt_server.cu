@@ -104,6 +104,8 @@ constexpr size_t kGraphsPerStream = 16;  // scenes whose merged-pass graph a mer
 struct MergeGroup {
   struct mt_server* server = nullptr;
   cudaStream_t stream = nullptr;
+  cudaStream_t side = nullptr;  // shadow rays beside the next bounce's extension rays
+  cudaEvent_t sfork = nullptr, sjoin = nullptr;
   std::vector<int> slots;
   FrameBufs fb{};  // path state of its slots' paths; the films of the whole arena
   Round rounds[kRounds];
@@ -293,6 +295,12 @@ void free_merged(mt_server* s) {
     G.graphs.clear();
     if (G.stream) cudaStreamDestroy(G.stream);
     G.stream = nullptr;
+    if (G.side) cudaStreamDestroy(G.side);
+    G.side = nullptr;
+    for (cudaEvent_t* e : {&G.sfork, &G.sjoin}) {
+      if (*e) cudaEventDestroy(*e);
+      *e = nullptr;
+    }
   }
 }
 
@@ -332,7 +340,10 @@ int alloc_merged(mt_server* s, size_t N, int m) {
       if (!r && cudaEventCreateWithFlags(&Rd.done, cudaEventDisableTiming) != cudaSuccess)
         r = fail(MT_ERR_CUDA, "event create");
     }
-    if (!r && cudaStreamCreateWithFlags(&G.stream, cudaStreamNonBlocking) != cudaSuccess)
+    if (!r && (cudaStreamCreateWithFlags(&G.stream, cudaStreamNonBlocking) != cudaSuccess ||
+               cudaStreamCreateWithFlags(&G.side, cudaStreamNonBlocking) != cudaSuccess ||
+               cudaEventCreateWithFlags(&G.sfork, cudaEventDisableTiming) != cudaSuccess ||
+               cudaEventCreateWithFlags(&G.sjoin, cudaEventDisableTiming) != cudaSuccess))
       r = fail(MT_ERR_CUDA, "stream create");
     if (r) break;
     G.fb = s->mfb;  // films stay whole: slot k's film is at k x N
@@ -439,8 +450,7 @@ int issue_round(mt_server* s, MergeGroup& G, const std::vector<int>& work, const
     CU(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     const int lr = launch_batch_pass(st, S, E, Rd.d_tab + Gr.tab, Rd.d_tab + Gr.tab + Gr.n + 1, Rd.d_pp + Gr.pp,
                                      Gr.n, Gr.total, c.max_depth, c.film_kahan, Rd.d_ctrl + g, G.fb,
-                                     s->ctx->num_sms, s->d_totals, s->groups.size() > 1,
-                                     tail_lanes(S, (int)s->groups.size()));
+                                     s->ctx->num_sms, s->d_totals, G.side, G.sfork, G.sjoin, (int)s->groups.size());
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(st, &graph);
     if (lr || e != cudaSuccess) {

@@ -2,6 +2,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cstdlib>
 #include <cmath>
 #include <cstdarg>
@@ -263,22 +264,12 @@ bool emitter_host(const Material& m) {
   return (0.2989f * x + 0.5866f * y) + 0.1145f * z != 0.0f;
 }
 
+// The mesh lights of the scene's materials.
 int upload_lights(mt_scene* s) {
-  // identifyMeshLights + prefix scan + prepareLightInfo (CLightConfiguration.java:43-87):
-  // the faces whose material emits, in face order.
-  std::vector<int> lf;
-  const Face* F = reinterpret_cast<const Face*>(s->h_faces.data());
   const Material* M = reinterpret_cast<const Material*>(s->h_materials.data());
-  for (int i = 0; i < s->ntri; ++i) {
-    int m = F[i].mat & 0xFFFF;
-    if (emitter_host(M[m])) lf.push_back(i);
-  }
-  dfree(s->d_light_faces);
-  s->nlights = (int)lf.size();
-  int r = dalloc(&s->d_light_faces, lf.size());
-  if (r) return r;
-  if (!lf.empty()) CU(cudaMemcpy(s->d_light_faces, lf.data(), lf.size() * 4, cudaMemcpyHostToDevice));
-  return MT_OK;
+  std::vector<unsigned char> emits(s->nmat);
+  for (int m = 0; m < s->nmat; ++m) emits[m] = emitter_host(M[m]);
+  return list_light_faces(s, emits);
 }
 
 template <class T>
@@ -291,10 +282,11 @@ int upload(T** d, const void* h, size_t count) {
 }
 
 void free_scene(mt_scene* s) {
-  dfree(s->d_points);
-  dfree(s->d_uvs);
-  dfree(s->d_normals);
-  dfree(s->d_faces);
+  dfree(s->d_mesh);
+  s->d_points = nullptr;
+  s->d_uvs = nullptr;
+  s->d_normals = nullptr;
+  s->d_faces = nullptr;
   dfree(s->d_materials);
   dfree(s->d_light_faces);
   dfree(s->d_nodes);
@@ -366,18 +358,8 @@ extern "C" int mt_scene_create(mt_context* ctx, const float* points, int npoints
   if (!ctx || !out || !points || !faces || !materials) return fail(MT_ERR_INVALID, "NULL argument");
   if (npoints <= 0 || nfaces <= 0 || nmaterials <= 0) return fail(MT_ERR_INVALID, "empty scene");
   if (nmaterials > 65536) return fail(MT_ERR_INVALID, "more than 65536 materials (16-bit material index)");
+  if ((uvs && nuvs < 0) || (normals && nnormals < 0)) return fail(MT_ERR_INVALID, "negative uv or normal count");
   *out = nullptr;
-  const Face* F = reinterpret_cast<const Face*>(faces);
-  for (int i = 0; i < nfaces; ++i) {
-    const Face& f = F[i];
-    if (f.vx < 0 || f.vy < 0 || f.vz < 0 || f.vx >= npoints || f.vy >= npoints || f.vz >= npoints)
-      return fail(MT_ERR_INVALID, "face %d: vertex index out of range", i);
-    if ((f.mat & 0xFFFF) >= nmaterials) return fail(MT_ERR_INVALID, "face %d: material %d of %d", i, f.mat & 0xFFFF, nmaterials);
-    if (f.uvx > -1 && (!uvs || f.uvx >= nuvs || f.uvy < 0 || f.uvy >= nuvs || f.uvz < 0 || f.uvz >= nuvs))
-      return fail(MT_ERR_INVALID, "face %d: uv index out of range", i);
-    if (f.nx > -1 && (!normals || f.nx >= nnormals || f.ny < 0 || f.ny >= nnormals || f.nz < 0 || f.nz >= nnormals))
-      return fail(MT_ERR_INVALID, "face %d: normal index out of range", i);
-  }
   std::lock_guard<std::recursive_mutex> lk(ctx->mu);
   CU(cudaSetDevice(ctx->device));
   auto* s = new mt_scene();
@@ -387,17 +369,44 @@ extern "C" int mt_scene_create(mt_context* ctx, const float* points, int npoints
   s->nnormals = nnormals;
   s->ntri = nfaces;
   s->nmat = nmaterials;
-  s->h_points.assign(points, points + 4 * (size_t)npoints);
-  s->h_faces.assign(faces, faces + 10 * (size_t)nfaces);
   s->h_materials.assign((const uint8_t*)materials, (const uint8_t*)materials + 144 * (size_t)nmaterials);
-  int r = upload(&s->d_points, points, (size_t)npoints);
-  if (!r) r = upload(&s->d_uvs, uvs, uvs ? (size_t)nuvs : 1);
-  if (!r) r = upload(&s->d_normals, normals, normals ? (size_t)nnormals : 1);
-  if (!r) r = upload(&s->d_faces, faces, (size_t)nfaces);
+  if (!uvs) s->nuvs = 0;
+  if (!normals) s->nnormals = 0;
+  const size_t b_pts = Workspace::round(16 * (size_t)npoints), b_uvs = Workspace::round(8 * (size_t)std::max(s->nuvs, 1)),
+               b_nrm = Workspace::round(16 * (size_t)std::max(s->nnormals, 1));
+  int r = dalloc(&s->d_mesh, b_pts + b_uvs + b_nrm + 40 * (size_t)nfaces);
+  if (!r) {
+    s->d_points = (float4*)s->d_mesh;
+    s->d_uvs = (float2*)(s->d_mesh + b_pts);
+    s->d_normals = (float4*)(s->d_mesh + b_pts + b_uvs);
+    s->d_faces = (Face*)(s->d_mesh + b_pts + b_uvs + b_nrm);
+    cudaError_t e = cudaMemcpyAsync(s->d_points, points, 16 * (size_t)npoints, cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess && s->nuvs > 0)
+      e = cudaMemcpyAsync(s->d_uvs, uvs, 8 * (size_t)s->nuvs, cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess && s->nnormals > 0)
+      e = cudaMemcpyAsync(s->d_normals, normals, 16 * (size_t)s->nnormals, cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(s->d_faces, faces, 40 * (size_t)nfaces, cudaMemcpyHostToDevice, ctx->stream);
+    if (e != cudaSuccess) r = fail(MT_ERR_CUDA, "mesh upload: %s", cudaGetErrorString(e));
+  }
+  int bad = INT_MAX;
+  if (!r) r = first_bad_face(s, nmaterials, false, &bad);
+  if (!r && bad < nfaces) {
+    const Face& f = reinterpret_cast<const Face*>(faces)[bad];
+    if (f.vx < 0 || f.vy < 0 || f.vz < 0 || f.vx >= npoints || f.vy >= npoints || f.vz >= npoints)
+      r = fail(MT_ERR_INVALID, "face %d: vertex index out of range", bad);
+    else if ((f.mat & 0xFFFF) >= nmaterials)
+      r = fail(MT_ERR_INVALID, "face %d: material %d of %d", bad, f.mat & 0xFFFF, nmaterials);
+    else if (f.uvx > -1 && (f.uvx >= s->nuvs || f.uvy < 0 || f.uvy >= s->nuvs || f.uvz < 0 || f.uvz >= s->nuvs))
+      r = fail(MT_ERR_INVALID, "face %d: uv index out of range", bad);
+    else
+      r = fail(MT_ERR_INVALID, "face %d: normal index out of range", bad);
+  }
   if (!r) r = upload(&s->d_materials, materials, (size_t)nmaterials);
   if (!r) r = upload_lights(s);
   if (r) {
     std::string keep = g_err;
+    cudaStreamSynchronize(ctx->stream);  // the caller's arrays are no longer read
     free_scene(s);
     delete s;
     g_err = keep;
@@ -409,13 +418,18 @@ extern "C" int mt_scene_create(mt_context* ctx, const float* points, int npoints
 
 extern "C" int mt_scene_set_materials(mt_scene* s, const void* materials, int nmaterials) {
   if (!s || !materials || nmaterials <= 0) return fail(MT_ERR_INVALID, "bad argument");
-  const Face* F = reinterpret_cast<const Face*>(s->h_faces.data());
-  for (int i = 0; i < s->ntri; ++i)
-    if ((F[i].mat & 0xFFFF) >= nmaterials) return fail(MT_ERR_INVALID, "face %d needs material %d", i, F[i].mat & 0xFFFF);
   std::lock_guard<std::recursive_mutex> lk(s->ctx->mu);
   CU(cudaSetDevice(s->ctx->device));
   int q = quiesce(s->ctx);
   if (q) return q;
+  int bad = INT_MAX;
+  q = first_bad_face(s, nmaterials, true, &bad);
+  if (q) return q;
+  if (bad < s->ntri) {
+    Face f;
+    CU(cudaMemcpy(&f, s->d_faces + bad, sizeof(Face), cudaMemcpyDeviceToHost));
+    return fail(MT_ERR_INVALID, "face %d needs material %d", bad, f.mat & 0xFFFF);
+  }
   ++s->version;
   s->h_materials.assign((const uint8_t*)materials, (const uint8_t*)materials + 144 * (size_t)nmaterials);
   s->nmat = nmaterials;
@@ -647,22 +661,10 @@ int import_bvh(mt_scene* s, const int32_t* nodes, const float* bounds, int nnode
     r[3] = make_float4(lf, rf, 0.f, 0.f);
   }
   if ((int)order.size() != n) return fail(MT_ERR_INVALID, "BVH reaches %zu of %d triangles", order.size(), n);
-  std::vector<float4> ht(3 * (size_t)n);
-  const Face* F = reinterpret_cast<const Face*>(s->h_faces.data());
-  const float* P = s->h_points.data();
-  for (int k = 0; k < n; ++k) {
-    int f = order[k];
-    const float* p1 = P + 4 * (size_t)F[f].vx;
-    const float* p2 = P + 4 * (size_t)F[f].vy;
-    const float* p3 = P + 4 * (size_t)F[f].vz;
-    float fid;
-    std::memcpy(&fid, &f, 4);
-    ht[3 * (size_t)k + 0] = make_float4(p1[0], p1[1], p1[2], fid);
-    ht[3 * (size_t)k + 1] = make_float4(p2[0] - p1[0], p2[1] - p1[1], p2[2] - p1[2], 0.f);
-    ht[3 * (size_t)k + 2] = make_float4(p3[0] - p1[0], p3[1] - p1[1], p3[2] - p1[2], 0.f);
-  }
   int r = upload(&s->d_nodes, hn.data(), hn.size());
-  if (!r) r = upload(&s->d_tris, ht.data(), ht.size());
+  dfree(s->d_tris);
+  if (!r) r = dalloc(&s->d_tris, 3 * (size_t)n);
+  if (!r) r = order_triangles(s, order, s->d_tris);
   if (r) return r;
   s->nrec = nrec;
   s->root_ref = root[5] ? ~0 : 0;
@@ -677,9 +679,17 @@ extern "C" int mt_bvh_build(mt_scene* s, int32_t* nodes_out, float* bounds_out, 
   const int n = s->ntri;
   std::vector<int32_t> nodes(7 * (size_t)(2 * n - 1), 0);
   std::vector<float> bounds(8 * (size_t)(2 * n - 1), 0.f);
+  std::vector<float> points(4 * (size_t)s->npoints);
+  std::vector<Face> faces((size_t)n);
+  {
+    std::lock_guard<std::recursive_mutex> lk(s->ctx->mu);
+    CU(cudaSetDevice(s->ctx->device));
+    CU(cudaMemcpy(points.data(), s->d_points, points.size() * 4, cudaMemcpyDeviceToHost));
+    CU(cudaMemcpy(faces.data(), s->d_faces, faces.size() * sizeof(Face), cudaMemcpyDeviceToHost));
+  }
   Builder b;
-  b.pts = s->h_points.data();
-  b.faces = reinterpret_cast<const Face*>(s->h_faces.data());
+  b.pts = points.data();
+  b.faces = faces.data();
   b.n = n;
   b.nodes = nodes.data();
   b.bounds = bounds.data();

@@ -94,9 +94,8 @@ bool traversal_bitstack();
 struct mt_scene {
   mt_context* ctx;
   int npoints = 0, nuvs = 0, nnormals = 0, ntri = 0, nmat = 0;
-  std::vector<float> h_points;
-  std::vector<int32_t> h_faces;
   std::vector<uint8_t> h_materials;
+  char* d_mesh = nullptr;  // points, uvs, normals and faces, one allocation
   float4* d_points = nullptr;
   float2* d_uvs = nullptr;
   float4* d_normals = nullptr;
@@ -305,6 +304,14 @@ void join_jobs(mt_context* ctx);
 int quiesce(mt_context* ctx);
 // Waits for the requests running on the context's servers' lanes.
 void servers_sync(mt_context* ctx);
+// Mesh arrays on the device (mt_mesh.cu), on the context's stream and waited for. The
+// first face with an index out of range, or (mat_only) with a material of nmat or
+// more: INT_MAX when there is none.
+int first_bad_face(mt_scene* s, int nmat, bool mat_only, int* bad);
+// The faces whose material (emits[m] != 0) emits, in face order.
+int list_light_faces(mt_scene* s, const std::vector<unsigned char>& emits);
+// Triangle slots in the given order of faces.
+int order_triangles(mt_scene* s, const std::vector<int>& order, float4* tris);
 // Rebuild or drop the scene's derived traversal formats from its FP32 records:
 // FP16 records (precision 1), 4-wide FP16 nodes (precision 3), and the wide BVH
 // (precision 2, refresh_wide).

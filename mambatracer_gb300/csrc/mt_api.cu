@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <type_traits>
 #include <cstdlib>
 #include <cmath>
 #include <cstdarg>
@@ -281,6 +282,14 @@ int upload(T** d, const void* h, size_t count) {
   return MT_OK;
 }
 
+void free_env(mt_scene* s) {
+  dfree(s->d_env);
+  s->env_bytes = 0;
+  s->d_env_rgb = nullptr;
+  s->d_env_lum = s->d_env_sat = s->d_env_marg = s->d_env_cond = nullptr;
+  s->d_env_sat64 = nullptr;
+}
+
 void free_scene(mt_scene* s) {
   dfree(s->d_mesh);
   s->d_points = nullptr;
@@ -296,32 +305,52 @@ void free_scene(mt_scene* s) {
   dfree(s->d_wtris);
   dfree(s->d_quad);
   dfree(s->d_up);
-  dfree(s->d_env_rgb);
-  dfree(s->d_env_lum);
-  dfree(s->d_env_sat);
-  dfree(s->d_env_sat64);
-  dfree(s->d_env_marg);
-  dfree(s->d_env_cond);
+  free_env(s);
   dfree(s->d_texels);
   dfree(s->d_tex_ref);
 }
 
-// CDF tables of the whole map for full-map environment sampling, from its FP32 SAT.
-int build_env_tables(mt_scene* s) {
-  dfree(s->d_env_marg);
-  dfree(s->d_env_cond);
-  if (!cdf_tables_enabled()) return MT_OK;
-  size_t m = 0;
-  const size_t c = map_table_floats(s->env_w, s->env_h, &m);
-  int r = dalloc(&s->d_env_marg, m);
-  if (!r) r = dalloc(&s->d_env_cond, c);
-  if (!r && launch_map_tables(s->ctx->stream, s->d_env_sat, s->env_w, s->env_h, s->d_env_marg, s->d_env_cond))
-    r = fail(MT_ERR_CUDA, "environment tables: %s", cudaGetErrorString(cudaGetLastError()));
-  if (r) {
-    dfree(s->d_env_marg);
-    dfree(s->d_env_cond);
+// Arrays of a w x h environment map, one allocation: texels, luminance, SATs (with64:
+// the FP64 one too) and, unless switched off, the CDF tables of full-map sampling. A
+// map of the same shape takes the arrays of the one before.
+int alloc_env(mt_scene* s, int w, int h, bool with64) {
+  const size_t n = (size_t)w * h;
+  size_t marg = 0;
+  const size_t cond = map_table_floats(w, h, &marg);
+  const bool tables = cdf_tables_enabled();
+  auto R = Workspace::round;
+  const size_t bytes = R(16 * n) + 2 * R(4 * n) + (with64 ? R(8 * n) : 0) + (tables ? R(4 * marg) + R(4 * cond) : 0);
+  if (bytes != s->env_bytes || w != s->env_w || h != s->env_h) {
+    free_env(s);
+    int r = dalloc(&s->d_env, bytes);
+    if (r) return r;
+    s->env_bytes = bytes;
   }
-  return r;
+  char* at = s->d_env;
+  auto take = [&](auto** p, size_t b) {
+    *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(at);
+    at += R(b);
+  };
+  take(&s->d_env_rgb, 16 * n);
+  take(&s->d_env_lum, 4 * n);
+  take(&s->d_env_sat, 4 * n);
+  s->d_env_sat64 = nullptr;
+  s->d_env_marg = s->d_env_cond = nullptr;
+  if (with64) take(&s->d_env_sat64, 8 * n);
+  if (tables) {
+    take(&s->d_env_marg, 4 * marg);
+    take(&s->d_env_cond, 4 * cond);
+  }
+  s->env_w = w;
+  s->env_h = h;
+  return MT_OK;
+}
+
+int build_env_tables(mt_scene* s) {
+  if (s->d_env_marg &&
+      launch_map_tables(s->ctx->stream, s->d_env_sat, s->env_w, s->env_h, s->d_env_marg, s->d_env_cond))
+    return fail(MT_ERR_CUDA, "environment tables: %s", cudaGetErrorString(cudaGetLastError()));
+  return MT_OK;
 }
 
 // Texel pool (all images back to back) and the per-material table of
@@ -775,16 +804,12 @@ extern "C" int mt_env_set(mt_scene* s, const float* rgb, int w, int h) {
   int q = quiesce(s->ctx);
   if (q) return q;
   ++s->version;
-  size_t n = (size_t)w * h;
-  int r = upload(&s->d_env_rgb, rgb, n);
-  if (!r) { dfree(s->d_env_lum); r = dalloc(&s->d_env_lum, n); }
-  if (!r) { dfree(s->d_env_sat); r = dalloc(&s->d_env_sat, n); }
-  if (!r) { dfree(s->d_env_sat64); r = dalloc(&s->d_env_sat64, n); }
+  s->env_present = 0;
+  int r = alloc_env(s, w, h, true);
   if (r) return r;
+  CU(cudaMemcpyAsync(s->d_env_rgb, rgb, 16 * (size_t)w * h, cudaMemcpyHostToDevice, s->ctx->stream));
   if (launch_env_build(s->ctx->stream, s->d_env_rgb, w, h, s->d_env_lum, s->d_env_sat64, s->d_env_sat))
     return fail(MT_ERR_CUDA, "environment build launch: %s", cudaGetErrorString(cudaGetLastError()));
-  s->env_w = w;
-  s->env_h = h;
   if ((r = build_env_tables(s))) return r;
   CU(cudaStreamSynchronize(s->ctx->stream));
   s->env_present = 1;
@@ -798,14 +823,13 @@ extern "C" int mt_env_set_with_sat(mt_scene* s, const float* rgb, const float* l
   int q = quiesce(s->ctx);
   if (q) return q;
   ++s->version;
-  size_t n = (size_t)w * h;
-  int r = upload(&s->d_env_rgb, rgb, n);
-  if (!r) r = upload(&s->d_env_lum, lum, n);
-  if (!r) r = upload(&s->d_env_sat, sat, n);
+  s->env_present = 0;
+  int r = alloc_env(s, w, h, false);
   if (r) return r;
-  dfree(s->d_env_sat64);
-  s->env_w = w;
-  s->env_h = h;
+  const size_t n = (size_t)w * h;
+  CU(cudaMemcpyAsync(s->d_env_rgb, rgb, 16 * n, cudaMemcpyHostToDevice, s->ctx->stream));
+  CU(cudaMemcpyAsync(s->d_env_lum, lum, 4 * n, cudaMemcpyHostToDevice, s->ctx->stream));
+  CU(cudaMemcpyAsync(s->d_env_sat, sat, 4 * n, cudaMemcpyHostToDevice, s->ctx->stream));
   if ((r = build_env_tables(s))) return r;
   CU(cudaStreamSynchronize(s->ctx->stream));
   s->env_present = 1;

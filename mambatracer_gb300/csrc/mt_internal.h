@@ -114,7 +114,9 @@ struct mt_scene {
   float4* d_wtris = nullptr;
   int nwide = 0, wdepth = 0;
   int nrec = 0, root_ref = 0, depth = 0, has_bvh = 0, precision = 0;
-  // environment
+  // environment: the arrays below, one allocation
+  char* d_env = nullptr;
+  size_t env_bytes = 0;
   float4* d_env_rgb = nullptr;
   float* d_env_lum = nullptr;
   float* d_env_sat = nullptr;

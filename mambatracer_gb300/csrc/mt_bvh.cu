@@ -629,30 +629,25 @@ extern "C" int mt_bvh_build_device(mt_scene* s, int32_t* nodes_out, float* bound
   const size_t node_cap = (size_t)n / kSmallTris + 2,
                small_cap = std::min((size_t)n, 2 * node_cap * (kStackDepth + 8)) + 1;
   const int chunk_cap = n / kChunk + (int)node_cap;
-  auto align = [](size_t b) { return (b + 255) / 256 * 256; };
+  auto align = Workspace::round;
   const size_t b_prim = align(sizeof(Prim) * (size_t)n), b_node = align(sizeof(Big) * node_cap),
                b_small = align(sizeof(Small) * small_cap), b_cnt = align(sizeof(int) * ((size_t)chunk_cap + 1)),
                b_ref = nodes_out ? align(28 * nn) : 0, b_bound = bounds_out ? align(32 * nn) : 0;
-  char* slab = nullptr;  // all scratch in one allocation
+  Workspace ws;
   float4 *recs = nullptr, *tris = nullptr;
-  int r = dalloc(&slab, 2 * b_prim + 2 * b_node + b_small + b_cnt + b_ref + b_bound + 256);
+  int r = ws.get(ctx, 2 * b_prim + 2 * b_node + b_small + b_cnt + b_ref + b_bound + 256);
   if (!r) r = dalloc(&recs, 4 * (size_t)std::max(nrec, 1));
   if (!r) r = dalloc(&tris, 3 * (size_t)n);
   auto fail_all = [&](int code, const char* msg) {
     std::string keep = msg ? std::string(msg) : mt_last_error();
     cudaStreamSynchronize(st);
-    dfree(slab);
+    ws.release();
     dfree(recs);
     dfree(tris);
     return fail(code, "%s", keep.c_str());
   };
   if (r) return fail_all(r, nullptr);
-  char* at = slab;
-  auto take = [&](size_t b) {
-    char* p = at;
-    at += b;
-    return p;
-  };
+  auto take = [&](size_t b) { return ws.take<char>(b); };
   Prim* prim[2] = {(Prim*)take(b_prim), nullptr};
   prim[1] = (Prim*)take(b_prim);
   Big* nodes[2] = {(Big*)take(b_node), nullptr};
@@ -695,7 +690,7 @@ extern "C" int mt_bvh_build_device(mt_scene* s, int32_t* nodes_out, float* bound
     return fail_all(MT_ERR_CUDA, cudaGetErrorString(cudaGetLastError()));
   const int depth = hh.depth;
   if (depth > kStackDepth) return fail_all(MT_ERR_DEPTH, "BVH deeper than the 64-level traversal stack");
-  dfree(slab);
+  ws.release();
   dfree(s->d_nodes);
   dfree(s->d_tris);
   s->d_nodes = recs;
@@ -733,8 +728,9 @@ int refresh_qnodes(mt_scene* s) {
   }
   if (int w = refresh_wide(s)) return w;
   if (s->precision == 3 && s->has_bvh && s->nrec > 0) {
+    Workspace ws;
     float4* sah = nullptr;
-    int r = build_sah_records(s, &sah);
+    int r = build_sah_records(s, ws, &sah);
     if (!r) r = dalloc(&s->d_quad, (sah ? 8 : 4) * (size_t)s->nrec);
     cudaError_t e = cudaSuccess;
     if (!r) {
@@ -746,7 +742,7 @@ int refresh_qnodes(mt_scene* s) {
       const cudaError_t w = cudaStreamSynchronize(st);
       if (e == cudaSuccess) e = w;
     }
-    dfree(sah);
+    ws.release();
     if (r || e != cudaSuccess) {
       dfree(s->d_quad);
       return r ? r : fail(MT_ERR_CUDA, "4-wide FP16 nodes: %s", cudaGetErrorString(e));

@@ -319,9 +319,10 @@ int order_triangles(mt_scene* s, const std::vector<int>& order, float4* tris);
 // (precision 2, refresh_wide).
 int refresh_qnodes(mt_scene* s);
 // FP32 records of a surface-area-heuristic tree over the scene's triangle slots
-// (mt_sah.cu; cudaFree'd by the caller), or NULL where that tree would be deeper
-// than the traversal stack holds. Two triangles or more.
-int build_sah_records(mt_scene* s, float4** recs_out);
+// (mt_sah.cu), in ws, which the caller releases; NULL where that tree would be
+// deeper than the traversal stack holds. Two triangles or more.
+struct Workspace;
+int build_sah_records(mt_scene* s, Workspace& ws, float4** recs_out);
 int refresh_wide(mt_scene* s);
 // MT_CDF_TABLES=0 turns the CDF tables of environment sampling off (the samplers
 // then search the SATs directly; the tables hold the same values).

@@ -658,36 +658,26 @@ __global__ void __launch_bounds__(32 * kSmallWarps)
 
 using namespace mt;
 
-int build_sah_records(mt_scene* s, float4** recs_out) {
+int build_sah_records(mt_scene* s, Workspace& ws, float4** recs_out) {
   *recs_out = nullptr;
   const int n = s->ntri;
   cudaStream_t st = s->ctx->stream;
   const int node_cap = n / kSmallTris + 2, small_cap = n / 2 + 1;
-  // one slab: records, the triangles twice, the node lists, the small subtrees, the bins, the heads
-  auto align = [](size_t b) { return (b + 255) / 256 * 256; };
+  // records, the triangles twice, the node lists, the small subtrees, the bins, the heads
+  auto align = Workspace::round;
   const size_t b_prim = align(sizeof(Prim) * (size_t)n), b_node = align(sizeof(Node) * (size_t)node_cap),
                b_small = align(sizeof(Small) * (size_t)small_cap),
                b_bins = align(sizeof(Bin) * 3 * kBins * (size_t)node_cap), b_head = align(sizeof(Heads));
-  char* slab = nullptr;
-  float4* recs = nullptr;
-  int r = dalloc(&recs, 4 * (size_t)(n - 1));
-  if (!r) r = dalloc(&slab, 2 * b_prim + 2 * b_node + b_small + b_bins + b_head);
-  if (r) {
-    dfree(recs);
-    return r;
-  }
+  int r = ws.get(s->ctx, align(64 * (size_t)(n - 1)) + 2 * b_prim + 2 * b_node + b_small + b_bins + b_head);
+  if (r) return r;
+  float4* recs = (float4*)ws.take<char>(64 * (size_t)(n - 1));
+  char* slab = ws.take<char>(2 * b_prim + 2 * b_node + b_small + b_bins + b_head);
   Prim* prim[2] = {(Prim*)slab, (Prim*)(slab + b_prim)};
   Node* nodes[2] = {(Node*)(slab + 2 * b_prim), (Node*)(slab + 2 * b_prim + b_node)};
   Small* smalls = (Small*)(slab + 2 * b_prim + 2 * b_node);
   Bin* bins = (Bin*)(slab + 2 * b_prim + 2 * b_node + b_small);
   Heads* heads = (Heads*)(slab + 2 * b_prim + 2 * b_node + b_small + b_bins);
   auto blocks = [](size_t m, int t) { return (unsigned)((m + t - 1) / t); };
-  auto done = [&](int code) {
-    cudaStreamSynchronize(st);
-    dfree(slab);
-    if (code) dfree(recs);
-    return code;
-  };
   k_start<<<1, 1, 0, st>>>(nodes[0], smalls, heads, n);
   k_boxes<<<blocks(n, kPartThreads), kPartThreads, 0, st>>>(s->d_tris, s->d_points, s->d_faces, n, prim[0], nodes[0]);
   // the levels, as in mt_bvh_build_device: without waiting for the host at each
@@ -707,25 +697,17 @@ int build_sah_records(mt_scene* s, float4** recs_out) {
     }
     if (cudaMemcpyAsync(&hh, heads, sizeof(hh), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
-      return done(fail(MT_ERR_CUDA, "surface-area tree: %s", cudaGetErrorString(cudaGetLastError())));
+      return fail(MT_ERR_CUDA, "surface-area tree: %s", cudaGetErrorString(cudaGetLastError()));
     if (hh.nodes[level & 1] == 0) break;
-    if (level > kStackDepth) {  // too deep: the caller keeps the reference tree
-      done(MT_OK);
-      dfree(recs);
-      return MT_OK;
-    }
+    if (level > kStackDepth) return MT_OK;  // too deep: the caller keeps the reference tree
   }
   const int nsmall = n > kSmallTris ? std::min(hh.smalls, small_cap) : 1;
   if (nsmall > 0)
     k_small<<<blocks(nsmall, kSmallWarps), 32 * kSmallWarps, 0, st>>>(prim[0], prim[1], smalls, small_cap, recs, heads);
   if (cudaMemcpyAsync(&hh, heads, sizeof(hh), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
       cudaStreamSynchronize(st) != cudaSuccess)
-    return done(fail(MT_ERR_CUDA, "surface-area tree: %s", cudaGetErrorString(cudaGetLastError())));
-  done(MT_OK);
-  if (hh.depth > kStackDepth) {
-    dfree(recs);
-    return MT_OK;
-  }
+    return fail(MT_ERR_CUDA, "surface-area tree: %s", cudaGetErrorString(cudaGetLastError()));
+  if (hh.depth > kStackDepth) return MT_OK;
   *recs_out = recs;
   return MT_OK;
 }

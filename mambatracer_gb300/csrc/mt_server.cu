@@ -100,19 +100,39 @@ constexpr size_t kPathBytesPerPixel = 200;
 constexpr int kRounds = 3;
 constexpr size_t kGraphsPerStream = 16;  // scenes whose merged-pass graph a merge stream keeps
 
-// One merge stream: its slots, its share of the queues, its round ring.
-struct MergeGroup {
-  struct mt_server* server = nullptr;
+// What one round in flight of a merge stream needs: path state of its slots' paths
+// (the films are the whole arena's), streams, and per scene the executable graph of
+// its merged pass, updated every round.
+struct PathSet {
+  char* slab = nullptr;  // the second and later sets' arrays, and every set's log
+  FrameBufs fb{};
   cudaStream_t stream = nullptr;
   cudaStream_t side = nullptr;  // shadow rays beside the next bounce's extension rays
   cudaEvent_t sfork = nullptr, sjoin = nullptr;
+  cudaEvent_t done = nullptr;   // its last round's passes are in the films
+  std::vector<std::pair<const mt_scene*, cudaGraphExec_t>> graphs;
+};
+// Rounds of a merge stream that overlap, and the memory their sets may take in all
+// (beyond the first): passes log their contributions then, added in round order. One, two,
+// three, four at once, requests of 48 to 400 pixels a side with up to 4 passes on four
+// streams: 2 requests 5.28, 2.91, 2.88, 1.70 ms, 16 8.66, 7.87, 8.02, 8.00, 24 13.9, 12.0,
+// 9.1, 9.8.
+constexpr int kSets = 3;
+constexpr size_t kSetBytes = 8ull << 30;
+
+// One merge stream: its slots, its sets of queues, its round ring.
+struct MergeGroup {
+  struct mt_server* server = nullptr;
   std::vector<int> slots;
-  FrameBufs fb{};  // path state of its slots' paths; the films of the whole arena
+  std::vector<PathSet> sets;
+  int next_set = 0;
   Round rounds[kRounds];
   int next_round = 0;
   int inflight = 0;  // rounds whose end callback has not run (server lock)
-  // per scene: the executable graph of its merged pass, updated every round
-  std::vector<std::pair<const mt_scene*, cudaGraphExec_t>> graphs;
+  void sync() const {
+    for (const PathSet& Q : sets)
+      if (Q.stream) cudaStreamSynchronize(Q.stream);
+  }
 };
 
 }  // namespace
@@ -290,17 +310,16 @@ void free_merged(mt_server* s) {
       if (Rd.done) cudaEventDestroy(Rd.done);
       Rd.done = nullptr;
     }
-    for (auto& g : G.graphs)
-      if (g.second) cudaGraphExecDestroy(g.second);
-    G.graphs.clear();
-    if (G.stream) cudaStreamDestroy(G.stream);
-    G.stream = nullptr;
-    if (G.side) cudaStreamDestroy(G.side);
-    G.side = nullptr;
-    for (cudaEvent_t* e : {&G.sfork, &G.sjoin}) {
-      if (*e) cudaEventDestroy(*e);
-      *e = nullptr;
+    for (PathSet& Q : G.sets) {
+      for (auto& g : Q.graphs)
+        if (g.second) cudaGraphExecDestroy(g.second);
+      for (cudaStream_t st : {Q.stream, Q.side})
+        if (st) cudaStreamDestroy(st);
+      for (cudaEvent_t e : {Q.sfork, Q.sjoin, Q.done})
+        if (e) cudaEventDestroy(e);
+      dfree(Q.slab);
     }
+    G.sets.clear();
   }
 }
 
@@ -325,6 +344,11 @@ int alloc_merged(mt_server* s, size_t N, int m) {
   for (Lane& L : s->lanes)
     if (!r && cudaMallocHost((void**)&L.h_stage, sizeof(float4) * N) != cudaSuccess)
       r = fail(MT_ERR_NOMEM, "pinned film staging");
+  // sets of queues per stream: bytes a path of one set, and of a log
+  auto R = Workspace::round;
+  const size_t queue_bytes = 9 * 16 + 12, log_bytes = 32 * (size_t)s->cfg.max_depth + 4;
+  int nsets = kSets;
+  while (nsets > 1 && P * ((nsets - 1) * queue_bytes + nsets * log_bytes) > kSetBytes) --nsets;
   size_t base = 0;  // first path of the group's share
   for (MergeGroup& G : s->groups) {
     G.server = s;
@@ -340,25 +364,43 @@ int alloc_merged(mt_server* s, size_t N, int m) {
       if (!r && cudaEventCreateWithFlags(&Rd.done, cudaEventDisableTiming) != cudaSuccess)
         r = fail(MT_ERR_CUDA, "event create");
     }
-    if (!r && (cudaStreamCreateWithFlags(&G.stream, cudaStreamNonBlocking) != cudaSuccess ||
-               cudaStreamCreateWithFlags(&G.side, cudaStreamNonBlocking) != cudaSuccess ||
-               cudaEventCreateWithFlags(&G.sfork, cudaEventDisableTiming) != cudaSuccess ||
-               cudaEventCreateWithFlags(&G.sjoin, cudaEventDisableTiming) != cudaSuccess))
-      r = fail(MT_ERR_CUDA, "stream create");
-    if (r) break;
-    G.fb = s->mfb;  // films stay whole: slot k's film is at k x N
-    for (int q = 0; q < 2; ++q) {
-      G.fb.q_o[q] += base;
-      G.fb.q_d[q] += base;
-      G.fb.q_t[q] += base;
+    G.sets.resize(nsets);
+    const size_t paths = (size_t)n * N;
+    for (int k = 0; k < nsets && !r; ++k) {
+      PathSet& Q = G.sets[k];
+      if (cudaStreamCreateWithFlags(&Q.stream, cudaStreamNonBlocking) != cudaSuccess ||
+          cudaStreamCreateWithFlags(&Q.side, cudaStreamNonBlocking) != cudaSuccess ||
+          cudaEventCreateWithFlags(&Q.sfork, cudaEventDisableTiming) != cudaSuccess ||
+          cudaEventCreateWithFlags(&Q.sjoin, cudaEventDisableTiming) != cudaSuccess ||
+          cudaEventCreateWithFlags(&Q.done, cudaEventDisableTiming) != cudaSuccess) {
+        r = fail(MT_ERR_CUDA, "stream create");
+        break;
+      }
+      Q.fb = s->mfb;  // films stay whole: slot k's film is at k x N
+      const size_t queues = k > 0 ? 9 * R(16 * paths) + 3 * R(4 * paths) : 0;
+      const size_t log = nsets > 1 ? R(32 * paths * s->cfg.max_depth) + R(4 * paths) : 0;
+      if (queues + log > 0) r = dalloc(&Q.slab, queues + log);
+      if (r) break;
+      char* at = Q.slab;
+      auto take = [&](size_t b) {
+        char* p = at;
+        at += R(b);
+        return p;
+      };
+      for (auto* p : {&Q.fb.q_o[0], &Q.fb.q_o[1], &Q.fb.q_d[0], &Q.fb.q_d[1], &Q.fb.q_t[0], &Q.fb.q_t[1], &Q.fb.s_o,
+                      &Q.fb.s_d, &Q.fb.s_c})
+        *p = k > 0 ? (float4*)take(16 * paths) : *p + base;
+      Q.fb.hit_t = k > 0 ? (float*)take(4 * paths) : Q.fb.hit_t + base;
+      Q.fb.hit_prim = k > 0 ? (int*)take(4 * paths) : Q.fb.hit_prim + base;
+      Q.fb.live = k > 0 ? (int*)take(4 * paths) : Q.fb.live + base;
+      if (nsets > 1) {
+        Q.fb.log = (float4*)take(32 * paths * s->cfg.max_depth);
+        Q.fb.log_n = (int*)take(4 * paths);
+        Q.fb.log_stride = (int)paths;
+      }
     }
-    G.fb.hit_t += base;
-    G.fb.hit_prim += base;
-    G.fb.s_o += base;
-    G.fb.s_d += base;
-    G.fb.s_c += base;
-    G.fb.live += base;
-    base += (size_t)n * N;
+    if (r) break;
+    base += paths;
   }
   s->slot_px = N;
   return r;
@@ -371,7 +413,11 @@ int alloc_merged(mt_server* s, size_t N, int m) {
 int issue_round(mt_server* s, MergeGroup& G, const std::vector<int>& work, const std::vector<char>& cancel) {
   const mt_server_config& c = s->cfg;
   const size_t N = s->slot_px;
-  cudaStream_t st = G.stream;
+  const int nsets = (int)G.sets.size();
+  PathSet& Q = G.sets[G.next_set];
+  const cudaEvent_t before = nsets > 1 ? G.sets[(G.next_set + nsets - 1) % nsets].done : nullptr;
+  G.next_set = (G.next_set + 1) % nsets;
+  cudaStream_t st = Q.stream;
   Round& Rd = G.rounds[G.next_round];
   G.next_round = (G.next_round + 1) % kRounds;
   if (Rd.used) CU(cudaEventSynchronize(Rd.done));  // its tables were read, its passes ran
@@ -380,6 +426,8 @@ int issue_round(mt_server* s, MergeGroup& G, const std::vector<int>& work, const
   for (size_t i = 0; i < work.size(); ++i) {
     Lane& L = s->lanes[work[i]];
     if (cancel[i]) {
+      // its slot is free once its earlier passes, in the rounds before, have ended
+      if (before) CU(cudaStreamWaitEvent(st, before, 0));
       CU(cudaLaunchHostFunc(st, lane_done, &L));
       L.issued = true;
       continue;
@@ -449,8 +497,9 @@ int issue_round(mt_server* s, MergeGroup& G, const std::vector<int>& work, const
     const DevEnv E = Gr.scene->env_view();  // full-map environment sampling
     CU(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     const int lr = launch_batch_pass(st, S, E, Rd.d_tab + Gr.tab, Rd.d_tab + Gr.tab + Gr.n + 1, Rd.d_pp + Gr.pp,
-                                     Gr.n, Gr.total, c.max_depth, c.film_kahan, Rd.d_ctrl + g, G.fb,
-                                     s->ctx->num_sms, s->d_totals, G.side, G.sfork, G.sjoin, (int)s->groups.size());
+                                     Gr.n, Gr.total, c.max_depth, c.film_kahan, Rd.d_ctrl + g, Q.fb,
+                                     s->ctx->num_sms, before ? nullptr : s->d_totals, Q.side, Q.sfork, Q.sjoin,
+                                     (int)s->groups.size());
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(st, &graph);
     if (lr || e != cudaSuccess) {
@@ -458,16 +507,16 @@ int issue_round(mt_server* s, MergeGroup& G, const std::vector<int>& work, const
       return fail(MT_ERR_CUDA, "merged pass capture: %s", cudaGetErrorString(lr ? cudaGetLastError() : e));
     }
     cudaGraphExec_t* ex = nullptr;
-    for (auto& kv : G.graphs)
+    for (auto& kv : Q.graphs)
       if (kv.first == Gr.scene) ex = &kv.second;
     if (!ex) {
-      if (G.graphs.size() >= kGraphsPerStream) {
+      if (Q.graphs.size() >= kGraphsPerStream) {
         // the oldest scene's graph goes (a graph still running is freed when it ends)
-        if (G.graphs.front().second) cudaGraphExecDestroy(G.graphs.front().second);
-        G.graphs.erase(G.graphs.begin());
+        if (Q.graphs.front().second) cudaGraphExecDestroy(Q.graphs.front().second);
+        Q.graphs.erase(Q.graphs.begin());
       }
-      G.graphs.emplace_back(Gr.scene, nullptr);
-      ex = &G.graphs.back().second;
+      Q.graphs.emplace_back(Gr.scene, nullptr);
+      ex = &Q.graphs.back().second;
     }
     if (*ex) {
       cudaGraphExecUpdateResultInfo info;
@@ -484,6 +533,23 @@ int issue_round(mt_server* s, MergeGroup& G, const std::vector<int>& work, const
       return fail(MT_ERR_CUDA, "merged pass graph: %s", cudaGetErrorString(e));
     }
     CU(cudaGraphLaunch(*ex, st));
+    if (before) {
+      if (g == 0) CU(cudaStreamWaitEvent(st, before, 0));  // the rounds before are in the films
+      Replay Rp{};
+      Rp.log[0] = Q.fb.log;
+      Rp.count[0] = Q.fb.log_n;
+      Rp.ctrl[0] = Rd.d_ctrl + g;
+      Rp.passes = 1;
+      Rp.stride = Q.fb.log_stride;
+      Rp.n = Gr.total;
+      Rp.max_depth = c.max_depth;
+      Rp.kahan = c.film_kahan;
+      Rp.start = Rd.d_tab + Gr.tab;
+      Rp.film = Rd.d_tab + Gr.tab + Gr.n + 1;
+      Rp.frames = Gr.n;
+      if (launch_replay(st, Rp, Q.fb.film, Q.fb.film_c, s->d_totals))
+        return fail(MT_ERR_CUDA, "merged pass film: %s", cudaGetErrorString(cudaGetLastError()));
+    }
   }
   for (int k : go) {
     Lane& L = s->lanes[k];
@@ -493,6 +559,7 @@ int issue_round(mt_server* s, MergeGroup& G, const std::vector<int>& work, const
     CU(cudaLaunchHostFunc(st, lane_done, &L));
     L.issued = true;
   }
+  CU(cudaEventRecord(Q.done, st));
   CU(cudaEventRecord(Rd.done, st));
   CU(cudaLaunchHostFunc(st, round_done, &G));
   return MT_OK;
@@ -620,7 +687,7 @@ void worker_main(mt_server* s) {
         cudaSetDevice(s->ctx->device);
         r = issue_round(s, G, work, cancel);
         if (r)
-          for (MergeGroup& H : s->groups) cudaStreamSynchronize(H.stream);
+          for (MergeGroup& H : s->groups) H.sync();
       }
       lk.lock();
       if (r) {
@@ -729,8 +796,7 @@ extern "C" int mt_server_destroy(mt_server* s) {
   {
     std::lock_guard<std::recursive_mutex> lk(s->ctx->mu);
     cudaSetDevice(s->ctx->device);
-    for (MergeGroup& G : s->groups)
-      if (G.stream) cudaStreamSynchronize(G.stream);
+    for (MergeGroup& G : s->groups) G.sync();
     for (Lane& L : s->lanes) {
       for (cudaStream_t q : {L.stream, L.side})
         if (q) cudaStreamSynchronize(q);
@@ -876,8 +942,7 @@ extern "C" int mt_server_stats(mt_server* s, mt_served_stats* out) {
 
 void servers_sync(mt_context* ctx) {
   for (mt_server* s : ctx->servers) {
-    for (MergeGroup& G : s->groups)
-      if (G.stream) cudaStreamSynchronize(G.stream);
+    for (MergeGroup& G : s->groups) G.sync();
     for (Lane& L : s->lanes)
       for (cudaStream_t q : {L.stream, L.side})
         if (q) cudaStreamSynchronize(q);

@@ -551,6 +551,8 @@ int issue_round(mt_server* s, MergeGroup& G, const std::vector<int>& work, const
         return fail(MT_ERR_CUDA, "merged pass film: %s", cudaGetErrorString(cudaGetLastError()));
     }
   }
+  // before the finished requests' copies and callbacks: the next round does not wait for those
+  CU(cudaEventRecord(Q.done, st));
   for (int k : go) {
     Lane& L = s->lanes[k];
     if (++L.pass < L.req->spp) continue;
@@ -559,7 +561,6 @@ int issue_round(mt_server* s, MergeGroup& G, const std::vector<int>& work, const
     CU(cudaLaunchHostFunc(st, lane_done, &L));
     L.issued = true;
   }
-  CU(cudaEventRecord(Q.done, st));
   CU(cudaEventRecord(Rd.done, st));
   CU(cudaLaunchHostFunc(st, round_done, &G));
   return MT_OK;

@@ -193,7 +193,8 @@ typedef struct mt_render_config {
   int mode;          /* 0 = reference semantics, 1 = benchmark semantics (pixel-keyed RNG, RR, Q1/Q2 fixed) */
   int rr_depth;      /* mode 1: Russian roulette from this bounce on (0 = off) */
   int film_kahan;    /* 1 = compensated film sums (default), 0 = plain FP32 adds as the reference */
-  int spp;           /* passes per mt_render_frame call */
+  int spp;           /* passes per mt_render_frame call; up to four run side by side, where the path
+                        state for them (160 + 32 max_depth bytes per pixel each) fits 8 GiB */
   int use_graph;     /* 1 = replay each frame's launches as a CUDA graph */
   int profile;       /* 1 = time every kernel launch with CUDA events (no graph) */
   int inflight;      /* frames kept in flight on their own streams, 0 or 1 = one (1..8); each
@@ -259,8 +260,9 @@ int mt_job_total_rays(mt_job* job, int64_t* rays3);
 int mt_job_last_ms(mt_job* job, float* ms);
 /* Kernels the job's frames have launched (graph nodes included): per pass the
  * ray generation, per bounce the closest-hit traversal, shading (one launch or
- * two) and the shadow rays, and the ray totals; per frame the film merge of
- * jobs with frames in flight. Light-grid updates are not counted. */
+ * two) and the shadow rays, and the ray totals or, where passes overlap, their
+ * contributions added to the film; per frame the film merge of jobs with frames in
+ * flight. Light-grid updates are not counted. */
 int mt_job_launches(mt_job* job, int64_t* n);
 /* Profiled jobs: device time of each launch of the last frame, in ms, pass by
  * pass: [raygen, then per bounce trace_closest, shade, trace_shadow] =
@@ -351,14 +353,16 @@ int mt_trace_closest_dev(mt_scene* scene, mt_buffer* rays, int n, mt_buffer* t_o
  * benchmark-semantics passes (mode 1) of one camera and returns its
  * accumulated film. A scheduler thread admits requests first come, first
  * served onto `lanes` preallocated lanes (stream + path state for the largest
- * frame) within a budget of path-state bytes (200 B per pixel; 0 = no limit);
- * no device memory is allocated while requests run. Scenes used by queued or
+ * frame) within a budget of path-state bytes (counted as 200 B per pixel; 0 = no
+ * limit); no device memory is allocated while requests run. Scenes used by queued or
  * running requests cannot be destroyed (MT_ERR_BUSY).
  * merged = m (1..lanes): the running requests share wavefront queues (lanes x
  * the largest frame paths, at most 2^30) instead of a lane each; the slots are
  * split over m streams, and each stream issues rounds, a round being one merged
  * pass per scene holding the next pass of every running request of its slots.
- * A request joins at its stream's next round. A cancelled running request
+ * A request joins at its stream's next round; up to three rounds of a stream
+ * overlap, on path state of their own (at most 8 GiB in all beyond the lanes').
+ * A cancelled running request
  * stops at the next round (state CANCELLED, no film). Films are the same, bit
  * for bit, in both modes. */
 typedef struct mt_server mt_server;
@@ -398,7 +402,8 @@ typedef struct {
  * camera, size, spp, frame number and path settings, bit for bit.
  * films_out: the frames' float4 films back to back in frame order (sum over
  * the frame's passes, not divided); rays_out (may be NULL): [primary,
- * extension, shadow] rays traced. Synchronous; allocates its queues per call. */
+ * extension, shadow] rays traced. Synchronous; its queues are the context's scratch,
+ * kept between calls up to 2 GiB (larger ones are allocated per call). */
 int mt_batch_render(mt_context* ctx, mt_scene* scene, const mt_batch_frame* frames, int nframes, int max_depth,
                     int rr_depth, int film_kahan, float* films_out, int64_t* rays_out);
 /* Cancels queued requests, waits for running ones, frees the lanes. */

@@ -64,9 +64,11 @@ int Workspace::get(mt_context* c, size_t bytes) {
     cudaStreamSynchronize(c->stream);
     dfree(c->ws);
     c->ws_bytes = 0;
+    size_t got = grown;
     int r = dalloc(&c->ws, grown);
+    if (r && bytes < grown) r = dalloc(&c->ws, got = bytes);
     if (r) return r;
-    c->ws_bytes = grown;
+    c->ws_bytes = got;
   }
   base = c->ws;
   return MT_OK;
@@ -77,7 +79,22 @@ void Workspace::release() {
   base = nullptr;
 }
 
+bool drop_workspace(mt_context* c) {
+  if (!c->ws) return false;
+  cudaStreamSynchronize(c->stream);
+  dfree(c->ws);
+  c->ws_bytes = 0;
+  return true;
+}
+
 void prefault(void* p, size_t bytes, cudaEvent_t ready) {
+  // only the process's own pages: pinned memory is mapped, and a device pointer, which
+  // the copy that follows refuses, is not the host's to write
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess || a.type != cudaMemoryTypeUnregistered) {
+    cudaGetLastError();
+    return;
+  }
   constexpr size_t kPage = 4096, kStep = 64 * kPage;
   auto* b = static_cast<volatile char*>(p);
   for (size_t o = 0; o < bytes; o += kStep) {
@@ -188,6 +205,7 @@ extern "C" int mt_buf_alloc(mt_context* ctx, size_t bytes, mt_buffer** out) {
   CU(cudaSetDevice(ctx->device));
   void* p = nullptr;
   cudaError_t e = cudaMalloc(&p, bytes ? bytes : 1);
+  if (e == cudaErrorMemoryAllocation && drop_workspace(ctx)) e = cudaMalloc(&p, bytes ? bytes : 1);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(MT_ERR_NOMEM, "cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));

@@ -78,8 +78,7 @@ extern "C" int mt_batch_render(mt_context* ctx, mt_scene* s, const mt_batch_fram
   const size_t queues = 9 * R(total * 16) + 3 * R(total * 4),
                log = R(total * 16 * 2 * (size_t)max_depth) + R(total * 4);
   const size_t room = kWorkspaceMax > fixed ? (kWorkspaceMax - fixed) / (queues + log) : 0;
-  const int nbuf = (int)std::max<size_t>(1, std::min<size_t>({room, (size_t)max_spp, 4}));
-  const bool logged = nbuf > 1;
+  int nbuf = (int)std::max<size_t>(1, std::min<size_t>({room, (size_t)max_spp, 4}));
   while ((int)ctx->pass_streams.size() < nbuf) {
     mt_context::PassStream p;
     cudaError_t e = cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking);
@@ -90,8 +89,10 @@ extern "C" int mt_batch_render(mt_context* ctx, mt_scene* s, const mt_batch_fram
     if (e != cudaSuccess) return fail(MT_ERR_CUDA, "batch streams: %s", cudaGetErrorString(e));
   }
   Workspace ws;
-  int r = ws.get(ctx, fixed + nbuf * (queues + (logged ? log : 0)));
+  int r = ws.get(ctx, fixed + nbuf * (queues + (nbuf > 1 ? log : 0)));
+  if (r && nbuf > 1) r = ws.get(ctx, fixed + (nbuf = 1) * queues);  // memory is short: one pass after the other
   if (r) return r;
+  const bool logged = nbuf > 1;
   float4* film = ws.take<float4>(total);
   float4* film_c = ws.take<float4>(total);
   std::vector<FrameBufs> fbs(nbuf);

@@ -204,7 +204,6 @@ struct JobSlot {
   cudaEvent_t pfork = nullptr;  // the other buffers' streams start after the frame's set-up
   cudaEvent_t fork = nullptr, ev0 = nullptr, ev1 = nullptr, done = nullptr;
   cudaGraphExec_t graphs[2] = {nullptr, nullptr};  // of a frame among others, and of one alone (logged jobs)
-  unsigned graph_version = 0;  // scene version the graph was captured against
   bool ran = false;            // a frame has run on this slot (its control blocks hold its counts)
 };
 
@@ -287,6 +286,9 @@ struct Workspace {
   }
   static size_t round(size_t b) { return (b + 255) / 256 * 256; }
 };
+// Gives the scratch kept between calls back, where an allocation has failed (the context
+// lock held, no call using it); whether there was any.
+bool drop_workspace(mt_context* c);
 // Touches the pages of a host buffer that the caller is about to fill from the device,
 // until `ready` has happened: a fresh buffer's pages are then mapped while the GPU
 // still works, not one fault after the other during the copy (33 MB: 2 ms).

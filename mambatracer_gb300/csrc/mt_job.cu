@@ -328,16 +328,23 @@ extern "C" int mt_job_create(mt_context* ctx, mt_scene* scene, const mt_render_c
   const size_t fit = kOverlapBytes / (N * pass_bytes(cfg->max_depth));
   const int overlap =
       cfg->profile ? 1 : (int)std::min<size_t>(frames > 1 ? kOverlapMerged : kOverlap, std::max<size_t>(fit, 1));
-  const int nbuf = std::max(1, std::min({cfg->spp, kOverlap, overlap / frames}));
   j->merge = frames > 1;
-  j->nslots = j->merge ? frames : std::max(1, overlap / nbuf);
-  j->logged = nbuf > 1 || (!j->merge && j->nslots > 1);
-  j->slots.resize(j->nslots);
-  for (JobSlot& s : j->slots)
-    if (!r) r = alloc_slot(s, *cfg, nbuf, j->logged, j->merge || !j->logged, j->status_stride);
-  if (!r) r = dalloc(&j->d_totals, 4);
-  if (!r && (j->merge || j->logged)) r = dalloc(&j->d_film, N);
-  if (!r && (j->merge || j->logged)) r = dalloc(&j->d_film_c, N);
+  // Where memory is short: without the scratch kept for other calls, one pass at a time.
+  for (int at_once : {overlap, 1}) {
+    const int nbuf = std::max(1, std::min({cfg->spp, kOverlap, at_once / frames}));
+    j->nslots = j->merge ? frames : std::max(1, at_once / nbuf);
+    j->logged = nbuf > 1 || (!j->merge && j->nslots > 1);
+    j->slots.resize(j->nslots);
+    for (JobSlot& s : j->slots)
+      if (!r) r = alloc_slot(s, *cfg, nbuf, j->logged, j->merge || !j->logged, j->status_stride);
+    if (!r) r = dalloc(&j->d_totals, 4);
+    if (!r && (j->merge || j->logged)) r = dalloc(&j->d_film, N);
+    if (!r && (j->merge || j->logged)) r = dalloc(&j->d_film_c, N);
+    if (r != MT_ERR_NOMEM || at_once == 1) break;
+    free_job(j);
+    drop_workspace(ctx);
+    r = MT_OK;
+  }
   if (!r && cudaStreamCreateWithFlags(&j->rstream, cudaStreamNonBlocking) != cudaSuccess)
     r = fail(MT_ERR_CUDA, "stream create");
   if (!r && cudaEventCreateWithFlags(&j->rfork, cudaEventDisableTiming) != cudaSuccess)
@@ -718,6 +725,7 @@ int enqueue_read(mt_job* j, float* rgba, int resolve, mt_job::Read** out) {
   const bool divide = resolve && j->frames > 0;
   if (divide && !j->d_resolved) {
     int r = dalloc(&j->d_resolved, N);
+    if (r && drop_workspace(ctx)) r = dalloc(&j->d_resolved, N);
     if (r) return r;
   }
   CU(cudaEventRecord(j->rfork, ctx->stream));

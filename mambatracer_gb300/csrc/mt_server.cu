@@ -11,7 +11,7 @@
 // requests run at once; their kernels overlap on the GPU (persistent traversal
 // grids are sized by the frame, so a small request leaves SMs to the others).
 // Admission is first come, first served within a budget of path-state and film
-// bytes (200 B per pixel). A completed request's film is copied to pinned
+// bytes (counted as 200 B per pixel). A completed request's film is copied to pinned
 // staging and from there to the caller's buffer by the scheduler thread; a
 // host callback on the lane's stream wakes the scheduler, which measures the
 // request's latency from submission. Scenes are reference-counted while
@@ -25,9 +25,10 @@
 // kernel for all of them, and the streams overlap one another's last bounces.
 // Requests join at their stream's next round and leave when their last pass is
 // issued (continuous batching at pass granularity); a cancelled running request
-// stops at the next round. Slot k's film is the arena's k-th frame-sized
-// region, a stream's path state its slots' share of the arena. Per-round frame
-// tables live in a ring of kRounds entries per stream; a host callback at the
+// stops at the next round. A stream's rounds overlap on up to kSets sets of path
+// state, each with a log of its paths' contributions that is added to the films in
+// round order. Slot k's film is the arena's k-th frame-sized region, a stream's first
+// set its slots' share of the arena's queues. Per-round frame tables live in a ring of kRounds entries per stream; a host callback at the
 // end of each round frees its entry, which also keeps the scheduler at most
 // kRounds rounds ahead of the GPU on each stream. A merged pass keys every
 // path's samples on its own frame's pixel and frame number, so each film equals
@@ -319,14 +320,14 @@ void free_merged(mt_server* s) {
         if (e) cudaEventDestroy(e);
       dfree(Q.slab);
     }
-    G.sets.clear();
   }
+  s->groups.clear();
 }
 
 // Merged mode: the queues for lanes x N paths, the slots' films and pinned
 // staging, and per merge stream its slots, its share of the queues, its round
 // ring and its stream.
-int alloc_merged(mt_server* s, size_t N, int m) {
+int alloc_merged(mt_server* s, size_t N, int m, int nsets) {
   const size_t P = N * s->lanes.size();
   const int lanes = (int)s->lanes.size();
   s->groups.resize((size_t)m);
@@ -342,12 +343,11 @@ int alloc_merged(mt_server* s, size_t N, int m) {
   if (!r) r = dalloc(&s->mfb.hit_prim, P);
   if (!r) r = dalloc(&s->mfb.live, P);
   for (Lane& L : s->lanes)
-    if (!r && cudaMallocHost((void**)&L.h_stage, sizeof(float4) * N) != cudaSuccess)
+    if (!r && !L.h_stage && cudaMallocHost((void**)&L.h_stage, sizeof(float4) * N) != cudaSuccess)
       r = fail(MT_ERR_NOMEM, "pinned film staging");
   // sets of queues per stream: bytes a path of one set, and of a log
   auto R = Workspace::round;
   const size_t queue_bytes = 9 * 16 + 12, log_bytes = 32 * (size_t)s->cfg.max_depth + 4;
-  int nsets = kSets;
   while (nsets > 1 && P * ((nsets - 1) * queue_bytes + nsets * log_bytes) > kSetBytes) --nsets;
   size_t base = 0;  // first path of the group's share
   for (MergeGroup& G : s->groups) {
@@ -769,7 +769,14 @@ extern "C" int mt_server_create(mt_context* ctx, const mt_server_config* cfg, mt
     L.server = s;
     if (!r && !c.merged) r = alloc_lane(L, N, c.max_spp, c.max_depth, s->status_stride);
   }
-  if (!r && c.merged) r = alloc_merged(s, N, c.merged);
+  if (!r && c.merged) {
+    r = alloc_merged(s, N, c.merged, kSets);
+    if (r == MT_ERR_NOMEM) {  // memory is short: no kept scratch, one set of queues per stream
+      free_merged(s);
+      drop_workspace(ctx);
+      r = alloc_merged(s, N, c.merged, 1);
+    }
+  }
   if (!r && cudaMemset(s->d_totals, 0, 32) != cudaSuccess) r = fail(MT_ERR_CUDA, "memset");
   if (r) {
     std::string keep = mt_last_error();

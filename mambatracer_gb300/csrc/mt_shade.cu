@@ -143,8 +143,7 @@ __global__ void __launch_bounds__(kShadeThreads, MINB) k_shade(DevScene S, DevEn
   }
 }
 
-// Benchmark semantics in two launches (the default; MT_SHADE_SPLIT=0 runs the
-// single kernel above). k_shade_hit runs the hit record, the BSDF set-up and
+// Benchmark semantics in two launches (shade_split, by the pass's size). k_shade_hit runs the hit record, the BSDF set-up and
 // LightHitPass over the whole queue and lists the slots of the paths that go
 // on; k_shade_cont runs the texture pass, DirectLight, SampleBSDFRayDirection
 // and Russian roulette over that list alone. Each is half the code (less

@@ -756,5 +756,21 @@ __device__ __forceinline__ V radiance_env_grid(const DevEnv& E, const float* cam
   return c;
 }
 
+// The pixel of place i in an order by tiles of kTileW x kTileH pixels (ragged ones at the
+// right and the bottom): a warp's camera rays are a tile, and the queues of the later
+// bounces, which follow theirs, start near it too. By rows, tiles of 8 x 4, 4 x 8, 16 x 8, 16 x 16:
+// the 200k soup at 800 x 600, 4 passes, 6.70, 6.61, 6.57, 6.64, 6.63 ms, the 1M soup at 1080p,
+// 8 frames, 40.6, 40.4, 40.3, 40.5, 40.4 ms, a preview at 1280 x 720 826, 799, 793, 814, 814 us.
+constexpr int kTileW = 4, kTileH = 8;
+__device__ __forceinline__ int tile_pixel(int i, int W, int H) {
+  if (W < kTileW || H < kTileH) return i;  // also keeps the products below in range
+  const int band = i / (kTileH * W), h = min(kTileH, H - kTileH * band);
+  i -= band * kTileH * W;
+  const int col = i / (kTileW * h), w = min(kTileW, W - kTileW * col);
+  i -= col * kTileW * h;
+  const int y = i / w;
+  return (kTileH * band + y) * W + kTileW * col + i - y * w;
+}
+
 }  // namespace dv
 }  // namespace mt

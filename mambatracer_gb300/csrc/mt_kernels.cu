@@ -35,9 +35,11 @@ __global__ void k_raygen(const PassParams* __restrict__ pp, Ctrl* ctrl, FrameBuf
   const int id = blockIdx.x * blockDim.x + threadIdx.x;
   if (id == 0) ctrl->count[1] = N;
   if (id >= N) return;
+  // reference semantics key samples on the slot, which is the pixel
+  const int pixel = pp->mode == 0 ? id : tile_pixel(id, pp->width, pp->height);
   V o, dw;
-  camera_ray(pp, id, &o, &dw);
-  start_path(fb, id, o, dw);
+  camera_ray(pp, pixel, &o, &dw);
+  start_path(fb, id, pixel, o, dw);
 }
 
 // ----------------------------------------------------------- traversal
@@ -377,14 +379,15 @@ int launch_pass(cudaStream_t st, const DevScene& S, const DevEnv& E, const PassP
 namespace {
 // Camera rays of a merged batch pass: path g is pixel g - start[k] of frame k.
 __global__ void k_raygen_batch(BatchFrames B, int total, Ctrl* ctrl, FrameBufs fb) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g == 0) ctrl->count[1] = total;
-  if (g >= total) return;
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j == 0) ctrl->count[1] = total;
+  if (j >= total) return;
   PathState P;
-  B(g, P);
+  B(j, P);
+  const int pixel = tile_pixel(P.local, P.pp->width, P.pp->height);
   V o, dw;
-  camera_ray(P.pp, P.local, &o, &dw);
-  start_path(fb, g, o, dw);
+  camera_ray(P.pp, pixel, &o, &dw);
+  start_path(fb, j, j - P.local + pixel, o, dw);
 }
 }  // namespace
 

@@ -27,7 +27,8 @@ __device__ __forceinline__ int pack_argb(float r, float g, float b, float a) {  
 
 struct CameraRays {  // InitCameraRayData (Raytrace.cl:1-31)
   PassParams pp;
-  __device__ __forceinline__ tr::RayT operator()(int id) const {
+  __device__ __forceinline__ tr::RayT operator()(int i) const {
+    const int id = tile_pixel(i, pp.width, pp.height);
     const int W = pp.width;
     const float px = (float)(id % W), py = (float)(id / W);
     V d = normalize4(mk(pp.cam_a * (2.f * px / pp.dim_w - 1.f), -2.f * py / pp.dim_h + 1.f, -pp.cam_d, 0.f));
@@ -47,7 +48,9 @@ struct PreviewOut {  // setupBsdf's cosine, fastShade, backgroundShade, group
   DevEnv E;
   int* argb;
   int* group;
-  __device__ __forceinline__ void operator()(int id, const tr::RayT& r, int hit) const {
+  int width, height;
+  __device__ __forceinline__ void operator()(int i, const tr::RayT& r, int hit) const {
+    const int id = tile_pixel(i, width, height);
     const V d = mk(r.dx, r.dy, r.dz, 0.f);
     if (hit >= 0) {
       Hit H;
@@ -85,7 +88,7 @@ template <int MINB>
 __global__ void __launch_bounds__(kTraceThreads, MINB)
     k_preview(DevScene S, DevEnv E, PassParams pp, int n, int* argb, int* group, int* work, int* err) {
   bool overflow = false;
-  tr::trace_persistent<false, 32>(S, n, work, CameraRays{pp}, PreviewOut{S, E, argb, group}, &overflow);
+  tr::trace_persistent<false, 32>(S, n, work, CameraRays{pp}, PreviewOut{S, E, argb, group, pp.width, pp.height}, &overflow);
   if (overflow) atomicExch(err, kDevErrStack);
 }
 

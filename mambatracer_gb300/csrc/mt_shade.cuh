@@ -63,11 +63,11 @@ __device__ __forceinline__ void camera_ray(const PassParams* __restrict__ pp, in
   *o_out = o;
   *d_out = dw;
 }
-// Queue slot g of a new path. Its state is InitPathData's constants, which bounce 1
+// Queue slot j of a new path g. Its state is InitPathData's constants, which bounce 1
 // knows (queue_state).
-__device__ __forceinline__ void start_path(FrameBufs& fb, int g, V o, V dw) {
-  fb.q_o[0][g] = mk(o.x, o.y, o.z, __int_as_float(g));
-  fb.q_d[0][g] = mk(dw.x, dw.y, dw.z, 1.f);
+__device__ __forceinline__ void start_path(FrameBufs& fb, int j, int g, V o, V dw) {
+  fb.q_o[0][j] = mk(o.x, o.y, o.z, __int_as_float(g));
+  fb.q_d[0][j] = mk(dw.x, dw.y, dw.z, 1.f);
   if (fb.log) fb.log_n[g] = 0;
 }
 

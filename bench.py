@@ -67,7 +67,7 @@ WORKLOAD = WORKLOADS["soup"]["name"]
 RECORDS = {0: "FP32 child boxes, binary, 64 B records",
            1: "FP16 child boxes rounded outward, binary, 32 B records",
            2: "wide BVH: up to 8 children with 8-bit child boxes rounded outward, 96 B nodes",
-           3: "4-wide: a record's grandchildren with FP16 boxes rounded outward, 64 B nodes"}
+           3: "4-wide over a surface-area tree: FP16 boxes rounded outward, 64 B nodes"}
 
 
 def make_scene(kind, small, width, height):
@@ -605,7 +605,7 @@ def run_gpu(args):
             "gpu_launches": gpu_launches, "clocks": clk,
             "inflight_frames": args.inflight,
             "msamples_per_s": round(width * height * spp * args.steps * world / (ms * 1e-3) / 1e6, 2),
-            "bvh_depth": S.depth, "bvh_build_ms": round(bvh_build_ms, 2), "bvh_build": "GPU, level-synchronous",
+            "bvh_depth": S.depth, "bvh_build_ms": round(bvh_build_ms, 2), "bvh_build": "GPU",
             "bvh_records": RECORDS[args.precision],
             "alg_bytes_seconds": round(t_alg, 1), "launch_shapes": launch_shapes, "image_error": image_error,
         }

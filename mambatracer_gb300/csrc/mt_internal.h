@@ -294,8 +294,7 @@ bool drop_workspace(mt_context* c);
 // still works, not one fault after the other during the copy (33 MB: 2 ms).
 void prefault(void* p, size_t bytes, cudaEvent_t ready);
 
-// Resets the job's ARGB image to opaque black (InitIntDataRGB), on the context stream.
-void image_reset(mt_job* j);
+constexpr int kOpaqueBlack = (int)0xFF000000u;  // getIntARGB((0, 0, 0, 1))
 
 // Per-pass camera constants of InitCameraRayDataJitter from a 64-byte
 // CameraStruct, for a width x height frame.

@@ -235,14 +235,25 @@ int alloc_slot(JobSlot& s, const mt_render_config& c, int nbuf, bool logged, boo
   return r;
 }
 
-// Zeroes the job's film (a slot's film of a merge job is zeroed by each frame) on the
-// context stream.
-int clear_films(mt_job* j) {
+// Zeroes a film, and (where given) makes the ARGB image opaque black (InitIntDataRGB) and
+// zeroes the ray totals: one launch for a job's clear, where four cost 15 us.
+__global__ void k_clear(float4* __restrict__ film, float4* __restrict__ film_c, size_t n, int* __restrict__ argb,
+                        unsigned long long* __restrict__ totals) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (totals && i < 4) totals[i] = 0;
+  if (i >= n) return;
+  film[i] = film_c[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (argb) argb[i] = kOpaqueBlack;
+}
+
+// Clears the job's film (a slot's film of a merge job is zeroed by each frame), image and
+// ray totals on the context stream.
+int clear_job(mt_job* j) {
   const size_t N = (size_t)j->cfg.width * j->cfg.height;
   float4* f = j->d_film ? j->d_film : j->slots[0].film;
   float4* c = j->d_film ? j->d_film_c : j->slots[0].film_c;
-  CU(cudaMemsetAsync(f, 0, N * 16, j->ctx->stream));
-  CU(cudaMemsetAsync(c, 0, N * 16, j->ctx->stream));
+  k_clear<<<(unsigned)((N + 255) / 256), 256, 0, j->ctx->stream>>>(f, c, N, j->d_argb, j->d_totals);
+  CU(cudaGetLastError());
   return MT_OK;
 }
 
@@ -372,8 +383,7 @@ extern "C" int mt_job_create(mt_context* ctx, mt_scene* scene, const mt_render_c
     return r;
   }
   j->h_ctrl.resize(cfg->spp);
-  clear_films(j);
-  cudaMemsetAsync(j->d_totals, 0, 32, ctx->stream);
+  clear_job(j);
   CU(cudaStreamSynchronize(ctx->stream));
   ctx->jobs.push_back(j);
   *out = j;
@@ -449,11 +459,10 @@ int enqueue_frame(mt_job* j, JobSlot& s, bool direct) {
   const size_t per_pass_events = 2 + 3 * (size_t)c.max_depth;
   const size_t N = (size_t)c.width * c.height, status = j->status_stride * (size_t)c.max_depth;
   if (j->merge) {
-    CU(cudaMemsetAsync(s.film, 0, N * 16, s.stream));
-    CU(cudaMemsetAsync(s.film_c, 0, N * 16, s.stream));
+    k_clear<<<(unsigned)((N + 255) / 256), 256, 0, s.stream>>>(s.film, s.film_c, N, nullptr, nullptr);
+    CU(cudaGetLastError());
   }
   CU(cudaMemcpyAsync(s.d_pp, s.h_pp, sizeof(PassParams) * c.spp, cudaMemcpyHostToDevice, s.stream));
-  CU(cudaMemsetAsync(s.d_ctrl, 0, sizeof(Ctrl) * c.spp, s.stream));
   if (c.mode == 0) CU(cudaMemsetAsync(s.d_status, 0, status * c.spp * 8, s.stream));
   const int nbuf = (int)s.bufs.size();
   if (nbuf > 1) CU(cudaEventRecord(s.pfork, s.stream));
@@ -781,10 +790,8 @@ extern "C" int mt_film_clear(mt_job* j) {
   int r = finish_reads(j);
   if (r) return r;
   join_jobs(ctx);
-  r = clear_films(j);
+  r = clear_job(j);
   if (r) return r;
-  CU(cudaMemsetAsync(j->d_totals, 0, 32, ctx->stream));
-  image_reset(j);
   j->frames = 0;
   return MT_OK;
 }

@@ -15,6 +15,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cstddef>
 #include <cstdlib>
 
 #include "mt_device.cuh"
@@ -29,11 +30,14 @@ using namespace dv;
 // ----------------------------------------------------------------- raygen
 // InitCameraRayDataJitter (src/cl/kernel/Initialize.cl:129-172) with the
 // per-frame camera constants precomputed on the host, plus the path and queue
-// resets of InitPathData / InitIntersection / InitIntDataToIndex.
+// resets of InitPathData / InitIntersection / InitIntDataToIndex. Starts the pass's
+// control block too (a memset of its own in front of the pass costs 2 us).
 __global__ void k_raygen(const PassParams* __restrict__ pp, Ctrl* ctrl, FrameBufs fb) {
   const int N = pp->width * pp->height;
   const int id = blockIdx.x * blockDim.x + threadIdx.x;
-  if (id == 0) ctrl->count[1] = N;
+  static_assert(offsetof(Ctrl, count) == 0, "count[1] is word 1");
+  if (blockIdx.x == 0)
+    for (int k = threadIdx.x; k < (int)(sizeof(Ctrl) / 4); k += blockDim.x) reinterpret_cast<int*>(ctrl)[k] = k == 1 ? N : 0;
   if (id >= N) return;
   // reference semantics key samples on the slot, which is the pixel
   const int pixel = pp->mode == 0 ? id : tile_pixel(id, pp->width, pp->height);

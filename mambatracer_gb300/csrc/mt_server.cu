@@ -270,7 +270,6 @@ int start_request(mt_server* s, Lane& L, Request* R) {
   }
   const size_t stride = (N + kShadeThreads - 1) / kShadeThreads;
   CU(cudaMemcpyAsync(L.d_pp, L.h_pp, sizeof(PassParams) * R->spp, cudaMemcpyHostToDevice, L.stream));
-  CU(cudaMemsetAsync(L.d_ctrl, 0, sizeof(Ctrl) * R->spp, L.stream));
   CU(cudaMemsetAsync(L.d_status, 0, stride * (size_t)c.max_depth * R->spp * 8, L.stream));
   CU(cudaMemsetAsync(L.fb.film, 0, N * 16, L.stream));
   CU(cudaMemsetAsync(L.fb.film_c, 0, N * 16, L.stream));

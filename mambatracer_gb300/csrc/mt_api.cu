@@ -12,6 +12,7 @@
 #include <deque>
 #include <mutex>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "mt_compact.h"
@@ -25,6 +26,31 @@ thread_local std::string g_err;
 
 extern "C" const char* mt_last_error(void) { return g_err.c_str(); }
 
+namespace {
+// MT_DEVICE_ROOM's account of the library's arrays.
+struct DeviceRoom {
+  const bool on = std::getenv("MT_DEVICE_ROOM") != nullptr;
+  std::mutex mu;
+  std::unordered_map<void*, size_t> sizes;
+  size_t live = 0, limit = SIZE_MAX;
+  std::string seen;
+  // bytes the arrays may still grow by (mu held)
+  size_t left() {
+    const char* e = std::getenv("MT_DEVICE_ROOM");
+    if (!e) e = "";
+    if (seen != e) {
+      seen = e;
+      limit = *e ? live + (size_t)std::strtoull(e, nullptr, 10) : SIZE_MAX;
+    }
+    return limit > live ? limit - live : 0;
+  }
+};
+DeviceRoom& device_room() {
+  static DeviceRoom r;
+  return r;
+}
+}  // namespace
+
 namespace mt {
 __attribute__((visibility("hidden"))) void set_last_error(const char* msg) { g_err = msg; }
 __attribute__((visibility("hidden"))) int fail(int code, const char* fmt, ...) {
@@ -35,6 +61,25 @@ __attribute__((visibility("hidden"))) int fail(int code, const char* fmt, ...) {
   va_end(ap);
   g_err = buf;
   return code;
+}
+
+__attribute__((visibility("hidden"))) cudaError_t device_malloc(void** p, size_t bytes) {
+  DeviceRoom& r = device_room();
+  if (!r.on) return cudaMalloc(p, bytes);
+  std::lock_guard<std::mutex> lk(r.mu);
+  if (bytes > r.left()) return cudaErrorMemoryAllocation;
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaSuccess) r.live += r.sizes[*p] = bytes;
+  return e;
+}
+__attribute__((visibility("hidden"))) void device_free(void* p) {
+  DeviceRoom& r = device_room();
+  if (r.on) {
+    std::lock_guard<std::mutex> lk(r.mu);
+    r.live -= r.sizes[p];
+    r.sizes.erase(p);
+  }
+  cudaFree(p);
 }
 }  // namespace mt
 
@@ -57,7 +102,7 @@ int Workspace::get(mt_context* c, size_t bytes) {
   ctx = c;
   at = 0;
   own = bytes > kWorkspaceMax;
-  if (own) return dalloc(&base, bytes);
+  if (own) return dalloc(c, &base, bytes);
   if (bytes > c->ws_bytes) {
     // grown in steps, so calls of slowly growing sizes do not allocate each time
     const size_t grown = std::min(kWorkspaceMax, std::max({bytes, 2 * c->ws_bytes, (size_t)1 << 20}));
@@ -71,16 +116,18 @@ int Workspace::get(mt_context* c, size_t bytes) {
     c->ws_bytes = got;
   }
   base = c->ws;
+  c->ws_used = true;
   return MT_OK;
 }
 
 void Workspace::release() {
   if (own) dfree(base);
+  else if (base) ctx->ws_used = false;
   base = nullptr;
 }
 
 bool drop_workspace(mt_context* c) {
-  if (!c->ws) return false;
+  if (!c->ws || c->ws_used) return false;
   cudaStreamSynchronize(c->stream);
   dfree(c->ws);
   c->ws_bytes = 0;
@@ -204,8 +251,8 @@ extern "C" int mt_buf_alloc(mt_context* ctx, size_t bytes, mt_buffer** out) {
   std::lock_guard<std::recursive_mutex> lk(ctx->mu);
   CU(cudaSetDevice(ctx->device));
   void* p = nullptr;
-  cudaError_t e = cudaMalloc(&p, bytes ? bytes : 1);
-  if (e == cudaErrorMemoryAllocation && drop_workspace(ctx)) e = cudaMalloc(&p, bytes ? bytes : 1);
+  cudaError_t e = device_malloc(&p, bytes ? bytes : 1);
+  if (e == cudaErrorMemoryAllocation && drop_workspace(ctx)) e = device_malloc(&p, bytes ? bytes : 1);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(MT_ERR_NOMEM, "cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
@@ -268,7 +315,7 @@ extern "C" int mt_buf_free(mt_buffer* b) {
     std::lock_guard<std::recursive_mutex> lk(b->ctx->mu);
     cudaSetDevice(b->ctx->device);
     cudaStreamSynchronize(b->ctx->stream);
-    cudaFree(b->ptr);
+    device_free(b->ptr);
   }
   delete b;
   return MT_OK;
@@ -292,9 +339,9 @@ int upload_lights(mt_scene* s) {
 }
 
 template <class T>
-int upload(T** d, const void* h, size_t count) {
+int upload(mt_context* c, T** d, const void* h, size_t count) {
   dfree(*d);
-  int r = dalloc(d, count);
+  int r = dalloc(c, d, count);
   if (r) return r;
   if (h && count) CU(cudaMemcpy(*d, h, count * sizeof(T), cudaMemcpyHostToDevice));
   return MT_OK;
@@ -340,7 +387,7 @@ int alloc_env(mt_scene* s, int w, int h, bool with64) {
   const size_t bytes = R(16 * n) + 2 * R(4 * n) + (with64 ? R(8 * n) : 0) + (tables ? R(4 * marg) + R(4 * cond) : 0);
   if (bytes != s->env_bytes || w != s->env_w || h != s->env_h) {
     free_env(s);
-    int r = dalloc(&s->d_env, bytes);
+    int r = dalloc(s->ctx, &s->d_env, bytes);
     if (r) return r;
     s->env_bytes = bytes;
   }
@@ -390,8 +437,8 @@ int upload_textures(mt_scene* s) {
     ref[i] = make_int4(t.argb.empty() ? 0 : (int)pool.size(), t.argb.empty() ? 0 : t.w, t.argb.empty() ? 0 : t.h, 0);
     pool.insert(pool.end(), t.argb.begin(), t.argb.end());
   }
-  int r = upload(&s->d_texels, pool.data(), pool.size());
-  if (!r) r = upload(&s->d_tex_ref, ref.data(), ref.size());
+  int r = upload(s->ctx, &s->d_texels, pool.data(), pool.size());
+  if (!r) r = upload(s->ctx, &s->d_tex_ref, ref.data(), ref.size());
   if (r) return r;
   s->tex_on = 1;
   return MT_OK;
@@ -421,7 +468,7 @@ extern "C" int mt_scene_create(mt_context* ctx, const float* points, int npoints
   if (!normals) s->nnormals = 0;
   const size_t b_pts = Workspace::round(16 * (size_t)npoints), b_uvs = Workspace::round(8 * (size_t)std::max(s->nuvs, 1)),
                b_nrm = Workspace::round(16 * (size_t)std::max(s->nnormals, 1));
-  int r = dalloc(&s->d_mesh, b_pts + b_uvs + b_nrm + 40 * (size_t)nfaces);
+  int r = dalloc(ctx, &s->d_mesh, b_pts + b_uvs + b_nrm + 40 * (size_t)nfaces);
   if (!r) {
     s->d_points = (float4*)s->d_mesh;
     s->d_uvs = (float2*)(s->d_mesh + b_pts);
@@ -449,7 +496,7 @@ extern "C" int mt_scene_create(mt_context* ctx, const float* points, int npoints
     else
       r = fail(MT_ERR_INVALID, "face %d: normal index out of range", bad);
   }
-  if (!r) r = upload(&s->d_materials, materials, (size_t)nmaterials);
+  if (!r) r = upload(ctx, &s->d_materials, materials, (size_t)nmaterials);
   if (!r) r = upload_lights(s);
   if (r) {
     std::string keep = g_err;
@@ -480,7 +527,7 @@ extern "C" int mt_scene_set_materials(mt_scene* s, const void* materials, int nm
   ++s->version;
   s->h_materials.assign((const uint8_t*)materials, (const uint8_t*)materials + 144 * (size_t)nmaterials);
   s->nmat = nmaterials;
-  int r = upload(&s->d_materials, materials, (size_t)nmaterials);
+  int r = upload(s->ctx, &s->d_materials, materials, (size_t)nmaterials);
   if (!r) r = upload_lights(s);
   if (!r) r = upload_textures(s);
   return r;
@@ -708,9 +755,9 @@ int import_bvh(mt_scene* s, const int32_t* nodes, const float* bounds, int nnode
     r[3] = make_float4(lf, rf, 0.f, 0.f);
   }
   if ((int)order.size() != n) return fail(MT_ERR_INVALID, "BVH reaches %zu of %d triangles", order.size(), n);
-  int r = upload(&s->d_nodes, hn.data(), hn.size());
+  int r = upload(s->ctx, &s->d_nodes, hn.data(), hn.size());
   dfree(s->d_tris);
-  if (!r) r = dalloc(&s->d_tris, 3 * (size_t)n);
+  if (!r) r = dalloc(s->ctx, &s->d_tris, 3 * (size_t)n);
   if (!r) r = order_triangles(s, order, s->d_tris);
   if (r) return r;
   s->nrec = nrec;
@@ -908,9 +955,9 @@ extern "C" int mt_env_grid_sat(mt_context* ctx, const float* func, float* sat_ou
   size_t n = (size_t)nu * nv;
   float *d_func = nullptr, *d_sat = nullptr;
   double* d_sat64 = nullptr;
-  int r = dalloc(&d_func, n);
-  if (!r) r = dalloc(&d_sat, n);
-  if (!r && fp64) r = dalloc(&d_sat64, n);
+  int r = dalloc(ctx, &d_func, n);
+  if (!r) r = dalloc(ctx, &d_sat, n);
+  if (!r && fp64) r = dalloc(ctx, &d_sat64, n);
   if (!r) {
     cudaMemcpyAsync(d_func, func, n * 4, cudaMemcpyHostToDevice, ctx->stream);
     if (launch_grid_sat(ctx->stream, d_func, d_sat, d_sat64, nu, nv, rx, ry, fp64))
@@ -1043,8 +1090,8 @@ extern "C" int mt_compact_isects(mt_context* ctx, const void* isects_in, const i
     dfree(ctx->cs_status);
     dfree(ctx->cs_words);
     ctx->cs_tiles = 0;
-    int r = dalloc(&ctx->cs_status, tiles ? tiles : 1);
-    if (!r) r = dalloc(&ctx->cs_words, 4);
+    int r = dalloc(ctx, &ctx->cs_status, tiles ? tiles : 1);
+    if (!r) r = dalloc(ctx, &ctx->cs_words, 4);
     if (r) return r;
     ctx->cs_tiles = tiles ? tiles : 1;
   }

@@ -635,9 +635,11 @@ extern "C" int mt_bvh_build_device(mt_scene* s, int32_t* nodes_out, float* bound
                b_ref = nodes_out ? align(28 * nn) : 0, b_bound = bounds_out ? align(32 * nn) : 0;
   Workspace ws;
   float4 *recs = nullptr, *tris = nullptr;
-  int r = ws.get(ctx, 2 * b_prim + 2 * b_node + b_small + b_cnt + b_ref + b_bound + 256);
-  if (!r) r = dalloc(&recs, 4 * (size_t)std::max(nrec, 1));
-  if (!r) r = dalloc(&tris, 3 * (size_t)n);
+  // the tree's arrays first: they can take the place of the scratch that is kept, not of
+  // the scratch in use
+  int r = dalloc(ctx, &recs, 4 * (size_t)std::max(nrec, 1));
+  if (!r) r = dalloc(ctx, &tris, 3 * (size_t)n);
+  if (!r) r = ws.get(ctx, 2 * b_prim + 2 * b_node + b_small + b_cnt + b_ref + b_bound + 256);
   auto fail_all = [&](int code, const char* msg) {
     std::string keep = msg ? std::string(msg) : mt_last_error();
     cudaStreamSynchronize(st);
@@ -717,7 +719,7 @@ int refresh_qnodes(mt_scene* s) {
   dfree(s->d_quad);
   dfree(s->d_up);
   if (traversal_bitstack() && s->has_bvh && s->nrec > 0) {
-    int r = dalloc(&s->d_up, (size_t)s->nrec);
+    int r = dalloc(s->ctx, &s->d_up, (size_t)s->nrec);
     if (r) return r;
     cudaStream_t st = s->ctx->stream;
     k_up_links<<<blocks(s->nrec), kT, 0, st>>>(s->d_nodes, s->nrec, s->root_ref, s->d_up);
@@ -750,7 +752,7 @@ int refresh_qnodes(mt_scene* s) {
     return MT_OK;
   }
   if (s->precision != 1 || !s->has_bvh || s->nrec == 0) return MT_OK;
-  int r = dalloc(&s->d_qnodes, 2 * (size_t)s->nrec);
+  int r = dalloc(s->ctx, &s->d_qnodes, 2 * (size_t)s->nrec);
   if (r) return r;
   cudaStream_t st = s->ctx->stream;
   k_quantize_fp16<<<blocks(s->nrec), kT, 0, st>>>(s->d_nodes, s->nrec, s->d_qnodes);

@@ -170,11 +170,11 @@ int ensure_image(mt_job* j) {
   if (j->d_argb) return MT_OK;
   const size_t N = (size_t)j->cfg.width * j->cfg.height;
   const int nparts = (int)((N + kToneThreads - 1) / kToneThreads);
-  int r = dalloc(&j->d_argb, N);
-  if (!r) r = dalloc(&j->d_fb, N);
-  if (!r) r = dalloc(&j->d_tone_part, (size_t)nparts);
-  if (!r) r = dalloc(&j->d_tone_cnt, (size_t)nparts);
-  if (!r) r = dalloc(&j->d_tone_tot, 3);  // total, count, blocks that have ended
+  int r = dalloc(j->ctx, &j->d_argb, N);
+  if (!r) r = dalloc(j->ctx, &j->d_fb, N);
+  if (!r) r = dalloc(j->ctx, &j->d_tone_part, (size_t)nparts);
+  if (!r) r = dalloc(j->ctx, &j->d_tone_cnt, (size_t)nparts);
+  if (!r) r = dalloc(j->ctx, &j->d_tone_tot, 3);  // total, count, blocks that have ended
   if (r) return r;
   CU(cudaMemsetAsync(j->d_tone_tot, 0, 12, j->ctx->stream));
   k_argb_fill<<<(unsigned)((N + 255) / 256), 256, 0, j->ctx->stream>>>(j->d_argb, N);

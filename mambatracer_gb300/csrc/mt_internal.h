@@ -16,6 +16,7 @@
 
 using namespace mt;
 
+struct mt_context;
 struct mt_job;
 struct mt_server;
 
@@ -23,8 +24,18 @@ struct mt_server;
 namespace mt {
 // Records the message mt_last_error() returns on this thread; returns code.
 __attribute__((visibility("hidden"))) int fail(int code, const char* fmt, ...);
+// cudaMalloc and cudaFree of the library's arrays. MT_DEVICE_ROOM in the environment, where
+// it is set when the process allocates its first array, makes the device look nearly
+// full: the arrays may grow by that many bytes beyond what they held when the value was
+// first seen (empty: no limit; the value may change while the process runs).
+__attribute__((visibility("hidden"))) cudaError_t device_malloc(void** p, size_t bytes);
+__attribute__((visibility("hidden"))) void device_free(void* p);
 }  // namespace mt
 using mt::fail;
+
+// Gives the scratch kept between calls back, where an allocation has failed (the context
+// lock held); false when there is none or a call is using it.
+bool drop_workspace(mt_context* c);
 
 namespace {
 #define CU(call)                                                                         \
@@ -37,16 +48,23 @@ template <class T>
 int dalloc(T** p, size_t count) {
   *p = nullptr;
   if (count == 0) count = 1;
-  cudaError_t e = cudaMalloc((void**)p, count * sizeof(T));
+  cudaError_t e = mt::device_malloc((void**)p, count * sizeof(T));
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(MT_ERR_NOMEM, "cudaMalloc(%zu B): %s", count * sizeof(T), cudaGetErrorString(e));
   }
   return MT_OK;
 }
+// As above, and once more without the scratch kept between the context's calls: what fits
+// the device without it is not refused because of an earlier call (the context lock held).
+template <class T>
+int dalloc(mt_context* c, T** p, size_t count) {
+  const int r = dalloc(p, count);
+  return r == MT_ERR_NOMEM && drop_workspace(c) ? dalloc(p, count) : r;
+}
 template <class T>
 void dfree(T*& p) {
-  if (p) cudaFree((void*)p);
+  if (p) mt::device_free((void*)p);
   p = nullptr;
 }
 }  // namespace
@@ -65,17 +83,19 @@ struct mt_context {
   int* cs_words = nullptr;
   size_t cs_tiles = 0;
   // Scratch of the calls that use device memory only until they return (ray queries,
-  // previews, batches), kept between them: allocating and freeing it cost 80-280 us a
+  // previews, batches, builds), kept between them: allocating and freeing it cost 80-280 us a
   // call. Used on `stream` under `mu`, so one call at a time; at most kWorkspaceMax
-  // bytes are kept (a larger call allocates its own), and they go with the context.
+  // bytes are kept (a larger call allocates its own), given back when an allocation of
+  // the context fails (drop_workspace) and with the context.
+  char* ws = nullptr;
+  size_t ws_bytes = 0;
+  bool ws_used = false;  // a call is using it
   // streams of a batch's overlapping passes, created by the first batch
   struct PassStream {
     cudaStream_t stream = nullptr, side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr, done = nullptr;
   };
   std::vector<PassStream> pass_streams;
-  char* ws = nullptr;
-  size_t ws_bytes = 0;
   std::vector<mt_job*> jobs;  // jobs whose streams join into `stream`
   std::vector<mt_server*> servers;  // served-mode schedulers on this context
   int* d_plain_err = nullptr;       // error latched by kernels launched by name
@@ -286,9 +306,6 @@ struct Workspace {
   }
   static size_t round(size_t b) { return (b + 255) / 256 * 256; }
 };
-// Gives the scratch kept between calls back, where an allocation has failed (the context
-// lock held, no call using it); whether there was any.
-bool drop_workspace(mt_context* c);
 // Touches the pages of a host buffer that the caller is about to fill from the device,
 // until `ready` has happened: a fresh buffer's pages are then mapped while the GPU
 // still works, not one fault after the other during the copy (33 MB: 2 ms).

@@ -178,7 +178,7 @@ size_t pass_bytes(int max_depth) { return 6 * 16 + 8 + 48 + 4 + 4 + 32 * (size_t
 
 // A slot's device memory is one allocation (an allocation costs 40 us and more, whatever
 // its size up to some MB): sized in a first walk over the arrays, handed out in a second.
-int alloc_slot(JobSlot& s, const mt_render_config& c, int nbuf, bool logged, bool own_film, size_t status_stride) {
+int alloc_slot(mt_context* ctx, JobSlot& s, const mt_render_config& c, int nbuf, bool logged, bool own_film, size_t status_stride) {
   const size_t N = (size_t)c.width * c.height;
   int r = MT_OK;
   if (cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking) != cudaSuccess)
@@ -211,7 +211,7 @@ int alloc_slot(JobSlot& s, const mt_render_config& c, int nbuf, bool logged, boo
     take(&s.d_ctrl, (size_t)c.spp);
     if (c.mode == 0) take(&s.d_status, status_stride * (size_t)c.max_depth * c.spp);
     take(&s.d_pp, (size_t)c.spp);
-    if (walk == 0) r = dalloc(&s.slab, at);
+    if (walk == 0) r = dalloc(ctx, &s.slab, at);
   }
   for (PassBuf& B : s.bufs) {
     B.fb.film = s.film;
@@ -292,17 +292,17 @@ int setup_grid(mt_job* j) {
     j->rx = sc->grid_rx;
     j->ry = sc->grid_ry;
     j->grid_fp64 = sc->grid_on == 2;
-    r = dalloc(&j->d_grid_func, n);
-    if (!r) r = dalloc(&j->d_grid_sat, n);
-    if (!r) r = dalloc(&j->d_grid_accum, n);
-    if (!r && j->grid_fp64) r = dalloc(&j->d_grid_sat64, n);
+    r = dalloc(j->ctx, &j->d_grid_func, n);
+    if (!r) r = dalloc(j->ctx, &j->d_grid_sat, n);
+    if (!r) r = dalloc(j->ctx, &j->d_grid_accum, n);
+    if (!r && j->grid_fp64) r = dalloc(j->ctx, &j->d_grid_sat64, n);
     size_t cm = 0, tm = 0;
     const size_t cc = cell_table_floats(j->nu, j->nv, j->rx, j->ry, &cm);
     const size_t tc = tile_table_floats(sc->env_w, sc->env_h, j->rx, j->ry, &tm);
-    if (!r) r = dalloc(&j->d_cell_marg, cm);
-    if (!r) r = dalloc(&j->d_cell_cond, cc);
-    if (!r) r = dalloc(&j->d_tile_marg, tm);
-    if (!r) r = dalloc(&j->d_tile_cond, tc);
+    if (!r) r = dalloc(j->ctx, &j->d_cell_marg, cm);
+    if (!r) r = dalloc(j->ctx, &j->d_cell_cond, cc);
+    if (!r) r = dalloc(j->ctx, &j->d_tile_marg, tm);
+    if (!r) r = dalloc(j->ctx, &j->d_tile_cond, tc);
     if (r) return r;
   }
   CU(cudaMemsetAsync(j->d_grid_accum, 0, n * 4, ctx->stream));
@@ -340,20 +340,19 @@ extern "C" int mt_job_create(mt_context* ctx, mt_scene* scene, const mt_render_c
   const int overlap =
       cfg->profile ? 1 : (int)std::min<size_t>(frames > 1 ? kOverlapMerged : kOverlap, std::max<size_t>(fit, 1));
   j->merge = frames > 1;
-  // Where memory is short: without the scratch kept for other calls, one pass at a time.
+  // Where memory is short: one pass at a time.
   for (int at_once : {overlap, 1}) {
     const int nbuf = std::max(1, std::min({cfg->spp, kOverlap, at_once / frames}));
     j->nslots = j->merge ? frames : std::max(1, at_once / nbuf);
     j->logged = nbuf > 1 || (!j->merge && j->nslots > 1);
     j->slots.resize(j->nslots);
     for (JobSlot& s : j->slots)
-      if (!r) r = alloc_slot(s, *cfg, nbuf, j->logged, j->merge || !j->logged, j->status_stride);
-    if (!r) r = dalloc(&j->d_totals, 4);
-    if (!r && (j->merge || j->logged)) r = dalloc(&j->d_film, N);
-    if (!r && (j->merge || j->logged)) r = dalloc(&j->d_film_c, N);
+      if (!r) r = alloc_slot(ctx, s, *cfg, nbuf, j->logged, j->merge || !j->logged, j->status_stride);
+    if (!r) r = dalloc(j->ctx, &j->d_totals, 4);
+    if (!r && (j->merge || j->logged)) r = dalloc(j->ctx, &j->d_film, N);
+    if (!r && (j->merge || j->logged)) r = dalloc(j->ctx, &j->d_film_c, N);
     if (r != MT_ERR_NOMEM || at_once == 1) break;
     free_job(j);
-    drop_workspace(ctx);
     r = MT_OK;
   }
   if (!r && cudaStreamCreateWithFlags(&j->rstream, cudaStreamNonBlocking) != cudaSuccess)
@@ -733,8 +732,7 @@ int enqueue_read(mt_job* j, float* rgba, int resolve, mt_job::Read** out) {
   const size_t N = (size_t)j->cfg.width * j->cfg.height;
   const bool divide = resolve && j->frames > 0;
   if (divide && !j->d_resolved) {
-    int r = dalloc(&j->d_resolved, N);
-    if (r && drop_workspace(ctx)) r = dalloc(&j->d_resolved, N);
+    int r = dalloc(ctx, &j->d_resolved, N);
     if (r) return r;
   }
   CU(cudaEventRecord(j->rfork, ctx->stream));

@@ -118,7 +118,7 @@ int list_light_faces(mt_scene* s, const std::vector<unsigned char>& emits) {
   if (e != cudaSuccess) r = fail(MT_ERR_CUDA, "light list: %s", cudaGetErrorString(e));
   else if (h[2]) r = fail(MT_ERR_DEVICE, "light list: device error %d", h[2]);
   if (!r && h[1] > 0) {
-    r = dalloc(&s->d_light_faces, (size_t)h[1]);
+    r = dalloc(ctx, &s->d_light_faces, (size_t)h[1]);
     if (!r && (cudaMemcpyAsync(s->d_light_faces, list, 4 * (size_t)h[1], cudaMemcpyDeviceToDevice, ctx->stream) !=
                    cudaSuccess ||
                cudaStreamSynchronize(ctx->stream) != cudaSuccess))

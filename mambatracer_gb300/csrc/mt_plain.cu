@@ -1082,7 +1082,7 @@ extern "C" int mt_kernel_create(mt_context* ctx, const char* name, mt_kernel** o
       std::lock_guard<std::recursive_mutex> lk(ctx->mu);
       CU(cudaSetDevice(ctx->device));
       if (!ctx->d_plain_err) {
-        int r = dalloc(&ctx->d_plain_err, 1);
+        int r = dalloc(ctx, &ctx->d_plain_err, 1);
         if (r) return r;
         CU(cudaMemset(ctx->d_plain_err, 0, 4));
       }
@@ -1301,8 +1301,8 @@ extern "C" int mt_launch_1d(mt_kernel* k, size_t global, size_t local) {
         dfree(ctx->cs_status);
         dfree(ctx->cs_words);
         ctx->cs_tiles = 0;
-        int r = dalloc(&ctx->cs_status, tiles);
-        if (!r) r = dalloc(&ctx->cs_words, 4);
+        int r = dalloc(ctx, &ctx->cs_status, tiles);
+        if (!r) r = dalloc(ctx, &ctx->cs_words, 4);
         if (r) return r;
         ctx->cs_tiles = tiles;
       }

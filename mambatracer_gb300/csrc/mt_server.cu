@@ -219,25 +219,25 @@ void free_lane(Lane& L) {
   }
 }
 
-int alloc_lane(Lane& L, size_t N, int spp, int depth, size_t stride) {
+int alloc_lane(mt_context* ctx, Lane& L, size_t N, int spp, int depth, size_t stride) {
   int r = MT_OK;
   for (int k = 0; k < 2 && !r; ++k) {
-    r = dalloc(&L.fb.q_o[k], N);
-    if (!r) r = dalloc(&L.fb.q_d[k], N);
+    r = dalloc(ctx, &L.fb.q_o[k], N);
+    if (!r) r = dalloc(ctx, &L.fb.q_d[k], N);
   }
-  if (!r) r = dalloc(&L.fb.hit_t, N);
-  if (!r) r = dalloc(&L.fb.hit_prim, N);
-  if (!r) r = dalloc(&L.fb.q_t[0], N);
-  if (!r) r = dalloc(&L.fb.q_t[1], N);
-  if (!r) r = dalloc(&L.fb.s_o, N);
-  if (!r) r = dalloc(&L.fb.s_d, N);
-  if (!r) r = dalloc(&L.fb.s_c, N);
-  if (!r) r = dalloc(&L.fb.film, N);
-  if (!r) r = dalloc(&L.fb.film_c, N);
-  if (!r) r = dalloc(&L.fb.live, N);
-  if (!r) r = dalloc(&L.d_ctrl, (size_t)spp);
-  if (!r) r = dalloc(&L.d_status, stride * (size_t)depth * spp);
-  if (!r) r = dalloc(&L.d_pp, (size_t)spp);
+  if (!r) r = dalloc(ctx, &L.fb.hit_t, N);
+  if (!r) r = dalloc(ctx, &L.fb.hit_prim, N);
+  if (!r) r = dalloc(ctx, &L.fb.q_t[0], N);
+  if (!r) r = dalloc(ctx, &L.fb.q_t[1], N);
+  if (!r) r = dalloc(ctx, &L.fb.s_o, N);
+  if (!r) r = dalloc(ctx, &L.fb.s_d, N);
+  if (!r) r = dalloc(ctx, &L.fb.s_c, N);
+  if (!r) r = dalloc(ctx, &L.fb.film, N);
+  if (!r) r = dalloc(ctx, &L.fb.film_c, N);
+  if (!r) r = dalloc(ctx, &L.fb.live, N);
+  if (!r) r = dalloc(ctx, &L.d_ctrl, (size_t)spp);
+  if (!r) r = dalloc(ctx, &L.d_status, stride * (size_t)depth * spp);
+  if (!r) r = dalloc(ctx, &L.d_pp, (size_t)spp);
   if (!r && cudaMallocHost((void**)&L.h_pp, sizeof(PassParams) * spp) != cudaSuccess)
     r = fail(MT_ERR_NOMEM, "pinned pass parameters");
   if (!r && cudaMallocHost((void**)&L.h_stage, sizeof(float4) * N) != cudaSuccess)
@@ -337,10 +337,10 @@ int alloc_merged(mt_server* s, size_t N, int m, int nsets) {
   int r = MT_OK;
   for (auto* p : {&s->mfb.q_o[0], &s->mfb.q_o[1], &s->mfb.q_d[0], &s->mfb.q_d[1], &s->mfb.q_t[0], &s->mfb.q_t[1],
                   &s->mfb.s_o, &s->mfb.s_d, &s->mfb.s_c, &s->mfb.film, &s->mfb.film_c})
-    if (!r) r = dalloc(p, P);
-  if (!r) r = dalloc(&s->mfb.hit_t, P);
-  if (!r) r = dalloc(&s->mfb.hit_prim, P);
-  if (!r) r = dalloc(&s->mfb.live, P);
+    if (!r) r = dalloc(s->ctx, p, P);
+  if (!r) r = dalloc(s->ctx, &s->mfb.hit_t, P);
+  if (!r) r = dalloc(s->ctx, &s->mfb.hit_prim, P);
+  if (!r) r = dalloc(s->ctx, &s->mfb.live, P);
   for (Lane& L : s->lanes)
     if (!r && !L.h_stage && cudaMallocHost((void**)&L.h_stage, sizeof(float4) * N) != cudaSuccess)
       r = fail(MT_ERR_NOMEM, "pinned film staging");
@@ -357,9 +357,9 @@ int alloc_merged(mt_server* s, size_t N, int m, int nsets) {
         r = fail(MT_ERR_NOMEM, "pinned round tables");
       if (!r && cudaMallocHost((void**)&Rd.h_pp, sizeof(PassParams) * n) != cudaSuccess)
         r = fail(MT_ERR_NOMEM, "pinned round tables");
-      if (!r) r = dalloc(&Rd.d_tab, (size_t)3 * n);
-      if (!r) r = dalloc(&Rd.d_pp, (size_t)n);
-      if (!r) r = dalloc(&Rd.d_ctrl, (size_t)n);
+      if (!r) r = dalloc(s->ctx, &Rd.d_tab, (size_t)3 * n);
+      if (!r) r = dalloc(s->ctx, &Rd.d_pp, (size_t)n);
+      if (!r) r = dalloc(s->ctx, &Rd.d_ctrl, (size_t)n);
       if (!r && cudaEventCreateWithFlags(&Rd.done, cudaEventDisableTiming) != cudaSuccess)
         r = fail(MT_ERR_CUDA, "event create");
     }
@@ -378,7 +378,7 @@ int alloc_merged(mt_server* s, size_t N, int m, int nsets) {
       Q.fb = s->mfb;  // films stay whole: slot k's film is at k x N
       const size_t queues = k > 0 ? 9 * R(16 * paths) + 3 * R(4 * paths) : 0;
       const size_t log = nsets > 1 ? R(32 * paths * s->cfg.max_depth) + R(4 * paths) : 0;
-      if (queues + log > 0) r = dalloc(&Q.slab, queues + log);
+      if (queues + log > 0) r = dalloc(s->ctx, &Q.slab, queues + log);
       if (r) break;
       char* at = Q.slab;
       auto take = [&](size_t b) {
@@ -763,16 +763,15 @@ extern "C" int mt_server_create(mt_context* ctx, const mt_server_config* cfg, mt
   const size_t N = (size_t)c.max_width * c.max_height;
   s->status_stride = (N + kShadeThreads - 1) / kShadeThreads;
   s->lanes.resize(c.lanes);
-  int r = dalloc(&s->d_totals, 4);
+  int r = dalloc(ctx, &s->d_totals, 4);
   for (Lane& L : s->lanes) {
     L.server = s;
-    if (!r && !c.merged) r = alloc_lane(L, N, c.max_spp, c.max_depth, s->status_stride);
+    if (!r && !c.merged) r = alloc_lane(ctx, L, N, c.max_spp, c.max_depth, s->status_stride);
   }
   if (!r && c.merged) {
     r = alloc_merged(s, N, c.merged, kSets);
-    if (r == MT_ERR_NOMEM) {  // memory is short: no kept scratch, one set of queues per stream
+    if (r == MT_ERR_NOMEM) {  // memory is short: one set of queues per stream
       free_merged(s);
-      drop_workspace(ctx);
       r = alloc_merged(s, N, c.merged, 1);
     }
   }

@@ -254,8 +254,8 @@ int refresh_wide(mt_scene* s) {
     return fail(MT_ERR_DEPTH, "wide BVH depth %d exceeds the traversal's %d groups", b.max_depth + 1, kWideStack);
   if ((int)(b.wt.size() / 3) != s->ntri)
     return fail(MT_ERR_INVALID, "wide BVH reaches %zu of %d triangles", b.wt.size() / 3, s->ntri);
-  int r = dalloc(&s->d_wnodes, b.nodes.size());
-  if (!r) r = dalloc(&s->d_wtris, b.wt.size());
+  int r = dalloc(s->ctx, &s->d_wnodes, b.nodes.size());
+  if (!r) r = dalloc(s->ctx, &s->d_wtris, b.wt.size());
   if (r) return r;
   CU(cudaMemcpy(s->d_wnodes, b.nodes.data(), b.nodes.size() * sizeof(uint4), cudaMemcpyHostToDevice));
   CU(cudaMemcpy(s->d_wtris, b.wt.data(), b.wt.size() * sizeof(float4), cudaMemcpyHostToDevice));

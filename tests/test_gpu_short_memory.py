@@ -1,0 +1,193 @@
+"""Calls on a device that is nearly full (MT_DEVICE_ROOM, which fails the library's own
+allocations; each case in a process of its own): what fits the device is not refused
+because of memory that an earlier call keeps, and gives the results it gives on an empty
+one."""
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+from mambatracer_gb300 import api, layout, scenes
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CASES = {}
+
+
+def case(f):
+    CASES[f.__name__] = f
+    return f
+
+
+def _room(n):
+    """The library's arrays may grow by n bytes from here on (None: by any number)."""
+    _room.calls += 1
+    os.environ["MT_DEVICE_ROOM"] = "" if n is None else f"{n}" + " " * _room.calls
+
+
+_room.calls = 0
+
+
+def _rays(sc, n):
+    o, d = scenes.random_rays(sc, n, seed=n)
+    return layout.make_rays(o, d)
+
+
+def _soup(n=20000):
+    sc = scenes.soup(n, seed=4, extent=0.8, edge_sigma=0.05, width=320, height=240)
+    return sc
+
+
+def _scene(ctx, sc):
+    S = api.Scene(ctx, sc)
+    S.build_bvh_device(want_arrays=False)
+    return S
+
+
+def _film(ctx, S, cam, **kw):
+    J = api.Job(ctx, S, 320, 240, **{**dict(max_depth=4, mode=1, rr_depth=3), **kw})
+    J.set_camera(cam)
+    for f in range(3):
+        J.render(None, float(1 + f * kw.get("spp", 1)))
+    film = J.film()
+    J.close()
+    return film
+
+
+# ---------------------------------------------------------------- the kept scratch
+def _beside_scratch(op, keep=400_000):
+    """op(ctx, S, sc) with no room but the scratch that a query of `keep` rays left (88 bytes
+    a ray), against op with room."""
+    ctx = api.Context(0)
+    sc = _soup()
+    S = _scene(ctx, sc)
+    rays = _rays(sc, keep)
+    want = op(ctx, S, sc)
+    S.trace_closest(rays)
+    _room(0)
+    got = op(ctx, S, sc)
+    _room(None)
+    for a, b in zip(want, got):
+        assert np.asarray(a).tobytes() == np.asarray(b).tobytes()
+    S.close()
+    ctx.close()
+
+
+@case
+def scene_beside_scratch():
+    big = _soup(100_000)  # 8.8 MB of mesh
+
+    def op(ctx, S, sc):
+        T = api.Scene(ctx, big)
+        n = T.light_count
+        T.close()
+        return [n]
+    _beside_scratch(op)
+
+
+@case
+def tree_beside_scratch():
+    big = _soup(100_000)  # 11.2 MB of tree, 7 MB while it is built
+    keep = {}
+
+    def op(ctx, S, sc):
+        T = keep.setdefault("T", None) or api.Scene(ctx, big)
+        keep["T"] = T
+        T.build_bvh_device(want_arrays=False)
+        return [T.trace_closest(_rays(sc, 1000))[0]]
+    _beside_scratch(op)
+
+@case
+def environment_beside_scratch():
+    maps = [(scenes.sky_env(w, w // 2), w, w // 2) for w in (256, 512)]  # 5 MB of map and tables the larger
+
+    def op(ctx, S, sc):
+        out = []
+        for m in maps:
+            S.set_env(*m)
+            out += S.env_arrays(*m[1:])
+        return out
+    _beside_scratch(op)
+
+
+@case
+def texture_beside_scratch():
+    img = np.arange(1 << 20, dtype=np.int32).reshape(1024, 1024)
+
+    def op(ctx, S, sc):
+        S.set_texture(0, 0, img)
+        S.set_texture(0, 0, None)
+        return []
+    _beside_scratch(op)
+
+
+@case
+def formats_beside_scratch():
+    def op(ctx, S, sc):
+        out = []
+        for p in (1, 2, 0):
+            S.set_precision(p)
+            out.append(S.trace_any(_rays(sc, 1000)))
+        return out
+    _beside_scratch(op)
+
+
+@case
+def image_beside_scratch():
+    jobs = []
+
+    def op(ctx, S, sc):
+        J = jobs.pop() if jobs else None
+        if J is None:
+            jobs.append(api.Job(ctx, S, 320, 240, max_depth=3, mode=1))  # its image is allocated by the next call
+            J = api.Job(ctx, S, 320, 240, max_depth=3, mode=1)
+        J.set_camera(sc.camera)
+        J.render(None, 1.0)
+        argb, la = J.image()
+        J.close()
+        return [argb]
+    _beside_scratch(op)
+
+
+@case
+def lanes_beside_scratch():
+    def op(ctx, S, sc):
+        srv = api.Server(ctx, lanes=1, max_width=320, max_height=240, max_spp=1, max_depth=4, merged=0)
+        rid = srv.submit(S, sc.camera, 320, 240, 1)
+        film = srv.wait(rid).copy()
+        srv.close()
+        return [film]
+    _beside_scratch(op)
+
+
+@case
+def job_beside_scratch():
+    # 22 MB a pass with its log and four of those side by side; one pass alone takes 15 MB
+    _beside_scratch(lambda ctx, S, sc: [_film(ctx, S, sc.camera)])
+
+
+@case
+def own_allocation_beside_scratch():
+    """A query above what is kept (2 GiB) beside a kept scratch of nearly that."""
+    ctx = api.Context(0)
+    sc = _soup(200)
+    S = _scene(ctx, sc)
+    rays = np.tile(_rays(sc, 1 << 16), 400)
+    S.trace_any(rays[:24_000_000])
+    _room(200 << 20)
+    occ = S.trace_any(rays[:25_000_000])
+    _room(None)
+    assert np.array_equal(occ[:1 << 16], occ[1 << 16:1 << 17])
+    S.close()
+    ctx.close()
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_short_memory(name):
+    code = f"import sys; sys.path.insert(0, {ROOT!r}); import tests.test_gpu_short_memory as m; m.CASES[{name!r}]()"
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, MT_DEVICE_ROOM=""), timeout=300, cwd=ROOT,
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-2000:]

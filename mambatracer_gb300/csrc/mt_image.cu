@@ -175,7 +175,13 @@ int ensure_image(mt_job* j) {
   if (!r) r = dalloc(j->ctx, &j->d_tone_part, (size_t)nparts);
   if (!r) r = dalloc(j->ctx, &j->d_tone_cnt, (size_t)nparts);
   if (!r) r = dalloc(j->ctx, &j->d_tone_tot, 3);  // total, count, blocks that have ended
-  if (r) return r;
+  if (r) {  // all of them or none: the next call looks at d_argb alone
+    dfree(j->d_argb);
+    dfree(j->d_fb);
+    dfree(j->d_tone_part);
+    dfree(j->d_tone_cnt);
+    return r;
+  }
   CU(cudaMemsetAsync(j->d_tone_tot, 0, 12, j->ctx->stream));
   k_argb_fill<<<(unsigned)((N + 255) / 256), 256, 0, j->ctx->stream>>>(j->d_argb, N);
   CU(cudaGetLastError());

@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 
 from mambatracer_gb300 import api, layout, scenes
+from mambatracer_gb300._lib import MTError
 
 pytestmark = pytest.mark.gpu
 
@@ -183,6 +184,30 @@ def own_allocation_beside_scratch():
     assert np.array_equal(occ[:1 << 16], occ[1 << 16:1 << 17])
     S.close()
     ctx.close()
+
+
+# ------------------------------------------------------- allocations that fail half-way
+@case
+def image_arrays_in_part():
+    """An image whose first arrays fit and whose later ones do not: refused each time it is asked
+    for, and there once it fits."""
+    ctx = api.Context(0)
+    sc = _soup()
+    S = _scene(ctx, sc)
+    jobs = [api.Job(ctx, S, 1280, 960, max_depth=3, mode=1) for _ in range(2)]
+    for J in jobs:
+        J.set_camera(sc.camera)
+        J.render(None, 1.0)
+    # the image takes 4.9 MB, the averaged film after it 19.7 MB; the scratch given back for them 2 MB
+    for room in (0, 6_400_000, 6_400_000, 22_000_000):
+        _room(room)
+        for _ in range(2):
+            with pytest.raises(MTError, match="NOMEM"):
+                jobs[0].image()
+    _room(None)
+    assert np.array_equal(jobs[0].image()[0], jobs[1].image()[0])
+    for o in (*jobs, S, ctx):
+        o.close()
 
 
 @pytest.mark.parametrize("name", sorted(CASES))

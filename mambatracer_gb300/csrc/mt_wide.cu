@@ -256,9 +256,15 @@ int refresh_wide(mt_scene* s) {
     return fail(MT_ERR_INVALID, "wide BVH reaches %zu of %d triangles", b.wt.size() / 3, s->ntri);
   int r = dalloc(s->ctx, &s->d_wnodes, b.nodes.size());
   if (!r) r = dalloc(s->ctx, &s->d_wtris, b.wt.size());
-  if (r) return r;
-  CU(cudaMemcpy(s->d_wnodes, b.nodes.data(), b.nodes.size() * sizeof(uint4), cudaMemcpyHostToDevice));
-  CU(cudaMemcpy(s->d_wtris, b.wt.data(), b.wt.size() * sizeof(float4), cudaMemcpyHostToDevice));
+  if (!r && (cudaMemcpy(s->d_wnodes, b.nodes.data(), b.nodes.size() * sizeof(uint4), cudaMemcpyHostToDevice) !=
+                 cudaSuccess ||
+             cudaMemcpy(s->d_wtris, b.wt.data(), b.wt.size() * sizeof(float4), cudaMemcpyHostToDevice) != cudaSuccess))
+    r = fail(MT_ERR_CUDA, "wide BVH: %s", cudaGetErrorString(cudaGetLastError()));
+  if (r) {  // nodes without triangles are not traversed: the FP32 records are
+    dfree(s->d_wnodes);
+    dfree(s->d_wtris);
+    return r;
+  }
   s->nwide = (int)(b.nodes.size() / kWideWords);
   s->wdepth = b.max_depth + 1;
   return MT_OK;

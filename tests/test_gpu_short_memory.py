@@ -210,6 +210,35 @@ def image_arrays_in_part():
         o.close()
 
 
+@case
+def formats_in_part():
+    """A format whose arrays do not all fit is refused, and the scene renders from its FP32
+    records meanwhile, whatever has been made of the format."""
+    ctx = api.Context(0)
+    sc = _soup()
+    S = _scene(ctx, sc)
+    rays = _rays(sc, 5000)
+    want = S.trace_any(rays)
+    refused = 0
+    for p in (2, 1):
+        for room in range(0, 2_400_000, 300_000):
+            S.set_precision(0)
+            _room(0)
+            with pytest.raises(MTError, match="NOMEM"):  # the scratch kept so far goes
+                api.Scene(ctx, sc)
+            _room(room)
+            try:
+                S.set_precision(p)
+            except MTError as e:
+                assert "NOMEM" in str(e)
+                refused += 1
+            _room(None)
+            assert np.array_equal(S.trace_any(rays), want), (p, room)
+    assert refused >= 4
+    S.close()
+    ctx.close()
+
+
 @pytest.mark.parametrize("name", sorted(CASES))
 def test_short_memory(name):
     code = f"import sys; sys.path.insert(0, {ROOT!r}); import tests.test_gpu_short_memory as m; m.CASES[{name!r}]()"

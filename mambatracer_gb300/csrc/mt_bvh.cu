@@ -732,8 +732,15 @@ int refresh_qnodes(mt_scene* s) {
   if (s->precision == 3 && s->has_bvh && s->nrec > 0) {
     Workspace ws;
     float4* sah = nullptr;
-    int r = build_sah_records(s, ws, &sah);
-    if (!r) r = dalloc(&s->d_quad, (sah ? 8 : 4) * (size_t)s->nrec);
+    // nodes over the surface-area tree and over the reference's (the array first, as above);
+    // over the latter alone where that tree would be too deep or memory is short
+    int r = dalloc(s->ctx, &s->d_quad, 8 * (size_t)s->nrec);
+    if (!r) r = build_sah_records(s, ws, &sah);
+    if (r == MT_ERR_NOMEM || (!r && !sah)) {
+      ws.release();
+      dfree(s->d_quad);
+      r = dalloc(s->ctx, &s->d_quad, 4 * (size_t)s->nrec);
+    }
     cudaError_t e = cudaSuccess;
     if (!r) {
       cudaStream_t st = s->ctx->stream;

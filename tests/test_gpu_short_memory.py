@@ -186,6 +186,30 @@ def own_allocation_beside_scratch():
     ctx.close()
 
 
+@case
+def quad_nodes_without_the_surface_area_tree():
+    """4-wide nodes where only those over the reference's tree fit (64 bytes a triangle): made, as
+    they were before that tree was built for them, and the same answers."""
+    ctx = api.Context(0)
+    sc = _soup()
+    S = _scene(ctx, sc)
+    rays = _rays(sc, 20_000)
+    t0, p0 = S.trace_closest(rays)
+    a0 = S.trace_any(rays)
+    for room in (1_300_000, 2_600_000, 4_000_000, None):
+        S.set_precision(0)
+        _room(0)
+        with pytest.raises(MTError, match="NOMEM"):  # the scratch kept so far goes
+            api.Scene(ctx, sc)
+        _room(room)
+        S.set_precision(3)
+        _room(None)
+        t, p = S.trace_closest(rays)
+        assert np.array_equal(t, t0) and np.array_equal(p, p0) and np.array_equal(S.trace_any(rays), a0)
+    S.close()
+    ctx.close()
+
+
 # ------------------------------------------------------- allocations that fail half-way
 @case
 def image_arrays_in_part():

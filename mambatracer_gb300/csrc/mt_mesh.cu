@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <climits>
+#include <cstring>
 #include <vector>
 
 #include "mt_internal.h"
@@ -87,6 +88,41 @@ int first_bad_face(mt_scene* s, int nmat, bool mat_only, int* bad) {
   return MT_OK;
 }
 
+namespace {
+// The two calls below without scratch, for a device that has none left: the arrays go
+// through the host.
+int host_light_faces(mt_scene* s, const std::vector<unsigned char>& emits) {
+  std::vector<Face> F((size_t)s->ntri);
+  CU(cudaMemcpy(F.data(), s->d_faces, F.size() * sizeof(Face), cudaMemcpyDeviceToHost));
+  std::vector<int> list;
+  for (int i = 0; i < s->ntri; ++i)
+    if (emits[F[i].mat & 0xFFFF]) list.push_back(i);
+  if (list.empty()) return MT_OK;
+  const int r = dalloc(s->ctx, &s->d_light_faces, list.size());
+  if (r) return r;
+  CU(cudaMemcpy(s->d_light_faces, list.data(), 4 * list.size(), cudaMemcpyHostToDevice));
+  s->nlights = (int)list.size();
+  return MT_OK;
+}
+int host_order_triangles(mt_scene* s, const std::vector<int>& order, float4* tris) {
+  std::vector<Face> F((size_t)s->ntri);
+  std::vector<float4> P((size_t)s->npoints), T(3 * order.size());
+  CU(cudaMemcpy(F.data(), s->d_faces, F.size() * sizeof(Face), cudaMemcpyDeviceToHost));
+  CU(cudaMemcpy(P.data(), s->d_points, P.size() * sizeof(float4), cudaMemcpyDeviceToHost));
+  for (size_t k = 0; k < order.size(); ++k) {
+    const Face& f = F[order[k]];
+    const float4 p1 = P[f.vx], p2 = P[f.vy], p3 = P[f.vz];
+    float id;
+    std::memcpy(&id, &order[k], 4);
+    T[3 * k + 0] = make_float4(p1.x, p1.y, p1.z, id);
+    T[3 * k + 1] = make_float4(p2.x - p1.x, p2.y - p1.y, p2.z - p1.z, 0.f);
+    T[3 * k + 2] = make_float4(p3.x - p1.x, p3.y - p1.y, p3.z - p1.z, 0.f);
+  }
+  CU(cudaMemcpy(tris, T.data(), T.size() * sizeof(float4), cudaMemcpyHostToDevice));
+  return MT_OK;
+}
+}  // namespace
+
 // identifyMeshLights + prefix scan + prepareLightInfo (CLightConfiguration.java:43-87).
 int list_light_faces(mt_scene* s, const std::vector<unsigned char>& emits) {
   mt_context* ctx = s->ctx;
@@ -99,6 +135,7 @@ int list_light_faces(mt_scene* s, const std::vector<unsigned char>& emits) {
   Workspace ws;
   int r = ws.get(ctx, Workspace::round(emits.size()) + Workspace::round(4 * (size_t)s->ntri) + Workspace::round(8 * tiles) +
                           Workspace::round(16));
+  if (r == MT_ERR_NOMEM) return host_light_faces(s, emits);
   if (r) return r;
   unsigned char* d_emits = ws.take<unsigned char>(emits.size());
   int* list = ws.take<int>((size_t)s->ntri);
@@ -126,13 +163,15 @@ int list_light_faces(mt_scene* s, const std::vector<unsigned char>& emits) {
     if (!r) s->nlights = h[1];
   }
   ws.release();
-  return r;
+  // the list's own array may need the kept scratch's bytes
+  return r == MT_ERR_NOMEM ? host_light_faces(s, emits) : r;
 }
 
 int order_triangles(mt_scene* s, const std::vector<int>& order, float4* tris) {
   mt_context* ctx = s->ctx;
   Workspace ws;
   int r = ws.get(ctx, Workspace::round(4 * order.size()));
+  if (r == MT_ERR_NOMEM) return host_order_triangles(s, order, tris);
   if (r) return r;
   int* d = ws.take<int>(order.size());
   cudaError_t e = cudaMemcpyAsync(d, order.data(), 4 * order.size(), cudaMemcpyHostToDevice, ctx->stream);

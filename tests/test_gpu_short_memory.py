@@ -210,6 +210,45 @@ def quad_nodes_without_the_surface_area_tree():
     ctx.close()
 
 
+@case
+def mesh_without_scratch():
+    """A mesh with lights and an imported tree where just their own arrays fit (88 bytes a triangle
+    and the light list; 112 bytes a triangle): made without scratch, with the same contents."""
+    ctx = api.Context(0)
+    sc = _soup()
+    sc.materials = np.concatenate([sc.materials, sc.materials[:1]])
+    sc.materials["emission_param"][-1] = 2.0
+    sc.materials["emission_color"][-1] = 1.0
+    rng = np.random.default_rng(1)
+    lit = rng.random(sc.ntri) < 0.3
+    sc.faces["mat"] = np.where(lit, len(sc.materials) - 1, 0)
+    nodes, bounds, _ = api.bvh_build_host(sc)
+    S = api.Scene(ctx, sc)
+    S.import_bvh(nodes, bounds)
+    assert S.light_count == lit.sum()
+    film = _film(ctx, S, sc.camera)
+    for extra in (0, 100_000):  # bytes beyond the arrays: none, and less than any scratch that is kept
+        _room(0)
+        with pytest.raises(MTError, match="NOMEM"):  # the scratch kept so far goes
+            api.Scene(ctx, sc)
+        mesh = -(-sc.points.nbytes // 256) * 256 + 512 + 40 * sc.ntri
+        _room(mesh + sc.materials.nbytes + 4 * int(lit.sum()) + extra)
+        T = api.Scene(ctx, sc)
+        assert T.light_count == lit.sum()
+        _room(0)
+        with pytest.raises(MTError, match="NOMEM"):
+            api.Scene(ctx, sc)
+        _room(64 * (sc.ntri - 1) + 48 * sc.ntri + extra)
+        T.import_bvh(nodes, bounds)
+        _room(None)
+        for a, b in zip(T.layout()[:2], S.layout()[:2]):
+            assert a.tobytes() == b.tobytes()
+        assert _film(ctx, T, sc.camera).tobytes() == film.tobytes()
+        T.close()
+    S.close()
+    ctx.close()
+
+
 # ------------------------------------------------------- allocations that fail half-way
 @case
 def image_arrays_in_part():

@@ -755,11 +755,31 @@ int import_bvh(mt_scene* s, const int32_t* nodes, const float* bounds, int nnode
     r[3] = make_float4(lf, rf, 0.f, 0.f);
   }
   if ((int)order.size() != n) return fail(MT_ERR_INVALID, "BVH reaches %zu of %d triangles", order.size(), n);
-  int r = upload(s->ctx, &s->d_nodes, hn.data(), hn.size());
-  dfree(s->d_tris);
-  if (!r) r = dalloc(s->ctx, &s->d_tris, 3 * (size_t)n);
-  if (!r) r = order_triangles(s, order, s->d_tris);
+  // The new tree beside the old one, which stays when this fails, or, where both do not
+  // fit, in its place.
+  float4 *recs = nullptr, *tris = nullptr;
+  auto make = [&] {
+    int r = upload(s->ctx, &recs, hn.data(), hn.size());
+    if (!r) r = dalloc(s->ctx, &tris, 3 * (size_t)n);
+    if (!r) r = order_triangles(s, order, tris);
+    if (r) {
+      dfree(recs);
+      dfree(tris);
+    }
+    return r;
+  };
+  int r = make();
+  if (r == MT_ERR_NOMEM && s->has_bvh) {
+    s->has_bvh = 0;  // until the new one is there, nothing is rendered
+    dfree(s->d_nodes);
+    dfree(s->d_tris);
+    r = make();
+  }
   if (r) return r;
+  dfree(s->d_nodes);
+  dfree(s->d_tris);
+  s->d_nodes = recs;
+  s->d_tris = tris;
   s->nrec = nrec;
   s->root_ref = root[5] ? ~0 : 0;
   s->depth = max_level;

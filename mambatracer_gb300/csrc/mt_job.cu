@@ -501,6 +501,7 @@ extern "C" int mt_render_frame(mt_job* j, const int32_t* seeds, float frame_coun
   mt_context* ctx = j->ctx;
   std::lock_guard<std::recursive_mutex> lk(ctx->mu);
   CU(cudaSetDevice(ctx->device));
+  if (!j->scene->has_bvh) return fail(MT_ERR_INVALID, "scene has no BVH (mt_bvh_build / mt_bvh_import)");
   if (j->scene_version != j->scene->version) {
     // The scene's arrays or grid configuration changed (the change waited for
     // every frame): recapture the graphs and set the light grid up again.

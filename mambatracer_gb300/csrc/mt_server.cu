@@ -255,6 +255,7 @@ int alloc_lane(mt_context* ctx, Lane& L, size_t N, int spp, int depth, size_t st
 // Enqueues request R on lane L (scheduler thread, context lock held).
 int start_request(mt_server* s, Lane& L, Request* R) {
   const mt_server_config& c = s->cfg;
+  if (!R->scene->has_bvh) return fail(MT_ERR_INVALID, "scene has no BVH");
   const size_t N = (size_t)R->width * R->height;
   for (int p = 0; p < R->spp; ++p) {
     PassParams& pp = L.h_pp[p];
@@ -492,6 +493,7 @@ int issue_round(mt_server* s, MergeGroup& G, const std::vector<int>& work, const
     // applied to the stream's executable graph of that scene by an update (the
     // same kernels every round), instantiated again only when an update fails.
     const Group& Gr = groups[g];
+    if (!Gr.scene->has_bvh) return fail(MT_ERR_INVALID, "scene has no BVH");
     const DevScene S = Gr.scene->view();
     const DevEnv E = Gr.scene->env_view();  // full-map environment sampling
     CU(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));

@@ -302,6 +302,53 @@ def formats_in_part():
     ctx.close()
 
 
+@case
+def import_in_part():
+    """An import beside a tree: in its place where both do not fit. Where no tree fits, the scene
+    stays without one: queries are refused, and an import works once there is room. A failed
+    import of one that is not a tree leaves the old one."""
+    ctx = api.Context(0)
+    sc = _soup()
+    nodes, bounds, _ = api.bvh_build_host(sc)
+    rays = _rays(sc, 5000)
+    S = api.Scene(ctx, sc)
+    for room in (0, 1_000_000, 1_400_000, 2_200_000):  # records 1.28 MB, triangles 0.96 MB
+        _room(0)
+        with pytest.raises(MTError, match="NOMEM"):
+            api.Scene(ctx, sc)
+        _room(room)
+        with pytest.raises(MTError, match="NOMEM"):
+            S.import_bvh(nodes, bounds)
+        _room(None)
+        with pytest.raises(MTError, match="no BVH"):
+            S.trace_any(rays)
+    S.import_bvh(nodes, bounds)
+    t, p = S.trace_closest(rays)
+    film = _film(ctx, S, sc.camera)
+    J = api.Job(ctx, S, 320, 240, max_depth=4, mode=1, rr_depth=3)
+    J.set_camera(sc.camera)
+    for room in (0, 1_000_000, 1_400_000, 2_200_000, 3_000_000):
+        _room(0)
+        with pytest.raises(MTError, match="NOMEM"):
+            api.Scene(ctx, sc)
+        _room(room)
+        S.import_bvh(nodes, bounds)
+        _room(None)
+        t1, p1 = S.trace_closest(rays)
+        assert np.array_equal(t1, t) and np.array_equal(p1, p)
+        J.clear()
+        for f in range(3):
+            J.render(None, float(1 + f))
+        assert J.film().tobytes() == film.tobytes()
+    bad = nodes.copy()
+    bad.reshape(-1, 7)[0, 2] = len(bad.reshape(-1, 7))
+    with pytest.raises(MTError, match="child"):
+        S.import_bvh(bad, bounds)
+    assert np.array_equal(S.trace_closest(rays)[0], t)
+    for o in (J, S, ctx):
+        o.close()
+
+
 @pytest.mark.parametrize("name", sorted(CASES))
 def test_short_memory(name):
     code = f"import sys; sys.path.insert(0, {ROOT!r}); import tests.test_gpu_short_memory as m; m.CASES[{name!r}]()"

@@ -703,6 +703,14 @@ __global__ void k_resolve(const float4* __restrict__ film, size_t n, float frame
   out[i] = make_float4(a.x / frames, a.y / frames, a.z / frames, 1.f);
 }
 
+// The same on the host, where the device has no room for the divided film.
+void resolve_on_host(float* rgba, size_t n, float frames) {
+  for (size_t i = 0; i < n; ++i) {
+    for (int k = 0; k < 3; ++k) rgba[4 * i + k] = rgba[4 * i + k] / frames;
+    rgba[4 * i + 3] = 1.f;
+  }
+}
+
 // Completes the oldest pending read: waits for its copy.
 int finish_oldest_read(mt_job* j) {
   mt_job::Read& rd = j->reads[j->r_head];
@@ -731,10 +739,12 @@ int enqueue_read(mt_job* j, float* rgba, int resolve, mt_job::Read** out) {
   mt_context* ctx = j->ctx;
   mt_job::Read& rd = j->reads[(j->r_head + j->r_count) % mt_job::kMaxReads];
   const size_t N = (size_t)j->cfg.width * j->cfg.height;
-  const bool divide = resolve && j->frames > 0;
+  bool divide = resolve && j->frames > 0, divide_host = false;
   if (divide && !j->d_resolved) {
-    int r = dalloc(ctx, &j->d_resolved, N);
-    if (r) return r;
+    const int r = dalloc(ctx, &j->d_resolved, N);
+    if (r && r != MT_ERR_NOMEM) return r;
+    divide_host = r == MT_ERR_NOMEM;
+    divide = !divide_host;
   }
   CU(cudaEventRecord(j->rfork, ctx->stream));
   CU(cudaStreamWaitEvent(j->rstream, j->rfork, 0));
@@ -750,6 +760,11 @@ int enqueue_read(mt_job* j, float* rgba, int resolve, mt_job::Read** out) {
   rd.host = rgba;
   ++j->r_count;
   *out = &rd;
+  if (divide_host) {  // now: a later read may be given the same buffer
+    const int r = finish_reads(j);
+    if (r) return r;
+    resolve_on_host(rgba, N, (float)j->frames);
+  }
   return MT_OK;
 }
 }  // namespace

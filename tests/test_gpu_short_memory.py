@@ -249,6 +249,37 @@ def mesh_without_scratch():
     ctx.close()
 
 
+@case
+def resolved_read_without_room():
+    """Resolved reads of a film, waited for and enqueued (the same buffer twice), where the divided
+    film has no room on the device: the values of a job that has it."""
+    ctx = api.Context(0)
+    sc = _soup(2000)
+    S = _scene(ctx, sc)
+    got = []
+    for room in (None, 3_000_000):  # the film is 4.9 MB, the scratch of the build less than 2
+        J = api.Job(ctx, S, 640, 480, max_depth=3, mode=1)
+        J.set_camera(sc.camera)
+        out = [np.empty((640 * 480, 4), np.float32) for _ in range(3)]
+        J.render(None, 1.0)
+        _room(room)
+        J.film_async(out[0], resolve=True)
+        J.render(None, 2.0)
+        J.film_async(out[1], resolve=True)
+        J.render(None, 3.0)
+        J.film_async(out[1], resolve=True)
+        J.wait()
+        out[2][:] = J.film(resolve=True)
+        _room(None)
+        got.append(out + [J.film()])
+        J.close()
+    for a, b in zip(*got):
+        assert a.tobytes() == b.tobytes()
+    assert np.array_equal(got[0][1][:, :3], got[0][3][:, :3] / np.float32(3))
+    S.close()
+    ctx.close()
+
+
 # ------------------------------------------------------- allocations that fail half-way
 @case
 def image_arrays_in_part():

@@ -81,6 +81,17 @@ __attribute__((visibility("hidden"))) void device_free(void* p) {
   }
   cudaFree(p);
 }
+__attribute__((visibility("hidden"))) size_t device_left() {
+  size_t free = 0, total = 0;
+  if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  DeviceRoom& r = device_room();
+  if (!r.on) return free;
+  std::lock_guard<std::mutex> lk(r.mu);
+  return std::min(free, r.left());
+}
 }  // namespace mt
 
 int quiesce(mt_context* ctx) {
@@ -132,6 +143,10 @@ bool drop_workspace(mt_context* c) {
   dfree(c->ws);
   c->ws_bytes = 0;
   return true;
+}
+
+size_t overlap_bytes(mt_context* c, size_t most) {
+  return std::min(most, (device_left() + (c->ws_used ? 0 : c->ws_bytes)) / 4);
 }
 
 void prefault(void* p, size_t bytes, cudaEvent_t ready) {

@@ -30,6 +30,7 @@ __attribute__((visibility("hidden"))) int fail(int code, const char* fmt, ...);
 // first seen (empty: no limit; the value may change while the process runs).
 __attribute__((visibility("hidden"))) cudaError_t device_malloc(void** p, size_t bytes);
 __attribute__((visibility("hidden"))) void device_free(void* p);
+__attribute__((visibility("hidden"))) size_t device_left();  // bytes that further arrays can take
 }  // namespace mt
 using mt::fail;
 
@@ -310,6 +311,12 @@ struct Workspace {
 // until `ready` has happened: a fresh buffer's pages are then mapped while the GPU
 // still works, not one fault after the other during the copy (33 MB: 2 ms).
 void prefault(void* p, size_t bytes, cudaEvent_t ready);
+
+// What the path state of passes that run side by side may take of the device: `most`
+// bytes, and a quarter of what is left (the scratch kept between calls, which is given back
+// where it is needed, counts as left), so that what a program makes next still fits
+// where it did without them. The context lock held.
+size_t overlap_bytes(mt_context* c, size_t most);
 
 constexpr int kOpaqueBlack = (int)0xFF000000u;  // getIntARGB((0, 0, 0, 1))
 

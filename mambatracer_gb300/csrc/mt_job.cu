@@ -75,7 +75,7 @@ namespace {
 // submitted: 8.8 ms with two at once, 7.7 with four).
 constexpr int kOverlap = 4;
 constexpr int kOverlapMerged = 8;
-constexpr size_t kOverlapBytes = 8ull << 30;  // the memory their buffers may take
+constexpr size_t kOverlapBytes = 8ull << 30;  // the memory their buffers may take (overlap_bytes)
 
 // Adds one frame's film (rendered from zero into its slot's film) into the
 // job's film. With Kahan adds on, the slot film's value is film - film_c and
@@ -336,7 +336,7 @@ extern "C" int mt_job_create(mt_context* ctx, mt_scene* scene, const mt_render_c
   // How many passes overlap, shared out over the caller's frames in flight; without
   // those, over the passes of a frame first and then over frames.
   const int frames = (cfg->profile || cfg->inflight < 1) ? 1 : cfg->inflight;
-  const size_t fit = kOverlapBytes / (N * pass_bytes(cfg->max_depth));
+  const size_t fit = overlap_bytes(ctx, kOverlapBytes) / (N * pass_bytes(cfg->max_depth));
   const int overlap =
       cfg->profile ? 1 : (int)std::min<size_t>(frames > 1 ? kOverlapMerged : kOverlap, std::max<size_t>(fit, 1));
   j->merge = frames > 1;
@@ -351,6 +351,8 @@ extern "C" int mt_job_create(mt_context* ctx, mt_scene* scene, const mt_render_c
     if (!r) r = dalloc(j->ctx, &j->d_totals, 4);
     if (!r && (j->merge || j->logged)) r = dalloc(j->ctx, &j->d_film, N);
     if (!r && (j->merge || j->logged)) r = dalloc(j->ctx, &j->d_film_c, N);
+    j->scene_version = scene->version;
+    if (!r) r = setup_grid(j);
     if (r != MT_ERR_NOMEM || at_once == 1) break;
     free_job(j);
     r = MT_OK;
@@ -361,10 +363,6 @@ extern "C" int mt_job_create(mt_context* ctx, mt_scene* scene, const mt_render_c
     r = fail(MT_ERR_CUDA, "event create");
   if (!r && cudaEventCreateWithFlags(&j->grid_ev, cudaEventDisableTiming) != cudaSuccess)
     r = fail(MT_ERR_CUDA, "event create");
-  if (!r) {
-    j->scene_version = scene->version;
-    r = setup_grid(j);
-  }
   for (auto& rd : j->reads)
     if (!r && cudaEventCreateWithFlags(&rd.ev, cudaEventDisableTiming) != cudaSuccess)
       r = fail(MT_ERR_CUDA, "event create");

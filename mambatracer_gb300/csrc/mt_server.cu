@@ -348,7 +348,8 @@ int alloc_merged(mt_server* s, size_t N, int m, int nsets) {
   // sets of queues per stream: bytes a path of one set, and of a log
   auto R = Workspace::round;
   const size_t queue_bytes = 9 * 16 + 12, log_bytes = 32 * (size_t)s->cfg.max_depth + 4;
-  while (nsets > 1 && P * ((nsets - 1) * queue_bytes + nsets * log_bytes) > kSetBytes) --nsets;
+  const size_t most = overlap_bytes(s->ctx, kSetBytes);
+  while (nsets > 1 && P * ((nsets - 1) * queue_bytes + nsets * log_bytes) > most) --nsets;
   size_t base = 0;  // first path of the group's share
   for (MergeGroup& G : s->groups) {
     G.server = s;

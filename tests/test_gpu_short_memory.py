@@ -2,6 +2,7 @@
 allocations; each case in a process of its own): what fits the device is not refused
 because of memory that an earlier call keeps, and gives the results it gives on an empty
 one."""
+import ctypes as C
 import os
 import subprocess
 import sys
@@ -10,7 +11,7 @@ import numpy as np
 import pytest
 
 from mambatracer_gb300 import api, layout, scenes
-from mambatracer_gb300._lib import MTError
+from mambatracer_gb300._lib import MTError, check, lib
 
 pytestmark = pytest.mark.gpu
 
@@ -278,6 +279,52 @@ def resolved_read_without_room():
     assert np.array_equal(got[0][1][:, :3], got[0][3][:, :3] / np.float32(3))
     S.close()
     ctx.close()
+
+
+# ------------------------------------------------ path state of overlapping passes
+def _leaves_room(make, needs, total):
+    """make(ctx, S, cam), which needs `needs` bytes of its own arrays, leaves room for the rest of
+    `total`, and gives what it gives on an empty device."""
+    ctx = api.Context(0)
+    sc = _soup()
+    S = _scene(ctx, sc)
+    S.set_env(scenes.sky_env(256, 128), 256, 128)
+    S.grid_config(160, 160, 16, 32, enable=2)
+    want, close = make(ctx, S, sc.camera)
+    close()
+    _room(total)
+    got, close = make(ctx, S, sc.camera)
+    b = C.c_void_p()
+    check(lib().mt_buf_alloc(ctx.h, total - needs, C.byref(b)))  # raises where the room is gone
+    check(lib().mt_buf_free(b))
+    _room(None)
+    close()
+    for a, b in zip(want, got):
+        assert a.tobytes() == b.tobytes()
+    S.close()
+    ctx.close()
+
+
+@case
+def job_leaves_room():
+    # 304 bytes a pixel and pass with its log (depth 4) would be 93 MB for four at once; 192 with
+    # films alone, 15 MB
+    def make(ctx, S, cam):
+        J = api.Job(ctx, S, 320, 240, max_depth=4, mode=1, rr_depth=3, spp=4, grid_updates=0)
+        J.set_camera(cam)
+        J.render(None, 1.0)
+        return [J.film()], J.close
+    _leaves_room(make, 20_000_000, 100_000_000)
+
+
+@case
+def server_leaves_room():
+    # two slots: 31 MB of queues and films; 2 x 24 MB of queues more and 3 x 20 MB of logs for three sets
+    def make(ctx, S, cam):
+        srv = api.Server(ctx, lanes=2, max_width=320, max_height=240, max_spp=3, max_depth=4, merged=1)
+        films = [srv.wait(srv.submit(S, cam, 320, 240, 3)).copy() for _ in range(2)]
+        return films, srv.close
+    _leaves_room(make, 36_000_000, 150_000_000)
 
 
 # ------------------------------------------------------- allocations that fail half-way

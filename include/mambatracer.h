@@ -256,7 +256,12 @@ int mt_job_stats(mt_job* job, int64_t* rays3, int32_t* counts);
 /* Rays traced since the job was created or its film cleared: [primary,
  * extension, shadow], counted on the device. */
 int mt_job_total_rays(mt_job* job, int64_t* rays3);
-/* Device time of the last mt_render_frame, in ms (CUDA events on the job's stream). */
+/* Device time of the last mt_render_frame, in ms (CUDA events on the job's stream): from the
+ * start of its passes until they are in the film (with frames in flight: in the frame's own
+ * film, before it is added to the job's). Frames submitted without waiting in between
+ * run side by side and are added in order, so this is then a span that includes the
+ * others' share of the GPU; a frame submitted after the one before has ended has it
+ * to itself. */
 int mt_job_last_ms(mt_job* job, float* ms);
 /* Kernels the job's frames have launched (graph nodes included): per pass the
  * ray generation, per bounce the closest-hit traversal, shading (one launch or

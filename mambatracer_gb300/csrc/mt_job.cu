@@ -583,6 +583,13 @@ extern "C" int mt_render_frame(mt_job* j, const int32_t* seeds, float frame_coun
     j->launches += (int64_t)c.spp * (2 + (int64_t)c.max_depth * (3 + two)) + (j->merge ? 1 : 0);
     if (j->logged && !replay_inside(j)) j->launches -= c.spp - 1;  // all its passes in one
   }
+  if (j->logged && !replay_inside(j) && !direct) {
+    // the frame into the film, after the frame before it and any film read still copying
+    // the film out
+    if (j->last >= 0) CU(cudaStreamWaitEvent(s.stream, j->slots[j->last].done, 0));
+    CU(cudaStreamWaitEvent(s.stream, j->rdone, 0));
+    if (replay(j, s, s.stream, 0, c.spp)) return fail(MT_ERR_CUDA, "film: %s", cudaGetErrorString(cudaGetLastError()));
+  }
   CU(cudaEventRecord(s.ev1, s.stream));
   if (accumulate) {
     // CAdaptiveEnvironment.update (CAdaptiveEnvironment.java:128-137): func = accum,
@@ -596,17 +603,14 @@ extern "C" int mt_render_frame(mt_job* j, const int32_t* seeds, float frame_coun
     CU(cudaEventRecord(j->grid_ev, s.stream));
     ++j->grid_frames;
   }
-  if (j->nslots > 1) {
+  if (j->merge) {
     // Add the frame into the job's film after the previous frame's add (frame
     // order) and after any film read still copying it out.
     if (j->last >= 0) CU(cudaStreamWaitEvent(s.stream, j->slots[j->last].done, 0));
     CU(cudaStreamWaitEvent(s.stream, j->rdone, 0));
     const size_t N = (size_t)c.width * c.height;
-    if (j->merge)
-      k_film_merge<<<(unsigned)((N + 255) / 256), 256, 0, s.stream>>>(s.film, s.film_c, c.film_kahan, N, j->d_film,
-                                                                      j->d_film_c);
-    else if (!direct)
-      replay(j, s, s.stream, 0, c.spp);
+    k_film_merge<<<(unsigned)((N + 255) / 256), 256, 0, s.stream>>>(s.film, s.film_c, c.film_kahan, N, j->d_film,
+                                                                    j->d_film_c);
     CU(cudaGetLastError());
   }
   CU(cudaEventRecord(s.done, s.stream));

@@ -2,6 +2,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstdlib>
 #include <type_traits>
 
 #include "mt_device.cuh"
@@ -209,7 +210,14 @@ int blocks_per_sm(int minb) {
   return bps[minb];
 }
 
+// MT_LIGHT_KINDS=0 in the environment (read once per process): the general instance of every
+// shading kernel, whatever lights the scene.
 Lights lights_of(const DevScene& S, const DevEnv& E) {
+  static const bool kinds = [] {
+    const char* e = std::getenv("MT_LIGHT_KINDS");
+    return !(e && std::atoi(e) == 0);
+  }();
+  if (!kinds) return kAnyLights;
   if (S.nlights > 0) return E.present ? kAnyLights : kMeshLights;
   if (!E.present) return kAnyLights;
   if (E.grid_on) return E.cell_marg && E.tile_marg ? kGridLights : kAnyLights;

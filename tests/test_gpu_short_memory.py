@@ -327,6 +327,28 @@ def server_leaves_room():
     _leaves_room(make, 36_000_000, 150_000_000)
 
 
+@case
+def batch_with_room_for_one_pass():
+    """A batch whose four passes do not fit side by side: one after the other, the same films."""
+    ctx = api.Context(0)
+    sc = _soup()
+    S = _scene(ctx, sc)
+    frames = [(sc.camera, 320, 240, 4, 1.0), (sc.camera, 200, 100, 2, 9.0)]
+    want, rays = api.batch_render(ctx, S, frames, max_depth=4)  # 97k pixels: 44 MB a pass with its log
+    _room(0)
+    with pytest.raises(MTError, match="NOMEM"):  # the scratch of that batch goes
+        api.Scene(ctx, scenes.soup(4_000_000, seed=1, width=64, height=64))
+    for room in (22_000_000, 60_000_000):
+        _room(room)
+        got, r = api.batch_render(ctx, S, frames, max_depth=4)
+        _room(0)
+        with pytest.raises(MTError, match="NOMEM"):
+            api.batch_render(ctx, S, [(sc.camera, 1920, 1080, 4, 1.0)], max_depth=4)
+        assert np.array_equal(r, rays) and all(a.tobytes() == b.tobytes() for a, b in zip(got, want))
+    S.close()
+    ctx.close()
+
+
 # ------------------------------------------------------- allocations that fail half-way
 @case
 def image_arrays_in_part():

@@ -194,7 +194,8 @@ typedef struct mt_render_config {
   int rr_depth;      /* mode 1: Russian roulette from this bounce on (0 = off) */
   int film_kahan;    /* 1 = compensated film sums (default), 0 = plain FP32 adds as the reference */
   int spp;           /* passes per mt_render_frame call; up to four run side by side, where the path
-                        state for them (160 + 32 max_depth bytes per pixel each) fits 8 GiB */
+                        state for them (160 + 32 max_depth bytes per pixel each) fits 8 GiB and a
+                        quarter of the device memory that is left */
   int use_graph;     /* 1 = replay each frame's launches as a CUDA graph */
   int profile;       /* 1 = time every kernel launch with CUDA events (no graph) */
   int inflight;      /* frames kept in flight on their own streams, 0 or 1 = one (1..8); each
@@ -227,7 +228,8 @@ int mt_film_read(mt_job* job, float* rgba, int resolve);
  * so the next frames can be submitted while this one finishes. Up to eight
  * reads stay pending; a ninth first completes the oldest. rgba must stay valid
  * until its read completes (mt_film_wait, mt_film_read, mt_film_clear, or the
- * ninth read after it); resolve is applied on the device before the copy. No counterpart in the
+ * ninth read after it); resolve is applied on the device before the copy, or, where the
+ * device has no room for the divided film, on the host, and the call then waits. No counterpart in the
  * reference, whose image read (CImage.processImage/readImage) blocks. */
 int mt_film_read_async(mt_job* job, float* rgba, int resolve);
 int mt_film_wait(mt_job* job);
@@ -366,7 +368,8 @@ int mt_trace_closest_dev(mt_scene* scene, mt_buffer* rays, int n, mt_buffer* t_o
  * split over m streams, and each stream issues rounds, a round being one merged
  * pass per scene holding the next pass of every running request of its slots.
  * A request joins at its stream's next round; up to three rounds of a stream
- * overlap, on path state of their own (at most 8 GiB in all beyond the lanes').
+ * overlap, on path state of their own (at most 8 GiB in all beyond the lanes', and a
+ * quarter of the device memory that is left).
  * A cancelled running request
  * stops at the next round (state CANCELLED, no film). Films are the same, bit
  * for bit, in both modes. */

@@ -225,7 +225,6 @@ struct JobSlot {
   cudaEvent_t pfork = nullptr;  // the other buffers' streams start after the frame's set-up
   cudaEvent_t fork = nullptr, ev0 = nullptr, ev1 = nullptr, done = nullptr;
   cudaGraphExec_t graphs[2] = {nullptr, nullptr};  // of a frame among others, and of one alone (logged jobs)
-  bool ran = false;            // a frame has run on this slot (its control blocks hold its counts)
 };
 
 struct mt_job {

@@ -575,7 +575,6 @@ extern "C" int mt_render_frame(mt_job* j, const int32_t* seeds, float frame_coun
     int r = enqueue_frame(j, s, direct);
     if (r) return r;
   }
-  s.ran = true;
   {
     // per pass: raygen, per bounce closest hits + shading (one launch or two) +
     // shadow rays, the ray totals; then the film merge

@@ -42,8 +42,11 @@ struct Replay {
 };
 int launch_replay(cudaStream_t st, const Replay& R, float4* film, float4* film_c, unsigned long long* totals);
 
-// Rays of a short queue kept together in a warp, by how many passes run side by
-// side. Alone, one ray to a warp is fastest (1, 2, 4, 8, 16, 32: the 200k soup at 800 x
+// Rays of a short queue kept together in a warp, by `beside`: the passes or frames that run
+// side by side over a job (the larger of its slots and a slot's buffers) or a batch, a
+// server's lanes or merge streams (the rounds of one stream that overlap, up to three, are
+// not counted: with them, one stream of 1 to 4 requests is 4 to 7 % slower, four streams with 2
+// requests 12 %, with 16 5 % faster, FP32 records). Alone, one ray to a warp is fastest (1, 2, 4, 8, 16, 32: the 200k soup at 800 x
 // 600, passes one by one, 12.2, 12.3, 12.5, 12.7, 13.3, 14.2 ms); with six 1080p frames of
 // the 1M soup in flight the GPU's issue slots are taken and the spread rays'
 // instructions cost (46.8, 46.6, 46.4, 46.1, 45.5, 45.2 ms for eight frames); a served
@@ -104,7 +107,8 @@ void launch_shade_batch(cudaStream_t st, const DevScene& S, const DevEnv& E, con
                         const PassParams* d_pp, int nframes, bool two, int num_sms, int total, Ctrl* ctrl, int b,
                         FrameBufs fb);
 // Whether a pass of n paths shades in two launches (MT_SHADE_SPLIT in the environment:
-// 0 never, 1 always): beside, other passes or frames run beside it. The second
+// 0 never, 1 always): beside, other passes or frames run beside it (on a server: other
+// lanes or merge streams). The second
 // launch's full warps and smaller code gain with the paths; its fixed cost of a few
 // us a bounce matters below a million paths alone and, hidden behind the others,
 // below 2^18 beside others. One launch against two, alone: room 256 x 256, 4 passes,

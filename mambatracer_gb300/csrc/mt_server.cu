@@ -501,7 +501,7 @@ int issue_round(mt_server* s, MergeGroup& G, const std::vector<int>& work, const
     const int lr = launch_batch_pass(st, S, E, Rd.d_tab + Gr.tab, Rd.d_tab + Gr.tab + Gr.n + 1, Rd.d_pp + Gr.pp,
                                      Gr.n, Gr.total, c.max_depth, c.film_kahan, Rd.d_ctrl + g, Q.fb,
                                      s->ctx->num_sms, before ? nullptr : s->d_totals, Q.side, Q.sfork, Q.sjoin,
-                                     (int)s->groups.size());
+                                     (int)s->groups.size());  // streams, not rounds: tail_lanes
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(st, &graph);
     if (lr || e != cudaSuccess) {

@@ -211,10 +211,9 @@ struct PassBuf {
   cudaStream_t side = nullptr;    // shadow rays beside the next bounce's extension rays
   cudaEvent_t sfork = nullptr, sjoin = nullptr, done = nullptr;
 };
-// One in-flight frame's resources: pass buffers, film, parameters, control blocks,
-// and the stream its frames run on.
+// One in-flight frame's resources: pass buffers, film, parameters, control blocks (device
+// arrays in the job's slab), and the stream its frames run on.
 struct JobSlot {
-  char* slab = nullptr;                    // the device arrays below, one allocation
   std::vector<PassBuf> bufs;               // passes of a frame that overlap
   float4 *film = nullptr, *film_c = nullptr;  // the slot's own film (not when passes go to the job's)
   Ctrl* d_ctrl = nullptr;                  // one per pass
@@ -237,6 +236,8 @@ struct mt_job {
   int nslots = 1;
   bool logged = false, merge = false;
   std::vector<JobSlot> slots;
+  char* slab = nullptr;         // the slots' device arrays, the film and the totals, one allocation
+  PassParams* h_pp = nullptr;   // the slots' pinned parameters, one allocation
   int next = 0;   // slot of the next frame
   int last = -1;  // slot of the last frame
   size_t status_stride = 0;

@@ -109,9 +109,6 @@ void free_slot(JobSlot& s) {
     if (B.stream && B.stream != s.stream) cudaStreamDestroy(B.stream);
   }
   s.bufs.clear();
-  dfree(s.slab);
-  if (s.h_pp) cudaFreeHost(s.h_pp);
-  s.h_pp = nullptr;
   for (cudaGraphExec_t& g : s.graphs) {
     if (g) cudaGraphExecDestroy(g);
     g = nullptr;
@@ -127,9 +124,11 @@ void free_slot(JobSlot& s) {
 void free_job(mt_job* j) {
   for (JobSlot& s : j->slots) free_slot(s);
   j->slots.clear();
-  dfree(j->d_totals);
-  dfree(j->d_film);
-  dfree(j->d_film_c);
+  dfree(j->slab);
+  if (j->h_pp) cudaFreeHost(j->h_pp);
+  j->h_pp = nullptr;
+  j->d_totals = nullptr;
+  j->d_film = j->d_film_c = nullptr;
   dfree(j->d_grid_func);
   dfree(j->d_grid_sat);
   dfree(j->d_grid_accum);
@@ -176,62 +175,88 @@ int check_cfg(const mt_render_config* c) {
 // contributions (two a bounce at most).
 size_t pass_bytes(int max_depth) { return 6 * 16 + 8 + 48 + 4 + 4 + 32 * (size_t)max_depth; }
 
-// A slot's device memory is one allocation (an allocation costs 40 us and more, whatever
-// its size up to some MB): sized in a first walk over the arrays, handed out in a second.
-int alloc_slot(mt_context* ctx, JobSlot& s, const mt_render_config& c, int nbuf, bool logged, bool own_film, size_t status_stride) {
-  const size_t N = (size_t)c.width * c.height;
-  int r = MT_OK;
-  if (cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking) != cudaSuccess)
-    r = fail(MT_ERR_CUDA, "stream create");
-  s.bufs.resize(nbuf);
+// A job's device memory is one allocation (an allocation costs 40 us and more, whatever its
+// size up to some MB), and so is its pinned memory: sized in a first walk over the arrays,
+// handed out in a second.
+struct Slab {
+  char* base = nullptr;  // NULL: sizing
   size_t at = 0;
-  auto take = [&](auto** p, size_t count) {
-    if (s.slab) *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(s.slab + at);
-    at += (count * sizeof(**p) + 255) / 256 * 256;
-  };
-  for (int walk = 0; walk < 2 && !r; ++walk) {
-    at = 0;
-    for (PassBuf& B : s.bufs) {
-      for (auto* p : {&B.fb.q_o[0], &B.fb.q_o[1], &B.fb.q_d[0], &B.fb.q_d[1], &B.fb.q_t[0], &B.fb.q_t[1], &B.fb.s_o,
-                      &B.fb.s_d, &B.fb.s_c})
-        take(p, N);
-      take(&B.fb.hit_t, N);
-      take(&B.fb.hit_prim, N);
-      take(&B.fb.live, N);
-      if (logged) {
-        take(&B.fb.log, 2 * (size_t)c.max_depth * N);
-        take(&B.fb.log_n, N);
-        B.fb.log_stride = (int)N;
-      }
-    }
-    if (own_film) {
-      take(&s.film, N);
-      take(&s.film_c, N);
-    }
-    take(&s.d_ctrl, (size_t)c.spp);
-    if (c.mode == 0) take(&s.d_status, status_stride * (size_t)c.max_depth * c.spp);
-    take(&s.d_pp, (size_t)c.spp);
-    if (walk == 0) r = dalloc(ctx, &s.slab, at);
+  template <class T>
+  void take(T** p, size_t count) {
+    if (base) *p = reinterpret_cast<T*>(base + at);
+    at += (count * sizeof(T) + 255) / 256 * 256;
   }
+};
+
+void take_slot(Slab& m, JobSlot& s, const mt_render_config& c, bool logged, bool own_film, size_t status_stride) {
+  const size_t N = (size_t)c.width * c.height;
   for (PassBuf& B : s.bufs) {
-    B.fb.film = s.film;
-    B.fb.film_c = s.film_c;
-    if (&B == &s.bufs[0]) B.stream = s.stream;
-    else if (!r && cudaStreamCreateWithFlags(&B.stream, cudaStreamNonBlocking) != cudaSuccess)
-      r = fail(MT_ERR_CUDA, "stream create");
-    if (!r && cudaStreamCreateWithFlags(&B.side, cudaStreamNonBlocking) != cudaSuccess)
-      r = fail(MT_ERR_CUDA, "stream create");
-    for (cudaEvent_t* e : {&B.sfork, &B.sjoin, &B.done})
-      if (!r && cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess)
-        r = fail(MT_ERR_CUDA, "event create");
+    for (auto* p : {&B.fb.q_o[0], &B.fb.q_o[1], &B.fb.q_d[0], &B.fb.q_d[1], &B.fb.q_t[0], &B.fb.q_t[1], &B.fb.s_o,
+                    &B.fb.s_d, &B.fb.s_c})
+      m.take(p, N);
+    m.take(&B.fb.hit_t, N);
+    m.take(&B.fb.hit_prim, N);
+    m.take(&B.fb.live, N);
+    if (logged) {
+      m.take(&B.fb.log, 2 * (size_t)c.max_depth * N);
+      m.take(&B.fb.log_n, N);
+      B.fb.log_stride = (int)N;
+    }
   }
-  if (!r && cudaMallocHost((void**)&s.h_pp, sizeof(PassParams) * c.spp) != cudaSuccess)
+  if (own_film) {
+    m.take(&s.film, N);
+    m.take(&s.film_c, N);
+  }
+  m.take(&s.d_ctrl, (size_t)c.spp);
+  if (c.mode == 0) m.take(&s.d_status, status_stride * (size_t)c.max_depth * c.spp);
+  m.take(&s.d_pp, (size_t)c.spp);
+}
+
+int alloc_slots(mt_job* j, int nbuf) {
+  const mt_render_config& c = j->cfg;
+  const size_t N = (size_t)c.width * c.height;
+  const bool own_film = j->merge || !j->logged, job_film = j->merge || j->logged;
+  for (JobSlot& s : j->slots) s.bufs.resize(nbuf);
+  int r = MT_OK;
+  for (int walk = 0; walk < 2 && !r; ++walk) {
+    Slab m;
+    m.base = j->slab;
+    for (JobSlot& s : j->slots) take_slot(m, s, c, j->logged, own_film, j->status_stride);
+    m.take(&j->d_totals, 4);
+    if (job_film) {
+      m.take(&j->d_film, N);
+      m.take(&j->d_film_c, N);
+    }
+    if (walk == 0) r = dalloc(j->ctx, &j->slab, m.at);
+  }
+  const size_t pp_bytes = sizeof(PassParams) * c.spp * j->slots.size();
+  if (!r && cudaMallocHost((void**)&j->h_pp, pp_bytes) != cudaSuccess) {
+    cudaGetLastError();
+    j->h_pp = nullptr;
     r = fail(MT_ERR_NOMEM, "pinned pass parameters");
-  for (cudaEvent_t* e : {&s.fork, &s.ev0, &s.ev1, &s.done})
-    if (!r && cudaEventCreate(e) != cudaSuccess) r = fail(MT_ERR_CUDA, "event create");
-  if (!r && cudaEventCreateWithFlags(&s.pfork, cudaEventDisableTiming) != cudaSuccess)
-    r = fail(MT_ERR_CUDA, "event create");
-  if (!r) std::memset(s.h_pp, 0, sizeof(PassParams) * c.spp);
+  }
+  if (!r) std::memset(j->h_pp, 0, pp_bytes);
+  for (JobSlot& s : j->slots) {
+    if (j->h_pp) s.h_pp = j->h_pp + (size_t)c.spp * (&s - j->slots.data());
+    if (!r && cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking) != cudaSuccess)
+      r = fail(MT_ERR_CUDA, "stream create");
+    for (PassBuf& B : s.bufs) {
+      B.fb.film = s.film;
+      B.fb.film_c = s.film_c;
+      if (&B == &s.bufs[0]) B.stream = s.stream;
+      else if (!r && cudaStreamCreateWithFlags(&B.stream, cudaStreamNonBlocking) != cudaSuccess)
+        r = fail(MT_ERR_CUDA, "stream create");
+      if (!r && cudaStreamCreateWithFlags(&B.side, cudaStreamNonBlocking) != cudaSuccess)
+        r = fail(MT_ERR_CUDA, "stream create");
+      for (cudaEvent_t* e : {&B.sfork, &B.sjoin, &B.done})
+        if (!r && cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess)
+          r = fail(MT_ERR_CUDA, "event create");
+    }
+    for (cudaEvent_t* e : {&s.fork, &s.ev0, &s.ev1, &s.done})
+      if (!r && cudaEventCreate(e) != cudaSuccess) r = fail(MT_ERR_CUDA, "event create");
+    if (!r && cudaEventCreateWithFlags(&s.pfork, cudaEventDisableTiming) != cudaSuccess)
+      r = fail(MT_ERR_CUDA, "event create");
+  }
   return r;
 }
 
@@ -346,11 +371,7 @@ extern "C" int mt_job_create(mt_context* ctx, mt_scene* scene, const mt_render_c
     j->nslots = j->merge ? frames : std::max(1, at_once / nbuf);
     j->logged = nbuf > 1 || (!j->merge && j->nslots > 1);
     j->slots.resize(j->nslots);
-    for (JobSlot& s : j->slots)
-      if (!r) r = alloc_slot(ctx, s, *cfg, nbuf, j->logged, j->merge || !j->logged, j->status_stride);
-    if (!r) r = dalloc(j->ctx, &j->d_totals, 4);
-    if (!r && (j->merge || j->logged)) r = dalloc(j->ctx, &j->d_film, N);
-    if (!r && (j->merge || j->logged)) r = dalloc(j->ctx, &j->d_film_c, N);
+    r = alloc_slots(j, nbuf);
     j->scene_version = scene->version;
     if (!r) r = setup_grid(j);
     if (r != MT_ERR_NOMEM || at_once == 1) break;
